@@ -233,6 +233,7 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
   OTM_CUDA(cudaMemsetAsync(p, 0, 3 * nv * sizeof(float), stream));
   nc = int(lv.back().d.nv());
   OTM_TRY(alloc((void**)&Ainv, size_t(nc) * nc * sizeof(double)));
+  OTM_TRY(plan_direct_inverse());
   OTM_TRY(alloc((void**)&table, 64 * 27 * sizeof(float)));
   OTM_TRY(alloc((void**)&sc, sizeof(SolveScalars)));
   OTM_TRY(alloc((void**)&partials, size_t(kMaxPartials) * 16 * sizeof(double)));
@@ -410,6 +411,78 @@ otm_status Homo::tile_attributes() {
   return OTM_OK;
 }
 
+// The cluster launch of the coarsest inverse.
+static cudaLaunchConfig_t direct_launch(const DirPlan& p, cudaStream_t s, cudaLaunchAttribute* at) {
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(p.ncl);
+  lc.blockDim = dim3(kDirThreads);
+  lc.dynamicSmemBytes = p.smem;
+  lc.stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = unsigned(p.ncl);
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return lc;
+}
+
+// The cluster size of the coarsest inverse on the current device: 16 CTAs (a non-portable size) where
+// one such cluster with the largest plan's shared memory can be scheduled, else 8 (0: neither). Asked
+// once per device; the attributes are set on every call (they belong to the context).
+static int direct_cluster_size() {
+  static std::atomic<int> known[64];  // -1: none, 0: not asked yet
+  void* ks[2] = {(void*)k_direct_inverse<true>, (void*)k_direct_inverse<false>};
+  bool set = true;
+  for (void* k : ks)
+    set = set &&
+          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem) == cudaSuccess &&
+          cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  int dev = 0;
+  if (!set || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();  // a refused attribute leaves no error behind
+    return 0;
+  }
+  int size = dev < 64 ? known[dev].load() : 0;
+  if (size != 0) return std::max(size, 0);
+  for (int ncl = kDirCl; ncl >= 8 && size == 0; ncl /= 2) {
+    DirPlan p{};
+    p.ncl = ncl;
+    p.smem = kMaxDynSmem;
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t lc = direct_launch(p, nullptr, at);
+    int a = 0, b = 0;
+    if (cudaOccupancyMaxActiveClusters(&a, ks[0], &lc) == cudaSuccess && a >= 1 &&
+        cudaOccupancyMaxActiveClusters(&b, ks[1], &lc) == cudaSuccess && b >= 1)
+      size = ncl;
+    cudaGetLastError();  // nor does a refused query
+  }
+  if (dev < 64) known[dev].store(size ? size : -1);
+  return size;
+}
+
+otm_status Homo::plan_direct_inverse() {
+  const int ncl = direct_cluster_size();
+  if (ncl == 0) {
+    set_error("the device cannot schedule a cluster for the coarsest direct solve");
+    return OTM_ERR_UNSUPPORTED;
+  }
+  dir = dir_plan(nc, ncl);
+  return alloc((void**)&dir_work, dir.work * sizeof(double));
+}
+
+otm_status Homo::launch_direct_inverse(cudaStream_t cs) {
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t lc = direct_launch(dir, cs, at);
+  const Dims d = lv.back().d;
+  const float* st = lv.back().st;
+  if (dir.smem_rows)
+    OTM_CUDA(cudaLaunchKernelEx(&lc, k_direct_inverse<true>, d, st, Ainv, dir_work, dir, flags + 1));
+  else
+    OTM_CUDA(cudaLaunchKernelEx(&lc, k_direct_inverse<false>, d, st, Ainv, dir_work, dir, flags + 1));
+  launched(1);
+  return OTM_OK;
+}
+
 otm_status Homo::join_coarse() {
   if (!coarse_pending) return OTM_OK;
   OTM_CUDA(cudaStreamWaitEvent(stream, ev_coarse, 0));
@@ -504,16 +577,7 @@ otm_status Homo::update_operators() {
     OTM_CHECK_LAUNCH("k_fine_stencil");
     launched(1);
   }
-  {
-    const size_t abytes = size_t(nc) * nc * sizeof(double);
-    const int use_smem = abytes <= size_t(kMaxDynSmem);
-    if (use_smem)
-      OTM_CUDA(cudaFuncSetAttribute(k_coarsest_build, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
-    k_coarsest_build<<<1, 1024, use_smem ? abytes : 0, cs>>>(lv.back().d, lv.back().st, Ainv, flags + 1,
-                                                              use_smem);
-  }
-  OTM_CHECK_LAUNCH("k_coarsest_build");
-  launched(1);
+  OTM_TRY(launch_direct_inverse(cs));
   if (side) {
     OTM_CUDA(cudaEventRecord(ev_coarse, side));
     coarse_pending = true;
@@ -641,8 +705,8 @@ void Homo::vcycle(int l) {
     return;
   }
   if (l == int(lv.size()) - 1) {
-    launch_pdl(k_coarsest_solve, dim3(1), dim3(std::min(1024, std::max(32, (nc + 31) / 32 * 32))), 3 * nc * sizeof(double), stream, 
-        nc, Ainv, L.f, L.u, sc);
+    launch_pdl(k_coarsest_solve, dim3(ceil_div(nc, kDirSolveThreads / 32)), dim3(kDirSolveThreads),
+               3 * nc * sizeof(double), stream, nc, (const double*)Ainv, (const float*)L.f, L.u, (const SolveScalars*)sc);
     launched(1);
     return;
   }

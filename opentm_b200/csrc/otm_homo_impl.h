@@ -8,6 +8,7 @@
 #include "otm_mg_kernels.cuh"
 #include "otm_solver_kernels.cuh"
 #include "otm_cluster.cuh"
+#include "otm_direct.cuh"
 #include "otm_tail.cuh"
 #include "otm_tile.cuh"
 #include "otm_ctile.cuh"
@@ -86,6 +87,8 @@ struct Homo {
   int tail_l = -1;          // first level handled by the single-CTA tail kernel (-1: none)
   size_t tail_smem = 0;     // its dynamic shared memory
   int nc = 0;
+  DirPlan dir{};               // the coarsest inverse's plan and its global scratch
+  double* dir_work = nullptr;
   float* table = nullptr;
   SolveScalars* sc = nullptr;
   SolveScalars* sc_host = nullptr;
@@ -144,6 +147,8 @@ struct Homo {
   } sens_req;
   otm_status heat_matrix_sensitivity(double C[9], const float dC[9], float* sens, int pitchT, int lexi);
   otm_status tile_attributes();
+  otm_status plan_direct_inverse();
+  otm_status launch_direct_inverse(cudaStream_t cs);
   otm_status join_coarse();
   otm_status enter();
   otm_status leave();

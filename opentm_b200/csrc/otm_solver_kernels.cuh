@@ -887,144 +887,6 @@ static __global__ void k_loop_ctrl(SolveScalars* sc, cudaGraphConditionalHandle 
 }
 
 // ---------------------------------------------------------------------------------------
-// Coarsest level: dense FP64 inverse of A_c + (alpha/n) 1 1^T (SPD on the periodic
-// nullspace), built once per update; each V-cycle applies it as a mat-vec. Replaces the
-// host BiCGSTAB(ILUT) + nullspace projection of Grid_H::solveHostEquation
-// (homogenization/grid.cpp:272-310).
-// ---------------------------------------------------------------------------------------
-// With use_smem the matrix is assembled and inverted in dynamic shared memory (n^2 doubles)
-// and copied to Aout at the end; otherwise it is worked on in place in Aout.
-constexpr int kGjRegs = 4;  // matrix elements per thread of the register-buffered elimination
-static __global__ void __launch_bounds__(1024) k_coarsest_build(Dims d, const float* __restrict__ st, double* Aout, int* status,
-                                        int use_smem) {
-  extern __shared__ double smA[];
-  const int n = int(d.nv());
-  double* A = use_smem ? smA : Aout;
-  for (size_t i = threadIdx.x; i < size_t(n) * n; i += blockDim.x) A[i] = 0.0;
-  __syncthreads();
-  __shared__ double dsum;
-  if (threadIdx.x == 0) dsum = 0.0;
-  __syncthreads();
-  // row v assembled by one thread (handles periodic aliasing of small dims)
-  for (int v = threadIdx.x; v < n; v += blockDim.x) {
-    const int x = v % d.nx, y = (v / d.nx) % d.ny, z = v / (d.nx * d.ny);
-    for (int o = 0; o < 27; o++) {
-      const int jx = (x + o % 3 - 1 + d.nx) % d.nx, jy = (y + (o / 3) % 3 - 1 + d.ny) % d.ny,
-                jz = (z + o / 9 - 1 + d.nz) % d.nz;
-      const int j = jx + d.nx * (jy + d.ny * jz);
-      A[size_t(v) * n + j] += double(st[size_t(o) * n + v]);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int v = 0; v < n; v++) s += A[size_t(v) * n + v];
-    dsum = s;
-  }
-  __syncthreads();
-  const double alpha = dsum / double(n) / double(n);
-  for (size_t i = threadIdx.x; i < size_t(n) * n; i += blockDim.x) A[i] += alpha;
-  __syncthreads();
-  // in-place Gauss-Jordan inversion without pivoting (SPD)
-  const int nn = n * n;  // n <= 1024
-  if (nn <= kGjRegs * int(blockDim.x)) {
-    // small systems: every element of step k is computed from the step's old values into
-    // registers, then written back (two barriers per pivot instead of four)
-    double nw[kGjRegs];
-    int ei[kGjRegs], ej[kGjRegs];  // (row, column) of the thread's elements, fixed over the pivots
-#pragma unroll
-    for (int e = 0; e < kGjRegs; e++) {
-      const int idx = int(threadIdx.x) + e * int(blockDim.x);
-      ei[e] = idx / n;
-      ej[e] = idx - ei[e] * n;
-    }
-    for (int k = 0; k < n; k++) {
-      const double pv = A[k * n + k];
-      if (threadIdx.x == 0 && !(pv > 0.0)) *status = 1;
-      const double pinv = 1.0 / pv;
-#pragma unroll
-      for (int e = 0; e < kGjRegs; e++) {
-        const int idx = int(threadIdx.x) + e * int(blockDim.x);
-        if (idx < nn) {
-          const int i = ei[e], j = ej[e];
-          const double a = A[idx];
-          if (i == k)
-            nw[e] = j == k ? pinv : a * pinv;
-          else if (j == k)
-            nw[e] = a * -pinv;
-          else
-            nw[e] = a - A[i * n + k] * (A[k * n + j] * pinv);
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int e = 0; e < kGjRegs; e++) {
-        const int idx = int(threadIdx.x) + e * int(blockDim.x);
-        if (idx < nn) A[idx] = nw[e];
-      }
-      __syncthreads();
-    }
-    if (use_smem)
-      for (int i = threadIdx.x; i < nn; i += blockDim.x) Aout[i] = A[i];
-    return;
-  }
-  __shared__ double piv_inv;
-  for (int k = 0; k < n; k++) {
-    if (threadIdx.x == 0) {
-      const double pv = A[size_t(k) * n + k];
-      if (!(pv > 0.0)) *status = 1;
-      piv_inv = 1.0 / pv;
-    }
-    __syncthreads();
-    const double pinv = piv_inv;
-    for (int j = threadIdx.x; j < n; j += blockDim.x)
-      if (j != k) A[size_t(k) * n + j] *= pinv;
-    __syncthreads();
-    for (size_t idx = threadIdx.x; idx < size_t(n) * n; idx += blockDim.x) {
-      const int i = int(idx / n), j = int(idx % n);
-      if (i != k && j != k) A[idx] -= A[size_t(i) * n + k] * A[size_t(k) * n + j];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-      if (i != k) A[size_t(i) * n + k] *= -pinv;
-    __syncthreads();
-    if (threadIdx.x == 0) A[size_t(k) * n + k] = pinv;
-    __syncthreads();
-  }
-  if (use_smem)
-    for (size_t i = threadIdx.x; i < size_t(n) * n; i += blockDim.x) Aout[i] = A[i];
-}
-
-// u = Ainv (f - mean f) for the 3 cases (one block).
-static __global__ void k_coarsest_solve(int n, const double* __restrict__ Ainv, const float* __restrict__ f, float* u,
-                                 const SolveScalars* sc) {
-  pdl_wait();
-  if (sc && solve_done(sc)) return;
-  extern __shared__ double bsh[];  // 3 * n
-  __shared__ double mean[3];
-  for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) bsh[i] = f[i];
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    double s = 0.0;
-    for (int i = 0; i < n; i++) s += bsh[threadIdx.x * n + i];
-    mean[threadIdx.x] = s / n;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int j = 0; j < n; j++) {
-      const double m = Ainv[size_t(j) * n + i];  // symmetric: column read is coalesced
-      a0 += m * (bsh[j] - mean[0]);
-      a1 += m * (bsh[n + j] - mean[1]);
-      a2 += m * (bsh[2 * n + j] - mean[2]);
-    }
-    u[i] = float(a0);
-    u[n + i] = float(a1);
-    u[2 * n + i] = float(a2);
-  }
-}
-
-// ---------------------------------------------------------------------------------------
 // K^H and sensitivity (homogenization/homogenization.cu:13-153, 255-412).
 // ---------------------------------------------------------------------------------------
 
