@@ -27,6 +27,10 @@ otm_status cuda_fail(cudaError_t e, const char* what);
 // Stream-ordered scratch from the library's per-device memory pool (freed with cudaFreeAsync).
 cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t s);
 
+// The OC sensitivity filter (periodic, Linear weights) in place, with d.nv() floats of scratch at tmp.
+otm_status oc_filter_run(const struct Dims& d, float* sens, const float* rho, size_t pitch, float* tmp, float radius,
+                         cudaStream_t s);
+
 #define OTM_CUDA(call)                                  \
   do {                                                  \
     cudaError_t e__ = (call);                           \

@@ -2,11 +2,12 @@
 // fused SIMP density chain and their adjoints (AutoDiff/TensorExpression.h:993-1185,
 // AutoDiff/TensorExpression.cuh:281-385).
 //
-// The nonzero normalised weights travel as a kernel parameter (constant bank, broadcast to the
+// The normalised weights travel as a kernel parameter (constant bank, broadcast to the
 // warp), so no device allocation or global state is used.
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "otm_common.cuh"
 
@@ -57,10 +58,16 @@ static otm_status make_weights(int type, float radius, ConvWeights* cw) {
   return OTM_OK;
 }
 
-// Shared-memory tiled convolution: a 256-thread block produces a 32 x 8 x 4 tile of outputs
-// from the (32+2h) x (8+2h) x (4+2h) input tile it stages in shared memory (with periodic wrap
-// or a validity mask for zero padding), so each input value is read from global memory about
-// once instead of (2h+1)^3 times. The taps are summed in the reference's order (x fastest).
+// Convolution streaming along z: a 128-thread block produces the outputs of a tile of 32 x 4 kNY
+// (x, y) columns for a chunk of z planes, kNY rows of outputs per thread and plane. Each input plane of
+// the chunk (and H planes either side) is staged once in shared memory, with periodic wrap or zeros
+// outside, the next one being fetched into registers meanwhile; a thread reads the (kNY + 2H) x (2H + 1)
+// window around its outputs once per plane and adds every value to the 2H + 1 outputs along z that it
+// is a tap of (rolling accumulators): 9 reads per output at radius 2 with one row, 17.5 at radius 3 with
+// four, where a read per tap takes 27 and 93. The weight depends on the squared distance only, and with the
+// loops unrolled its place in the parameter bank is a constant, so a tap is one FMA. The radii in common
+// use (1.5 to 2, 2.5, 3, 3.5, 4) have their set of taps compiled in; others skip the zero weights by
+// branches that all threads take alike. An output's taps are summed in the reference's order (x fastest, z slowest; the adjoint streams z downwards for that).
 //   MODE 0: forward            out = sum w src / sum_valid w
 //   MODE 1: forward + SIMP     also k = (k0 - kmin) out^p + kmin and dk = dk/dout
 //   MODE 2: adjoint            out = sum_off w g(i - off) / ws(i - off)
@@ -68,159 +75,290 @@ static otm_status make_weights(int type, float radius, ConvWeights* cw) {
 //   MODE 4: forward + SIMP + conductivity import: as 1, with k written as the solver's raw
 //           conductivity and ks = 1e-9 + k^pp beside it (k_import's arithmetic), a negative,
 //           NaN or Inf k flagged in *bad
-constexpr int kTX = 32, kTY = 8, kTZ = 4;
+//   MODE 5: OC sensitivity     out = sum w src / (sum w * rho), rho (ws_in) pitched like out
+constexpr int kTX = 32, kTYT = 4, kConvThreads = kTX * kTYT;
 
+// A radial filter: weight by squared distance, zero from smax on; the sums of a whole z plane of weights
+// by |oz| (for the valid weight of voxels cut along z only).
 template <int H>
-constexpr int tile_elems() {
-  return (kTX + 2 * H) * (kTY + 2 * H) * (kTZ + 2 * H);
-}
-
-// The nonzero taps of a filter in the reference's order (x fastest), each with its offset in
-// the shared-memory tile: a radial kernel has many zero weights in its cube (27 of 125 taps are
-// nonzero for radius 2), and skipping them leaves every sum unchanged.
-struct TapList {
-  int n;
-  int doff[kMaxTaps];  // oz * SX * SY + oy * SX + ox for the forward direction (negated for the adjoint)
-  float w[kMaxTaps];
+struct Radial {
+  float w[3 * H * H + 1];
+  int smax;
+  float plane[H + 1];
 };
 
 template <int H>
-static void make_taps(const ConvWeights& cw, TapList* tl) {
-  constexpr int SX = kTX + 2 * H, SY = kTY + 2 * H, W1 = 2 * H + 1;
-  tl->n = 0;
-  for (int t = 0; t < cw.taps; t++) {
-    if (cw.w[t] == 0.f) continue;
-    const int ox = t % W1 - H, oy = t / W1 % W1 - H, oz = t / (W1 * W1) - H;
-    tl->doff[tl->n] = oz * SX * SY + oy * SX + ox;
-    tl->w[tl->n] = cw.w[t];
-    tl->n++;
+static void make_radial(const ConvWeights& cw, Radial<H>* r) {
+  constexpr int W1 = 2 * H + 1;
+  for (float& w : r->w) w = 0.f;
+  r->smax = 0;
+  for (int k = 0; k <= H; k++) {
+    r->plane[k] = 0.f;
+    for (int oy = -H; oy <= H; oy++)
+      for (int ox = -H; ox <= H; ox++) {
+        const int s = ox * ox + oy * oy + k * k;
+        r->w[s] = cw.w[(ox + H) + W1 * ((oy + H) + W1 * (k + H))];
+        if (r->w[s] != 0.f && s >= r->smax) r->smax = s + 1;
+        r->plane[k] += r->w[s];
+      }
   }
 }
 
-template <int H, int MODE>
-__global__ void __launch_bounds__(256) k_conv_tiled(Dims d, const float* __restrict__ src, int src_pitch,
-                                                    const float* __restrict__ dk_in, const float* __restrict__ ws_in,
-                                                    float* __restrict__ dst, int dst_pitch,
-                                                    float* __restrict__ ws_out, int periodic, TapList tl,
-                                                    float wsum_all, float p, float k0, float kmin,
-                                                    float* __restrict__ kout, float* __restrict__ dkout,
-                                                    float* __restrict__ ksout, float pp, int* bad) {
-  constexpr int SX = kTX + 2 * H, SY = kTY + 2 * H, SZ = kTZ + 2 * H;
-  constexpr bool kFwd = MODE < 2 || MODE == 4;
-  extern __shared__ float sm[];
-  float* val = sm;
-  float* msk = sm + SX * SY * SZ;  // only used without periodicity
-  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * kTZ;
-  // stage the tile row by row: x from the thread's lane (two passes cover SX = 32 + 2H), the
-  // (y, z) row from one small division, the wrapped x coordinates computed once
-  int gxs[2];
-  bool inx[2];
+// kS: the filter's smax where it is known at compile time (then the taps are straight-line code), else 0.
+template <int H, int kS, int kNY, int MODE>
+__global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const float* __restrict__ src, size_t src_pitch,
+                                                              const float* __restrict__ dk_in,
+                                                              const float* __restrict__ ws_in,
+                                                              float* __restrict__ dst, size_t dst_pitch,
+                                                              float* __restrict__ ws_out, int periodic, int zchunk,
+                                                              const __grid_constant__ Radial<H> rw, float wsum_all,
+                                                              float p, float k0, float kmin, float* __restrict__ kout,
+                                                              float* __restrict__ dkout, float* __restrict__ ksout,
+                                                              float pp, int* bad) {
+  constexpr int kTY = kTYT * kNY;
+  constexpr int SX = kTX + 2 * H, SY = kTY + 2 * H, SN = SX * SY, NL = (SN + kConvThreads - 1) / kConvThreads;
+  constexpr bool kFwd = MODE < 2 || MODE >= 4, kValid = kFwd && MODE != 5;
+  constexpr int W1 = 2 * H + 1;
+  __shared__ float buf[2][SN];
+  __shared__ float wplane[kValid ? H + 1 : 1][kTY][kTX];  // zero padding: valid weights of a column by |oz|
+  const int tid = threadIdx.x + kTX * threadIdx.y;
+  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * zchunk;
+  const int z1 = min(z0 + zchunk, d.nz), planes = z1 - z0 + 2 * H;
+  const int ox = x0 + int(threadIdx.x), oyr = int(threadIdx.y) * kNY, oy0 = y0 + oyr;  // own outputs
+  if (kValid && !periodic) {
+    // in x, this thread's taps are inside from ex = xlo to xhi
+    const int xlo = max(-H, -ox), xhi = min(H, d.nx - 1 - ox);
 #pragma unroll
-  for (int k = 0; k < 2; k++) {
-    int gx = x0 + int(threadIdx.x) + k * kTX - H;
-    inx[k] = gx >= 0 && gx < d.nx;
-    if (!inx[k]) gx = ((gx % d.nx) + d.nx) % d.nx;
-    gxs[k] = gx;
-  }
-  for (int rowi = threadIdx.y; rowi < SY * SZ; rowi += kTY) {
-    const int ly = rowi % SY, lz = rowi / SY;
-    int gy = y0 + ly - H, gz = z0 + lz - H;
-    const bool inyz = gy >= 0 && gy < d.ny && gz >= 0 && gz < d.nz;
-    if (gy < 0 || gy >= d.ny) gy = ((gy % d.ny) + d.ny) % d.ny;
-    if (gz < 0 || gz >= d.nz) gz = ((gz % d.nz) + d.nz) % d.nz;
-    const size_t row = size_t(gy) + size_t(d.ny) * gz;
+    for (int j = 0; j < kNY; j++) {
+      const int oy = oy0 + j;
+      float t[H + 1];
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const int lx = int(threadIdx.x) + k * kTX;
-      if (lx >= SX) continue;
-      const int gx = gxs[k];
-      float v = 0.f, m = 0.f;
-      if ((inx[k] && inyz) || periodic) {
-        v = __ldg(src + row * src_pitch + gx);
-        if (!kFwd) {
-          const size_t q = row * d.nx + gx;
-          if (MODE == 3) v *= __ldg(dk_in + q);
-          v /= __ldg(ws_in + q);
-        }
-        m = 1.f;
+      for (int k = 0; k <= H; k++) t[k] = rw.plane[k];
+      if (xlo > -H || xhi < H || oy < H || oy >= d.ny - H) {
+#pragma unroll
+        for (int k = 0; k <= H; k++) t[k] = 0.f;
+#pragma unroll(H <= 3 ? 2 * H + 1 : 1)
+        for (int ey = -H; ey <= H; ey++)
+          if (oy + ey >= 0 && oy + ey < d.ny)
+#pragma unroll
+            for (int ex = -H; ex <= H; ex++) {
+              const bool in = ex >= xlo && ex <= xhi;
+#pragma unroll
+              for (int k = 0; k <= H; k++) t[k] += in ? rw.w[ex * ex + ey * ey + k * k] : 0.f;
+            }
       }
-      val[rowi * SX + lx] = v;
-      if (!periodic) msk[rowi * SX + lx] = m;
+#pragma unroll
+      for (int k = 0; k <= H; k++) wplane[k][oyr + j][threadIdx.x] = t[k];
     }
   }
+  // this thread's staged positions (the same in every plane): offsets in a plane of src and of the
+  // unpitched dk and ws
+  size_t off[NL], offw[kFwd ? 1 : NL];
+  bool ok[NL];
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    const int s = tid + i * kConvThreads;
+    int x = x0 + s % SX - H, y = y0 + s / SX - H;
+    const bool in = x >= 0 && x < d.nx && y >= 0 && y < d.ny;
+    if (!in) {
+      x = ((x % d.nx) + d.nx) % d.nx;
+      y = ((y % d.ny) + d.ny) % d.ny;
+    }
+    off[i] = size_t(y) * src_pitch + x;
+    if (!kFwd) offw[kFwd ? 0 : i] = size_t(y) * d.nx + x;
+    ok[i] = s < SN && (in || periodic);
+  }
+  // plane `pl` of the chunk, counted in streaming order: the loads into registers first (none waits for
+  // another), the arithmetic when the plane is staged
+  float v[NL], vk[MODE == 3 ? NL : 1], vw[kFwd ? 1 : NL];
+  auto fetch = [&](int pl) {
+    int gz = kFwd ? z0 - H + pl : z1 - 1 + H - pl;
+    const bool inz = gz >= 0 && gz < d.nz;
+    if (!inz) gz = ((gz % d.nz) + d.nz) % d.nz;
+    const float* ps = src + size_t(gz) * d.ny * src_pitch;
+    const size_t pw = size_t(gz) * d.ny * d.nx;
+    const bool any = inz || periodic;
+#pragma unroll
+    for (int i = 0; i < NL; i++) {
+      const bool take = ok[i] && any;
+      v[i] = take ? __ldg(ps + off[i]) : 0.f;
+      if (MODE == 3) vk[MODE == 3 ? i : 0] = take ? __ldg(dk_in + pw + offw[kFwd ? 0 : i]) : 0.f;
+      if (!kFwd) vw[kFwd ? 0 : i] = take ? __ldg(ws_in + pw + offw[kFwd ? 0 : i]) : 1.f;
+    }
+  };
+  auto stage = [&](float* b) {
+#pragma unroll
+    for (int i = 0; i < NL; i++) {
+      float t = v[i];
+      if (MODE == 3) t *= vk[MODE == 3 ? i : 0];
+      if (!kFwd) t /= vw[kFwd ? 0 : i];
+      if (tid + i * kConvThreads < SN) b[tid + i * kConvThreads] = t;
+    }
+  };
+  fetch(0);
+  stage(buf[0]);
   __syncthreads();
-  const int gx = x0 + threadIdx.x, gy = y0 + threadIdx.y;
-  if (gx >= d.nx || gy >= d.ny) return;
-  // the four z outputs of this thread together: each tap's weight and offset serve all four;
-  // every output still sums its taps in the reference's order
-  float sum[kTZ], wsv[kTZ];
+  const int base = (oyr + H) * SX + int(threadIdx.x) + H;
+  float acc[W1][kNY];  // acc[a]: the output H - a planes behind the current input plane
 #pragma unroll
-  for (int tz = 0; tz < kTZ; tz++) sum[tz] = wsv[tz] = 0.f;
-  const int base = H * SX * SY + (threadIdx.y + H) * SX + (threadIdx.x + H);
-#pragma unroll 8
-  for (int t = 0; t < tl.n; t++) {
-    const float w = tl.w[t];
-    const int li = base + (kFwd ? tl.doff[t] : -tl.doff[t]);
+  for (int a = 0; a < W1; a++)
 #pragma unroll
-    for (int tz = 0; tz < kTZ; tz++) {
-      sum[tz] += w * val[li + tz * SX * SY];
-      if (kFwd && !periodic) wsv[tz] += w * msk[li + tz * SX * SY];
-    }
-  }
+    for (int j = 0; j < kNY; j++) acc[a][j] = 0.f;
+  for (int pl = 0; pl < planes; pl++) {
+    if (pl + 1 < planes) fetch(pl + 1);
+    const float* b = buf[pl & 1] + base;
+    if (kS > 0) {
+      // row by row of the window, every value read once; an output meets its taps (oy, ox) in the
+      // reference's order (the adjoint's offsets are negated, so it takes the rows downwards)
 #pragma unroll
-  for (int tz = 0; tz < kTZ; tz++) {
-    const int gz = z0 + tz;
-    if (gz >= d.nz) break;
-    const float sumv = sum[tz];
-    float ws = wsv[tz];
-    const size_t row = size_t(gy) + size_t(d.ny) * gz;
-    if (kFwd) {
-      if (periodic) ws = wsum_all;
-      const float out = sumv / ws;
-      if (dst) dst[row * dst_pitch + gx] = out;
-      if (ws_out) ws_out[row * d.nx + gx] = ws;
-      if (MODE == 1 || MODE == 4) {
-        const float pw = (p == 3.f) ? out * out * out : powf(out, p);
-        const float k = (k0 - kmin) * pw + kmin;
-        kout[row * d.nx + gx] = k;
-        const float dpw = (p == 3.f) ? 3.f * out * out : p * powf(out, p - 1.f);
-        dkout[row * d.nx + gx] = (k0 - kmin) * dpw;
-        if (MODE == 4) {
-          if (!(k >= 0.f) || !isfinite(k)) atomicOr(bad, 1);
-          ksout[row * d.nx + gx] = kRhoPenalMin + (pp == 1.f ? k : powf(k, pp));
+      for (int i = 0; i < kNY + 2 * H; i++) {
+        const int r = kFwd ? i - H : kNY - 1 + H - i;
+#pragma unroll
+        for (int ex = -H; ex <= H; ex++) {
+          if (ex * ex >= kS) continue;
+          const float t = b[r * SX + (kFwd ? ex : -ex)];
+#pragma unroll
+          for (int j = 0; j < kNY; j++) {
+            const int ey = kFwd ? r - j : j - r;
+            if (ey < -H || ey > H) continue;
+#pragma unroll
+            for (int k = 0; k <= H; k++) {
+              const int q = ex * ex + ey * ey + k * k;
+              if (q >= kS) continue;
+              acc[H - k][j] += rw.w[q] * t;
+              if (k > 0) acc[H + k][j] += rw.w[q] * t;
+            }
+          }
         }
       }
     } else {
-      dst[row * dst_pitch + gx] = sumv;
+#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
+      for (int ey = -H; ey <= H; ey++)
+#pragma unroll
+        for (int ex = -H; ex <= H; ex++) {
+          const int d2 = ex * ex + ey * ey, off = kFwd ? ey * SX + ex : -(ey * SX + ex);
+          if (d2 >= rw.smax) continue;
+          float t[kNY];
+#pragma unroll
+          for (int j = 0; j < kNY; j++) t[j] = b[off + j * SX];
+#pragma unroll
+          for (int k = 0; k <= H; k++) {
+            if (d2 + k * k >= rw.smax) break;
+            const float w = rw.w[d2 + k * k];
+#pragma unroll
+            for (int j = 0; j < kNY; j++) {
+              acc[H - k][j] += w * t[j];
+              if (k > 0) acc[H + k][j] += w * t[j];
+            }
+          }
+        }
     }
+    if (pl >= 2 * H) {
+      const int gz = kFwd ? z0 + pl - 2 * H : z1 - 1 - (pl - 2 * H);
+#pragma unroll
+      for (int j = 0; j < kNY; j++) {
+        const int oy = oy0 + j;
+        if (ox >= d.nx || oy >= d.ny) continue;
+        const float sumv = acc[0][j];
+        const size_t row = size_t(oy) + size_t(d.ny) * gz;
+        const size_t e = row * d.nx + ox;
+        if (!kFwd) {
+          dst[row * dst_pitch + ox] = sumv;
+        } else if (MODE == 5) {
+          const size_t q = row * dst_pitch + ox;
+          dst[q] = sumv / (wsum_all * __ldg(ws_in + q));
+        } else {
+          float ws = wsum_all;
+          if (!periodic && (ox < H || ox >= d.nx - H || oy < H || oy >= d.ny - H || gz < H || gz >= d.nz - H)) {
+            ws = 0.f;
+            for (int k = -H; k <= H; k++)
+              if (gz + k >= 0 && gz + k < d.nz) ws += wplane[k < 0 ? -k : k][oyr + j][threadIdx.x];
+          }
+          const float out = sumv / ws;
+          if (dst) dst[row * dst_pitch + ox] = out;
+          if (ws_out) ws_out[e] = ws;
+          if (MODE == 1 || MODE == 4) {
+            const float pw = (p == 3.f) ? out * out * out : powf(out, p);
+            const float k = (k0 - kmin) * pw + kmin;
+            kout[e] = k;
+            const float dpw = (p == 3.f) ? 3.f * out * out : p * powf(out, p - 1.f);
+            dkout[e] = (k0 - kmin) * dpw;
+            if (MODE == 4) {
+              if (!(k >= 0.f) || !isfinite(k)) atomicOr(bad, 1);
+              ksout[e] = kRhoPenalMin + (pp == 1.f ? k : powf(k, pp));
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 2 * H; a++)
+#pragma unroll
+      for (int j = 0; j < kNY; j++) acc[a][j] = acc[a + 1][j];
+#pragma unroll
+    for (int j = 0; j < kNY; j++) acc[2 * H][j] = 0.f;
+    if (pl + 1 < planes) stage(buf[(pl + 1) & 1]);  // last read one plane ago, before the barrier below
+    __syncthreads();
   }
 }
 
+// Blocks of a launch with ny rows per thread and z chunks of zc planes, and the chunk to use: the longest
+// (least work on the 2H planes around it) that still gives the GPU enough blocks, at least 4.
+constexpr long long kConvFill = 8 * 148;
+static long long conv_blocks(const Dims& d, int ny, int zc) {
+  return (long long)((d.nx + kTX - 1) / kTX) * ((d.ny + kTYT * ny - 1) / (kTYT * ny)) * ((d.nz + zc - 1) / zc);
+}
+static int conv_zchunk(const Dims& d, int ny) {
+  int zc = 32;
+  while (zc > 4 && conv_blocks(d, ny, zc) < kConvFill) zc /= 2;
+  return zc;
+}
+
 template <int H, int MODE>
-static otm_status launch_tiled(const Dims& d, const float* src, int src_pitch, const float* dk_in,
-                               const float* ws_in, float* dst, int dst_pitch, float* ws_out, int periodic,
-                               const ConvWeights& cw, float wsum_all, float p, float k0, float kmin, float* kout,
-                               float* dkout, float* ksout, float pp, int* bad, cudaStream_t s) {
-  const size_t smem = size_t(tile_elems<H>()) * sizeof(float) * (periodic ? 1 : 2);
-  static bool attr = false;  // the attribute is per function and process-wide
-  if (!attr) {
-    cudaFuncSetAttribute(k_conv_tiled<H, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * tile_elems<H>() * 4);
-    attr = true;
-  }
-  dim3 grid((d.nx + kTX - 1) / kTX, (d.ny + kTY - 1) / kTY, (d.nz + kTZ - 1) / kTZ);
-  TapList tl;
-  make_taps<H>(cw, &tl);
-  k_conv_tiled<H, MODE><<<grid, dim3(kTX, kTY), smem, s>>>(d, src, src_pitch, dk_in, ws_in, dst, dst_pitch, ws_out,
-                                                          periodic, tl, wsum_all, p, k0, kmin, kout, dkout, ksout,
-                                                          pp, bad);
-  OTM_CHECK_LAUNCH("k_conv_tiled");
+static otm_status launch_stream(const Dims& d, const float* src, size_t src_pitch, const float* dk_in, const float* ws_in,
+                                float* dst, size_t dst_pitch, float* ws_out, int periodic, const ConvWeights& cw,
+                                float wsum_all, float p, float k0, float kmin, float* kout, float* dkout, float* ksout,
+                                float pp, int* bad, cudaStream_t s) {
+  Radial<H> rw;
+  make_radial<H>(cw, &rw);
+  auto run = [&](auto ny_tag) {
+    constexpr int kNY = decltype(ny_tag)::value;
+    const int zchunk = conv_zchunk(d, kNY);
+    dim3 grid((d.nx + kTX - 1) / kTX, (d.ny + kTYT * kNY - 1) / (kTYT * kNY), (d.nz + zchunk - 1) / zchunk);
+    auto launch = [&](auto kern) {
+      kern<<<grid, dim3(kTX, kTYT), 0, s>>>(d, src, src_pitch, dk_in, ws_in, dst, dst_pitch, ws_out, periodic, zchunk,
+                                            rw, wsum_all, p, k0, kmin, kout, dkout, ksout, pp, bad);
+    };
+    if (H == 2 && rw.smax == 3)
+      launch(k_conv_stream<H, (H == 2 ? 3 : 0), kNY, MODE>);
+    else if (H == 2 && rw.smax == 4)
+      launch(k_conv_stream<H, (H == 2 ? 4 : 0), kNY, MODE>);
+    else if (H == 3 && rw.smax == 7)
+      launch(k_conv_stream<H, (H == 3 ? 7 : 0), kNY, MODE>);
+    else if (H == 3 && rw.smax == 9)
+      launch(k_conv_stream<H, (H == 3 ? 9 : 0), kNY, MODE>);
+    else if (H == 4 && rw.smax == 13)
+      launch(k_conv_stream<H, (H == 4 ? 13 : 0), kNY, MODE>);
+    else if (H == 4 && rw.smax == 15)
+      launch(k_conv_stream<H, (H == 4 ? 15 : 0), kNY, MODE>);
+    else
+      launch(k_conv_stream<H, 0, kNY, MODE>);
+  };
+  // rows per thread: 4 where the window's values are shared by enough taps and the cell fills the GPU
+  // with the fewer threads, else 1
+  constexpr int kFew = H >= 5 ? 4 : 1, kMany = H >= 3 ? 4 : 1;
+  if (kFew != kMany && conv_blocks(d, kMany, 16) < kConvFill)
+    run(std::integral_constant<int, kFew>{});
+  else
+    run(std::integral_constant<int, kMany>{});
+  OTM_CHECK_LAUNCH("k_conv_stream");
   count_launches(1);
   return OTM_OK;
 }
 
 template <int MODE>
-static otm_status conv_dispatch(const Dims& d, const float* src, int src_pitch, const float* dk_in,
-                                const float* ws_in, float* dst, int dst_pitch, float* ws_out, int periodic,
+static otm_status conv_dispatch(const Dims& d, const float* src, size_t src_pitch, const float* dk_in,
+                                const float* ws_in, float* dst, size_t dst_pitch, float* ws_out, int periodic,
                                 const ConvWeights& cw, float p, float k0, float kmin, float* kout, float* dkout,
                                 cudaStream_t s, float* ksout = nullptr, float pp = 1.f, int* bad = nullptr) {
   // sum of the normalised weights in the reference's tap order (the in-bounds weight of a
@@ -230,7 +368,7 @@ static otm_status conv_dispatch(const Dims& d, const float* src, int src_pitch, 
   switch (cw.half) {
 #define OTM_H(HH) \
   case HH:        \
-    return launch_tiled<HH, MODE>(d, src, src_pitch, dk_in, ws_in, dst, dst_pitch, ws_out, periodic, cw, wsum_all, \
+    return launch_stream<HH, MODE>(d, src, src_pitch, dk_in, ws_in, dst, dst_pitch, ws_out, periodic, cw, wsum_all, \
                                   p, k0, kmin, kout, dkout, ksout, pp, bad, s);
     OTM_H(0) OTM_H(1) OTM_H(2) OTM_H(3) OTM_H(4) OTM_H(5) OTM_H(6)
 #undef OTM_H
@@ -252,6 +390,28 @@ otm_status density_forward_import(const Dims& d, const float* rho, int rho_pitch
   OTM_TRY(make_weights(weight_type, radius, &cw));
   return conv_dispatch<4>(d, rho, rho_pitchT, nullptr, nullptr, rho_f, d.nx, wsum, periodic, cw, p, k0, kmin, kraw,
                           dk, s, ks, pp, bad);
+}
+
+__global__ void __launch_bounds__(256) k_product(Dims d, const float* __restrict__ sens, const float* __restrict__ rho,
+                                                 size_t pitch, float* __restrict__ out) {
+  const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (v >= d.nv()) return;
+  const size_t row = v / d.nx, q = row * pitch + (v - row * d.nx);
+  out[v] = sens[q] * rho[q];
+}
+
+// OCOptimizer::filterSens (optimization/OCOptimizer.cu:76-152): s_e <- sum w s_n rho_n / (sum w * rho_e)
+// over the periodic Linear neighbourhood, in place. The products s rho go to tmp (d.nv() floats)
+// first, so that the convolution can write s; at 128^3, radius 2: 1457 us with every tap read and
+// wrapped from global memory by each voxel and a copy back.
+otm_status oc_filter_run(const Dims& d, float* sens, const float* rho, size_t pitch, float* tmp, float radius,
+                         cudaStream_t s) {
+  ConvWeights cw;
+  OTM_TRY(make_weights(OTM_WEIGHT_LINEAR, radius, &cw));
+  k_product<<<unsigned(ceil_div(d.nv(), 256)), 256, 0, s>>>(d, sens, rho, pitch, tmp);
+  OTM_CHECK_LAUNCH("k_product");
+  count_launches(1);
+  return conv_dispatch<5>(d, tmp, d.nx, nullptr, rho, sens, pitch, nullptr, 1, cw, 1.f, 1.f, 0.f, nullptr, nullptr, s);
 }
 
 static otm_status check_reso(const int reso[3]) {

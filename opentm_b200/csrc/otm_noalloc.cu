@@ -2,7 +2,7 @@
 //
 // For callers that cannot allocate GPU memory while they run (their allocator already owns the
 // device's memory, or a cudaMalloc/cudaFree with its possible device-wide synchronisation is
-// not allowed in their loop). The filter's temporary copy lives in `g_noalloc_scratch`, a
+// not allowed in their loop). The filter's products s rho live in `g_noalloc_scratch`, a
 // file-scope device array of OTM_NOALLOC_MAX_CELLS floats that every GPU loading the library
 // holds until the process exits. In host code that symbol is only a host-side stand-in, never
 // a device address: its device address is looked up once per device with
@@ -10,7 +10,6 @@
 // get. Calls share the array, so calls whose GPU work overlaps race on it.
 #include <cuda_runtime.h>
 
-#include <cmath>
 #include <mutex>
 
 #include "opentm_b200_noalloc.h"
@@ -45,43 +44,6 @@ static otm_status scratch_address(float** out) {
 
 constexpr int kNaMaxHalf = 6;
 
-struct NaWeights {
-  int half, taps;
-  float w[(2 * kNaMaxHalf + 1) * (2 * kNaMaxHalf + 1) * (2 * kNaMaxHalf + 1)];
-};
-
-// s_new(e) = sum_n w s_n rho_n / (sum_n w * rho_e) over the periodic Linear neighbourhood
-// (optimization/OCOptimizer.cu:76-104), written unpitched into the scratch array.
-static __global__ void __launch_bounds__(256) k_filter_to_scratch(Dims d, const float* __restrict__ sens,
-                                                                  const float* __restrict__ rho, size_t pitch,
-                                                                  float* __restrict__ scratch, NaWeights fw) {
-  const size_t nv = d.nv();
-  const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  const int x = int(v % d.nx), y = int((v / d.nx) % d.ny), z = int(v / (size_t(d.nx) * d.ny));
-  const int h = fw.half, w1 = 2 * h + 1;
-  float sum = 0.f, ws = 0.f;
-  for (int t = 0; t < fw.taps; t++) {
-    const int ox = t % w1 - h, oy = (t / w1) % w1 - h, oz = t / (w1 * w1) - h;
-    const int px = ((x + ox) % d.nx + d.nx) % d.nx, py = ((y + oy) % d.ny + d.ny) % d.ny,
-              pz = ((z + oz) % d.nz + d.nz) % d.nz;
-    const size_t q = (size_t(py) + size_t(d.ny) * pz) * pitch + px;
-    const float w = fw.w[t];
-    sum += __ldg(sens + q) * __ldg(rho + q) * w;
-    ws += w;
-  }
-  const size_t e = (size_t(y) + size_t(d.ny) * z) * pitch + x;
-  scratch[v] = sum / (ws * __ldg(rho + e));
-}
-
-static __global__ void __launch_bounds__(256) k_scratch_to_sens(Dims d, const float* __restrict__ scratch, float* sens,
-                                                                size_t pitch) {
-  const size_t nv = d.nv();
-  const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  sens[(v / d.nx) * pitch + v % d.nx] = scratch[v];
-}
-
 }  // namespace otm
 
 using namespace otm;
@@ -101,23 +63,7 @@ extern "C" otm_status otm_oc_filter_sens_noalloc(float* sens, const float* rho, 
     set_error("filter radius must be in (0, 6.5)");
     return OTM_ERR_INVALID_ARGUMENT;
   }
-  NaWeights fw;
-  fw.half = h;
-  fw.taps = (2 * h + 1) * (2 * h + 1) * (2 * h + 1);
-  float wsum = 0.f;
-  for (int t = 0; t < fw.taps; t++) {
-    const int ox = t % (2 * h + 1) - h, oy = t / (2 * h + 1) % (2 * h + 1) - h, oz = t / ((2 * h + 1) * (2 * h + 1)) - h;
-    const float q2 = float(ox * ox + oy * oy + oz * oz) / (radius * radius);
-    fw.w[t] = q2 < 1.f ? 1.f - std::sqrt(q2) : 0.f;  // WeightFunc<Linear>
-    wsum += fw.w[t];
-  }
-  for (int t = 0; t < fw.taps; t++) fw.w[t] /= wsum;
   float* scratch = nullptr;
   OTM_TRY(scratch_address(&scratch));
-  cudaStream_t s = (cudaStream_t)stream;
-  k_filter_to_scratch<<<ceil_div(d.nv(), 256), 256, 0, s>>>(d, sens, rho, pitchT, scratch, fw);
-  k_scratch_to_sens<<<ceil_div(d.nv(), 256), 256, 0, s>>>(d, scratch, sens, pitchT);
-  OTM_CHECK_LAUNCH("otm_oc_filter_sens_noalloc");
-  count_launches(2);
-  return OTM_OK;
+  return oc_filter_run(d, sens, rho, pitchT, scratch, radius, (cudaStream_t)stream);
 }

@@ -189,81 +189,11 @@ __global__ void __launch_bounds__(kBlock) k_oc_tree_pass(int ne, const float* __
   }
 }
 
-// One bisection step: volume of the candidate density at g = (gmax + gmin) / 2.
-__global__ void __launch_bounds__(kBlock) k_oc_pass(int ne, const float* __restrict__ sens,
-                                                    const float* __restrict__ rho, float volratio, float min_rho,
-                                                    float step, float damp, double* partials, OcState* st) {
-  if (*((volatile int*)&st->done)) return;
-  __shared__ double smem[32];
-  const float g = float((st->gmax + st->gmin) / 2);
-  double v[1] = {0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x)
-    v[0] += oc_new_rho(__ldg(sens + i), __ldg(rho + i), g, min_rho, step, damp);
-  block_reduce_f64<1>(v, smem);
-  if (threadIdx.x == 0) partials[blockIdx.x] = v[0];
-  if (last_block(&st->counter)) {
-    double t[1];
-    reduce_partials<1>(partials, gridDim.x, t, smem);
-    if (threadIdx.x == 0) {
-      const double vol = t[0] / ne;
-      st->vol = vol;
-      st->g = double(g);
-      st->iters += 1;
-      if (vol < volratio - 0.0001)
-        st->gmax = double(g);
-      else if (vol > volratio + 0.0001)
-        st->gmin = double(g);
-      else
-        st->done = 1;
-      if (st->iters >= kOcSteps) st->done = 1;
-      st->counter = 0;
-    }
-  }
-}
-
 __global__ void __launch_bounds__(kBlock) k_oc_apply(int ne, const float* __restrict__ sens, float* rho,
                                                      float min_rho, float step, float damp, const OcState* st) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ne) return;
   rho[i] = oc_new_rho(sens[i], rho[i], float(st->g), min_rho, step, damp);
-}
-
-// Sensitivity filter: periodic Linear weights, s_e <- sum w s rho / (sum w * rho_e).
-struct OcFilterWeights {
-  int half, taps;
-  float w[13 * 13 * 13];
-};
-
-__global__ void __launch_bounds__(256) k_oc_filter(Dims d, const float* __restrict__ sens,
-                                                   const float* __restrict__ rho, size_t pitch, float* __restrict__ out,
-                                                   OcFilterWeights fw) {
-  const size_t nv = d.nv();
-  const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  const Coord3 c3_ = split3(v, d.nx, d.ny);
-    const int x = c3_.x, y = c3_.y, z = c3_.z;
-  const int h = fw.half, w1 = 2 * h + 1;
-  float sum = 0.f, ws = 0.f;
-  for (int t = 0; t < fw.taps; t++) {
-    const int ox = t % w1 - h, oy = (t / w1) % w1 - h, oz = t / (w1 * w1) - h;
-    const int px = ((x + ox) % d.nx + d.nx) % d.nx, py = ((y + oy) % d.ny + d.ny) % d.ny,
-              pz = ((z + oz) % d.nz + d.nz) % d.nz;
-    const size_t q = (size_t(py) + size_t(d.ny) * pz) * pitch + px;
-    const float w = fw.w[t];
-    sum += __ldg(sens + q) * __ldg(rho + q) * w;
-    ws += w;
-  }
-  const size_t e = (size_t(y) + size_t(d.ny) * z) * pitch + x;
-  out[v] = sum / (ws * __ldg(rho + e));
-}
-
-__global__ void __launch_bounds__(256) k_copy_pitched(Dims d, const float* __restrict__ src, float* dst,
-                                                      size_t pitch) {
-  const size_t nv = d.nv();
-  const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  const int x = int(v % d.nx);
-  dst[(v / d.nx) * pitch + x] = src[v];
 }
 
 }  // namespace otm
@@ -283,27 +213,12 @@ otm_status otm_oc_filter_sens(float* sens, const float* rho, size_t pitchT, cons
     set_error("filter radius must be in (0, 6.5)");
     return OTM_ERR_INVALID_ARGUMENT;
   }
-  OcFilterWeights fw;
-  fw.half = h;
-  fw.taps = (2 * h + 1) * (2 * h + 1) * (2 * h + 1);
-  float wsum = 0.f;
-  for (int t = 0; t < fw.taps; t++) {
-    const int ox = t % (2 * h + 1) - h, oy = t / (2 * h + 1) % (2 * h + 1) - h, oz = t / ((2 * h + 1) * (2 * h + 1)) - h;
-    const float q2 = float(ox * ox + oy * oy + oz * oz) / (radius * radius);
-    fw.w[t] = q2 < 1.f ? 1.f - std::sqrt(q2) : 0.f;  // WeightFunc<Linear>
-    wsum += fw.w[t];
-  }
-  for (int t = 0; t < fw.taps; t++) fw.w[t] /= wsum;
   cudaStream_t s = (cudaStream_t)stream;
   float* tmp = nullptr;
   OTM_CUDA(scratch_malloc((void**)&tmp, d.nv() * sizeof(float), s));
-  k_oc_filter<<<ceil_div(d.nv(), 256), 256, 0, s>>>(d, sens, rho, pitchT, tmp, fw);
-  k_copy_pitched<<<ceil_div(d.nv(), 256), 256, 0, s>>>(d, tmp, sens, pitchT);
-  cudaError_t e = cudaGetLastError();
+  const otm_status st = oc_filter_run(d, sens, rho, pitchT, tmp, radius, s);
   cudaFreeAsync(tmp, s);
-  if (e != cudaSuccess) return cuda_fail(e, "k_oc_filter");
-  count_launches(2);
-  return OTM_OK;
+  return st;
 }
 
 otm_status otm_oc_update(int ne, const float* sens, float* rho, float volratio, float min_rho, float step_limit,
