@@ -367,23 +367,28 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
   return OTM_OK;
 }
 
+// Dynamic shared memory of the sweeps on storage T.
+template <typename T>
+static otm_status sweep_attributes() {
+  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromZero, false, T, T>, a, int(kTileSmemSweep)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, false, T, T>, a, int(kTileSmemSweep)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, true, T, T>, a, int(kTileSmemSweep)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromUProlong, true, T, T>, a, int(kTileSmemProlong)));
+  return OTM_OK;
+}
+
 // Dynamic shared memory of the tile kernels (a per-function attribute of the current device; set
 // at every build, which is cheap) and the TMA map of the fine right-hand side: a 4-D tensor
 // {nx, ny, nz, 3 cases} of FP32 read in boxes {8, 8, 4, 3}, eight per tile.
 otm_status Homo::tile_attributes() {
   const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  OTM_TRY(sweep_attributes<float>());
+  OTM_TRY(sweep_attributes<__nv_bfloat16>());
+  OTM_TRY(sweep_attributes<__half>());
   OTM_CUDA(cudaFuncSetAttribute(k_tile_apply_dot, a, int(kTileSmemResid)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromZero, float, float>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, float, float>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromUProlong, float, float>, a, int(kTileSmemProlong)));
   OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<float, float>, a, int(kTileSmemResid)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromZero, __nv_bfloat16, __nv_bfloat16>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, __nv_bfloat16, __nv_bfloat16>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromUProlong, __nv_bfloat16, __nv_bfloat16>, a, int(kTileSmemProlong)));
   OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<__nv_bfloat16, __nv_bfloat16>, a, int(kTileSmemResid)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromZero, __half, __half>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, __half, __half>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromUProlong, __half, __half>, a, int(kTileSmemProlong)));
   OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<__half, __half>, a, int(kTileSmemResid)));
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
@@ -809,11 +814,14 @@ void Homo::vcycle_fine_tiled(const KT* k, VT* u, VT* r, const FineOp& fop, const
   const unsigned nt = tile_count(L.d);
   VT* buf[2] = {u, (VT*)u2};
   const int npre = cfg.pre_smooth, npost = cfg.post_smooth;
-  launch_pdl(k_tile_sweep<kFromZero, KT, VT>, dim3(nt), dim3(kSmoothThreads), kTileSmemSweep, stream, fmap, L.d, C.d,
-             k, fop, (const VT*)nullptr, (const float*)nullptr, buf[0], fs, 0, 0, sc);
+  auto sweep = [&](auto kern, size_t smem, const VT* in, const float* uc, VT* out, int shift) {
+    launch_pdl(kern, dim3(nt), dim3(kSmoothThreads), smem, stream, L.d, C.d, k, fop, in, uc, out, (const float*)L.f, fs,
+               shift, (const SolveScalars*)sc);
+  };
+  const float* none = nullptr;
+  sweep(k_tile_sweep<kFromZero, false, KT, VT>, kTileSmemSweep, nullptr, none, buf[0], 0);
   for (int s = 1; s < npre; s++)
-    launch_pdl(k_tile_sweep<kFromU, KT, VT>, dim3(nt), dim3(kSmoothThreads), kTileSmemSweep, stream, fmap, L.d, C.d,
-               k, fop, (const VT*)buf[(s - 1) & 1], (const float*)nullptr, buf[s & 1], fs, s & 1, 0, sc);
+    sweep(k_tile_sweep<kFromU, false, KT, VT>, kTileSmemSweep, buf[(s - 1) & 1], none, buf[s & 1], s & 1);
   VT* pre = buf[(npre - 1) & 1];
   launch_pdl(k_tile_resid<KT, VT>, dim3(nt), dim3(kResidThreads), kTileSmemResid, stream, fmap, L.d, k, fop,
              (const VT*)pre, r, fs, sc);
@@ -836,11 +844,9 @@ void Homo::vcycle_fine_tiled(const KT* k, VT* u, VT* r, const FineOp& fop, const
     VT* out = (s == npost - 1) ? r : (in == buf[0] ? buf[1] : buf[0]);
     const int shift = (npost - 1 - s) & 1;
     if (s == 0)
-      launch_pdl(k_tile_sweep<kFromUProlong, KT, VT>, dim3(nt), dim3(kSmoothThreads), kTileSmemProlong, stream, fmap,
-                 L.d, C.d, k, fop, (const VT*)in, (const float*)C.u, out, fs, shift, 1, sc);
+      sweep(k_tile_sweep<kFromUProlong, true, KT, VT>, kTileSmemProlong, in, C.u, out, shift);
     else
-      launch_pdl(k_tile_sweep<kFromU, KT, VT>, dim3(nt), dim3(kSmoothThreads), kTileSmemSweep, stream, fmap, L.d,
-                 C.d, k, fop, (const VT*)in, (const float*)nullptr, out, fs, shift, 1, sc);
+      sweep(k_tile_sweep<kFromU, true, KT, VT>, kTileSmemSweep, in, none, out, shift);
     in = out;
   }
   if (timed) cudaEventRecordWithFlags(prof_ev[1][prof_slot], stream, evflag);

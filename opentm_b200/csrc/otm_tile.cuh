@@ -11,16 +11,11 @@
 // (cx,cy,1) updated together because the cube element couples no vertices one edge apart); across
 // tile faces it is block Jacobi. Block Jacobi alone leaves the error that is constant inside each
 // tile and alternates in sign from tile to tile nearly undamped, so consecutive sweeps alternate
-// between two tilings, the second shifted by half a tile along every axis: the faces of one tiling
-// lie inside the tiles of the other. The first sweep after the coarse-grid correction adds the
+// between two tilings, the second shifted by half a tile along every axis: the faces of one
+// tiling lie inside the tiles of the other. The first sweep after the coarse-grid correction adds the
 // trilinear prolongation P u_c while it stages the tile. Pre-smoothing runs forward with the
 // tilings 0, 1, 0, ..., post-smoothing in the reverse pair order with the tilings mirrored, so the
 // V-cycle stays symmetric (the post leg is the transpose of the pre leg), as PCG needs.
-//
-// The tile's right-hand side (3 cases, FP32, 24 KB) arrives by TMA tensor copies
-// (cp.async.bulk.tensor of eight 4-D boxes {8, 8, 4, 3}, whose periodic origins a shifted tile
-// may wrap, completion on one mbarrier) issued at kernel entry, so it lands while the threads
-// stage the sites.
 //
 // Shared-memory layout of the sites: site (lx, ly, lz), lx, ly in [0, 18), lz in [0, 10), lies at
 // lz * 342 + ly * 19 + (lx odd ? 9 + lx / 2 : lx / 2): within a row the even and the odd sites are
@@ -28,10 +23,16 @@
 // float4, and rows are padded to 19 float4 so that the rows two apart, which the other lanes of a
 // warp read, start in other banks.
 //
-// A thread owns a column segment of 4 vertices of one colour pair and streams the 6 planes around
-// it: every staged plane is read once (8 neighbour sites + the own site's conductivity) and added
-// to the three vertices it couples to (the one above, the one in the plane, the one below), so a
-// vertex costs about 13 shared-memory loads instead of 28.
+// A thread owns a block of 2 x 2 x 4 vertices and keeps its values and conductivities in registers; in
+// the pass of colour pair (cx, cy) it updates the 4 vertices of one of its four columns, streaming the
+// 6 planes around them: of the 8 neighbour columns 3 are its own, so a plane costs 5 shared-memory
+// loads (8 in the two planes above and below the block). Every plane is read once and added to the
+// three vertices it couples to (the one above, the one in the plane, the one below). The right-hand
+// side is read from global memory into registers, two columns at a time, ahead of their passes, and
+// the results are written to global memory from registers. The sweep is bound by latency at 12 warps per
+// SM and by the shared-memory pipe; the registers take it from 54 site loads and 12 right-hand-side
+// loads per thread and pass to 37 site loads (7.9 -> 3.5 M shared-memory wavefronts per launch at 128^3)
+// and free the shared memory of a third CTA per SM.
 #pragma once
 
 #include <cuda.h>
@@ -60,14 +61,14 @@ static_assert(kTX * kTY == kResidThreads, "one thread per column");
 static_assert(kSeg == kFBZ && kTX == 2 * kFBX && kTY == 2 * kFBY && kTZ == 2 * kFBZ,
               "a column segment lies in one right-hand-side box along z; 2 x 2 x 2 boxes per tile");
 
-// Dynamic shared memory: [right-hand-side boxes][mbarrier][sites][coarse block], after rounding the
-// base up to 128 bytes (the TMA destination's alignment).
+// Dynamic shared memory of a sweep: [sites][coarse block]; of the residual and the direction update:
+// [right-hand-side boxes][mbarrier][sites], after rounding the base up to 128 bytes (the TMA
+// destination's alignment).
+constexpr size_t kTileSmemSweep = size_t(kSSites) * sizeof(float4);                         // 54,720 B
+constexpr size_t kTileSmemProlong = kTileSmemSweep + size_t(kCSites) * sizeof(float4);       // 64,320 B
 constexpr size_t kOffBar = size_t(kFElems) * sizeof(float);
 constexpr size_t kOffSites = kOffBar + 128;
-constexpr size_t kOffCoarse = kOffSites + size_t(kSSites) * sizeof(float4);
-constexpr size_t kTileSmemSweep = kOffCoarse + 128;                                      // 79,552 B
-constexpr size_t kTileSmemProlong = kOffCoarse + size_t(kCSites) * sizeof(float4) + 128;  // 89,152 B
-constexpr size_t kTileSmemResid = kOffCoarse + 128;
+constexpr size_t kTileSmemResid = kOffSites + size_t(kSSites) * sizeof(float4) + 128;        // 79,552 B
 constexpr uint32_t kFBytes = uint32_t(kFElems * sizeof(float));
 
 // Polls of the right-hand-side copy's mbarrier before a CTA gives up (each poll may suspend the
@@ -105,7 +106,7 @@ __device__ __forceinline__ int fpos(int x, int y, int z) {
   return ((x >> 3) + 2 * (y >> 3) + 4 * (z >> 2)) * kFBox + ((z & 3) * kFBY + (y & 7)) * kFBX + (x & 7);
 }
 
-// ---- the right-hand-side copy: TMA tensor loads completing on an mbarrier ---------------------
+// ---- the residual's right-hand-side copy: TMA tensor loads completing on an mbarrier -----------
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -202,6 +203,14 @@ __device__ __forceinline__ void st4(__half* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = q;
 }
 
+// 2 consecutive values (8 bytes in FP32, 4 bytes in 16-bit storage)
+__device__ __forceinline__ void st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void st2(__nv_bfloat16* p, float a, float b) {
+  *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
+}
+__device__ __forceinline__ void st2(__half* p, float a, float b) {
+  *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
+}
 // ---- coefficients ------------------------------------------------------------------------------
 // Coefficients of the 8 neighbour columns of a vertex for one element plane, from the 4
 // conductivities K[b] (b = bx + 2 by: the element whose lower corner is (x - 1 + bx, y - 1 + by)
@@ -246,46 +255,61 @@ __device__ __forceinline__ void sub_inplane(float (&acc)[3], const float (&Kb)[4
   }
 }
 
-// One colour-pair pass (PX, PY) over the tile's interior: every thread updates the 4 vertices
-// (lx, ly, lz0 .. lz0 + 3) of its column segment, reading planes lz0 - 1 .. lz0 + 4. fsm holds the
-// staged right-hand side (see fpos), fs the per-case scale applied to it.
-template <int PX, int PY>
-__device__ __forceinline__ void tile_pass(float4* sm, const float* fsm, const FineOp& op, const float (&fs)[3]) {
-  const int t = int(threadIdx.x);
-  const int i = t & 7, j = (t >> 3) & 7, seg = t >> 6;
-  const int lx = 2 * i + 1 + PX, ly = 2 * j + 1 + PY, lz0 = 1 + kSeg * seg;
+// The block of vertices a thread owns: column PX + 2 PY, plane q.
+struct TileBlock {
+  float u[4][kSeg][3];
+  float k[4][kSeg];
+};
+
+// The right-hand side of the two columns of row PY of the own block (both PX), from global memory.
+struct TileRhs {
+  float2 v[kSeg][3];
+};
+
+// One colour-pair pass (PX, PY): the thread updates the vertices of its column (PX, PY), planes
+// lz0 .. lz0 + 3 (lz0 = 1 + 4 seg), reading planes lz0 - 1 .. lz0 + 4. fs: the per-case scale of the
+// right-hand side. kLast: no pass follows, so the values stay in registers.
+template <int PX, int PY, bool kLast>
+__device__ __forceinline__ void tile_pass(float4* sm, TileBlock& own, const TileRhs& rhs, const FineOp& op,
+                                          const float (&fs)[3], int lx, int ly, int lz0) {
+  constexpr int kCol = PX + 2 * PY;
   // positions of the left / right neighbour columns relative to the own site: the parity of lx
   // is fixed by the pass, so they are compile-time offsets in the parity-split row
   constexpr int oL = PX ? kSHalf - 1 : -kSHalf, oR = PX ? kSHalf : -kSHalf + 1;
-  const float* fcol = fsm + fpos(lx - 1, ly - 1, lz0 - 1);  // vertex q of the segment: + q * 64
+  constexpr int dxn[8] = {-1, 0, 1, -1, 1, -1, 0, 1}, dyn[8] = {-1, -1, -1, 0, 0, 1, 1, 1};
+  const float4* col = sm + tsite(lx + PX, ly + PY, lz0 - 1);
   float Kp[4] = {0.f, 0.f, 0.f, 0.f};  // conductivities of the previous plane
   PlaneCoef Cp;                        // coefficients of the previous plane
   float accA[3] = {0.f, 0.f, 0.f}, accB[3] = {0.f, 0.f, 0.f}, accC[3] = {0.f, 0.f, 0.f};  // P-1, P, P+1
   float dA = 0.f, dB = 0.f;  // their conductivity sums so far
 #pragma unroll
-  for (int s = 0; s < kSeg + 2; s++) {
-    const int P = lz0 - 1 + s;
-    const float4* b = sm + tsite(lx, ly, P);
+  for (int s = 0; s < kSeg + 2; s++) {  // plane P = lz0 - 1 + s
+    const float4* b = col + s * kSPlane;
     float4 nb[8];
-    nb[0] = b[oL - kSRow];
-    nb[1] = b[-kSRow];
-    nb[2] = b[oR - kSRow];
-    nb[3] = b[oL];
-    nb[4] = b[oR];
-    nb[5] = b[oL + kSRow];
-    nb[6] = b[kSRow];
-    nb[7] = b[oR + kSRow];
-    const float kown = reinterpret_cast<const float*>(b)[3];
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+      const int cx = PX + dxn[n], cy = PY + dyn[n];
+      if (s >= 1 && s <= kSeg && cx >= 0 && cx <= 1 && cy >= 0 && cy <= 1) {
+        const int c = cx + 2 * cy;
+        nb[n] = make_float4(own.u[c][s - 1][0], own.u[c][s - 1][1], own.u[c][s - 1][2], own.k[c][s - 1]);
+      } else {
+        nb[n] = b[(dxn[n] < 0 ? oL : (dxn[n] > 0 ? oR : 0)) + dyn[n] * kSRow];
+      }
+    }
+    float kown = 0.f;
+    if (s >= 1 && s <= kSeg)
+      kown = own.k[kCol][s - 1];
+    else if (s == 0)
+      kown = reinterpret_cast<const float*>(b)[3];
     const float K[4] = {nb[0].w, nb[1].w, nb[3].w, kown};
     const float sK = (K[0] + K[1]) + (K[2] + K[3]);
     PlaneCoef C;
-    C.make(K, op);
+    if (s <= kSeg) C.make(K, op);
     // vertex P + 1 (segment index s): its lower element plane is P
     float dC = 0.f;
     if (s < kSeg) {
-      const float* fv = fcol + s * (kFBX * kFBY);
 #pragma unroll
-      for (int c = 0; c < 3; c++) accC[c] = fv[c * kFCase] * fs[c];
+      for (int c = 0; c < 3; c++) accC[c] = (PX ? rhs.v[s][c].y : rhs.v[s][c].x) * fs[c];
       sub_plane(accC, C, nb);
       dC = sK;
     }
@@ -298,12 +322,11 @@ __device__ __forceinline__ void tile_pass(float4* sm, const float* fsm, const Fi
     if (s >= 2) {
       sub_plane(accA, Cp, nb);
       const float inv = 1.0f / (op.c0 * dA);
-      float4 o;
-      o.x = accA[0] * inv;
-      o.y = accA[1] * inv;
-      o.z = accA[2] * inv;
-      o.w = Kp[3];  // own element of plane P - 1
-      sm[tsite(lx, ly, P - 1)] = o;
+#pragma unroll
+      for (int c = 0; c < 3; c++) own.u[kCol][s - 2][c] = accA[c] * inv;
+      if (!kLast)
+        sm[tsite(lx + PX, ly + PY, lz0 + s - 2)] =
+            make_float4(own.u[kCol][s - 2][0], own.u[kCol][s - 2][1], own.u[kCol][s - 2][2], own.k[kCol][s - 2]);
     }
     // rotate: P becomes P - 1, P + 1 becomes P
 #pragma unroll
@@ -506,28 +529,51 @@ __device__ __forceinline__ unsigned char* tile_smem_base() {
 // trilinear prolongation of the coarse correction (the first post-smoothing sweep).
 enum TileStart { kFromZero = 0, kFromU = 1, kFromUProlong = 2 };
 
+// The right-hand side of row PY of the own block (its two columns), from global memory.
+template <int PY>
+__device__ __forceinline__ void tile_rhs(const Dims& d, const float* __restrict__ f, int X, const int (&Y)[2],
+                                         const int (&Z)[kSeg], TileRhs& rhs) {
+  const size_t nv = d.nv();
+#pragma unroll
+  for (int q = 0; q < kSeg; q++) {
+    const float* p = f + size_t(X) + size_t(d.nx) * (size_t(Y[PY]) + size_t(d.ny) * Z[q]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) rhs.v[q][c] = __ldg(reinterpret_cast<const float2*>(p + c * nv));
+  }
+}
+
 // One Gauss-Seidel sweep of the fine level on the tiles of tiling `shift` (see above): the tile is
 // staged from the start values (kStart), the four colour-pair passes run in the order 0,1,2,3, or
-// 3,2,1,0 when `reverse`, and the interior goes to u_out, which must not alias u_in. ks: fine
-// conductivity (storage KT); fmap: TMA map of the right-hand side (FP32, 3 cases, scaled per case
-// by fscale when given); u_in / u_out in storage VT; uc: the coarse correction (FP32, kFromUProlong,
+// 3,2,1,0 when kReverse, and the interior goes to u_out, which must not alias u_in. ks: fine
+// conductivity (storage KT); f: the right-hand side (FP32, 3 cases, scaled per case by fscale when
+// given); u_in / u_out in storage VT; uc: the coarse correction (FP32, kFromUProlong,
 // homogenization/grid.cu:881-940); arithmetic and shared memory FP32.
-template <int kStart, typename KT, typename VT>
-__global__ void __launch_bounds__(kSmoothThreads, 2)
-    k_tile_sweep(const __grid_constant__ CUtensorMap fmap, Dims d, Dims dc, const KT* __restrict__ ks, FineOp op,
-                 const VT* __restrict__ u_in, const float* __restrict__ uc, VT* __restrict__ u_out,
-                 const double* fscale, int shift, int reverse, SolveScalars* sc) {
-  unsigned char* base = tile_smem_base();
-  float* fsm = reinterpret_cast<float*>(base);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base + kOffBar);
-  float4* sm = reinterpret_cast<float4*>(base + kOffSites);
-  float4* cb = reinterpret_cast<float4*>(base + kOffCoarse);
-  pdl_wait();
-  if (sc && solve_done(sc)) return;
+// Per launch at 128^3 (from zero, from u, prolonging): 33.8 / 38.3 / 64.3 us; with the right-hand side
+// and the own block read from shared memory in every pass, 2 CTAs per SM: 45.7 / 55.2 / 82.1 us. At
+// two CTAs per SM (no spills, 190-226 registers) the 128^3 and 256^3 solves are 2% slower than at three.
+template <int kStart, bool kReverse, typename KT, typename VT>
+__global__ void __launch_bounds__(kSmoothThreads, 3)
+    k_tile_sweep(Dims d, Dims dc, const KT* __restrict__ ks, FineOp op, const VT* __restrict__ u_in,
+                 const float* __restrict__ uc, VT* __restrict__ u_out, const float* __restrict__ f,
+                 const double* fscale, int shift, const SolveScalars* sc) {
+  extern __shared__ float4 sweep_sm[];
+  float4* sm = sweep_sm;
+  float4* cb = sweep_sm + kSSites;
+  const int t = int(threadIdx.x);
   int x0, y0, z0;
   tile_origin(d, blockIdx.x, shift, x0, y0, z0);
-  const size_t nv = d.nv();
-  tile_f_copy_start(&fmap, fsm, bar, d, x0, y0, z0);
+  // the own block: 2 x 2 columns from (lx, ly), planes lz0 .. lz0 + 3
+  const int lx = 2 * (t & 7) + 1, ly = 2 * ((t >> 3) & 7) + 1, lz0 = 1 + kSeg * (t >> 6);
+  const int X = wrapm(x0 + lx - 1, d.nx);
+  int Y[2], Z[kSeg];
+#pragma unroll
+  for (int e = 0; e < 2; e++) Y[e] = wrapm(y0 + ly - 1 + e, d.ny);
+#pragma unroll
+  for (int q = 0; q < kSeg; q++) Z[q] = wrapm(z0 + lz0 - 1 + q, d.nz);
+  pdl_wait();
+  if (sc && solve_done(sc)) return;
+  TileRhs rhs;
+  tile_rhs<kReverse ? 1 : 0>(d, f, X, Y, Z, rhs);
   float fs[3] = {1.f, 1.f, 1.f};
   if (fscale)
 #pragma unroll
@@ -535,46 +581,44 @@ __global__ void __launch_bounds__(kSmoothThreads, 2)
   stage_tile<kStart != kFromZero, kSmoothThreads, true>(d, dc, x0, y0, z0, ks, u_in,
                                                         kStart == kFromUProlong ? uc : nullptr, sm, cb);
   __syncthreads();
-  if (!tile_f_copy_wait(bar, sc)) return;
-  if (!reverse) {
-    tile_pass<0, 0>(sm, fsm, op, fs);
-    __syncthreads();
-    tile_pass<1, 0>(sm, fsm, op, fs);
-    __syncthreads();
-    tile_pass<0, 1>(sm, fsm, op, fs);
-    __syncthreads();
-    tile_pass<1, 1>(sm, fsm, op, fs);
-  } else {
-    tile_pass<1, 1>(sm, fsm, op, fs);
-    __syncthreads();
-    tile_pass<0, 1>(sm, fsm, op, fs);
-    __syncthreads();
-    tile_pass<1, 0>(sm, fsm, op, fs);
-    __syncthreads();
-    tile_pass<0, 0>(sm, fsm, op, fs);
-  }
-  __syncthreads();
-  // interior to global memory, 4 consecutive x at a time
-  for (int w = int(threadIdx.x); w < kTX * kTY * kTZ / 4; w += kSmoothThreads) {
-    const int q = w & 3, row = w >> 2;
-    const int ly = 1 + row % kTY, lz = 1 + row / kTY;
-    float o0[4], o1[4], o2[4];
+  TileBlock own;
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const float4 v = sm[tsite(1 + 4 * q + e, ly, lz)];
-      o0[e] = v.x, o1[e] = v.y, o2[e] = v.z;
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int q = 0; q < kSeg; q++) {
+      const float4 v = sm[tsite(lx + (c & 1), ly + (c >> 1), lz0 + q)];
+      own.u[c][q][0] = v.x;
+      own.u[c][q][1] = v.y;
+      own.u[c][q][2] = v.z;
+      own.k[c][q] = v.w;
     }
-    const size_t g = size_t(wrapm(x0 + 4 * q, d.nx)) +
-                     size_t(d.nx) * (size_t(wrapm(y0 + ly - 1, d.ny)) + size_t(d.ny) * size_t(wrapm(z0 + lz - 1, d.nz)));
-    st4(u_out + g, o0);
-    st4(u_out + nv + g, o1);
-    st4(u_out + 2 * nv + g, o2);
-  }
+  // two passes on one row of columns, the other row's right-hand side fetched before the second
+  TileRhs rhs2;
+  constexpr int PA = kReverse ? 1 : 0, PB = 1 - PA;
+  tile_pass<PA, PA, false>(sm, own, rhs, op, fs, lx, ly, lz0);
+  __syncthreads();
+  tile_rhs<PB>(d, f, X, Y, Z, rhs2);
+  tile_pass<PB, PA, false>(sm, own, rhs, op, fs, lx, ly, lz0);
+  __syncthreads();
+  tile_pass<PA, PB, false>(sm, own, rhs2, op, fs, lx, ly, lz0);
+  __syncthreads();
+  tile_pass<PB, PB, true>(sm, own, rhs2, op, fs, lx, ly, lz0);
+  const size_t nv = d.nv();
+#pragma unroll
+  for (int q = 0; q < kSeg; q++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const size_t g = size_t(X) + size_t(d.nx) * (size_t(Y[e]) + size_t(d.ny) * Z[q]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) st2(u_out + c * nv + g, own.u[2 * e][q][c], own.u[2 * e + 1][q][c]);
+    }
 }
 
 // r = f - A u on the fine level for every vertex of a tile (tiling 0), from a staged tile with its
 // halo (natural site order here: lanes take consecutive sites of a row). A thread owns one column
-// of the tile and streams its 10 planes.
+// of the tile and streams its 10 planes. The right-hand side (3 cases, FP32, 24 KB) arrives by TMA
+// (cp.async.bulk.tensor of eight 4-D boxes {8, 8, 4, 3}, completion on one mbarrier), issued at kernel
+// entry so that it lands while the threads stage the sites.
 template <typename KT, typename VT>
 __global__ void __launch_bounds__(kResidThreads, 2)
     k_tile_resid(const __grid_constant__ CUtensorMap fmap, Dims d, const KT* __restrict__ ks, FineOp op,
