@@ -6,8 +6,13 @@
 // needs (sums with a fixed-order last-block finalisation, maxima). A Newton step is two passes:
 // the step bounds of the direction, then the line-search trial, which recomputes the direction,
 // writes the trial point to spare arrays and reduces both the residual there and the next Newton
-// system (accepting the step swaps the arrays). The (m+1) x (m+1) KKT system (m <= 8) is solved
-// in FP64 on the host, where the reference used Eigen.
+// system (accepting the step swaps the arrays). The dual variables, the (m+1) x (m+1) KKT system
+// (m <= 8, where the reference used Eigen on the host) and every decision of the interior-point
+// iteration live on the device: the last block of a pass takes the step that the pass was for and
+// says which pass comes next (MmaState), so the host only queues passes and looks once in a while
+// whether the subproblem is solved. A pass queued for another step than the one that is due returns
+// at once. When epsi falls, the residual and the Newton system at the same point follow from the
+// sums of the pass before (they are polynomials in epsi), without another pass.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,12 +41,39 @@ struct MmaWork {
   double *alfa = nullptr, *beta = nullptr, *p0 = nullptr, *q0 = nullptr, *P = nullptr, *Q = nullptr;
   double *xs = nullptr, *xsi = nullptr, *eta = nullptr, *dx = nullptr, *dxsi = nullptr, *deta = nullptr;
   double* partials = nullptr;  // kMaxPartials * 96
-  double* result = nullptr;    // 96
+  double* result = nullptr;    // kMmaSlots
   unsigned int* counter = nullptr;
-  double* host = nullptr;      // pinned, 96
+  struct MmaState* state = nullptr;
+  int* host = nullptr;         // pinned copy of the state's mode and error
 };
 
-constexpr int kMmaSlots = 128;  // >= 2 + 3 m + m^2 for m <= 8
+constexpr int kMmaSlots = 128;  // >= 5 + 3 m + m^2 for m <= 8
+
+// The pass that is due: the residual at the start point, the step bounds of a direction, a line-search
+// trial, nothing any more.
+enum MmaMode { kMmaInit = 0, kMmaDirmax = 1, kMmaTrial = 2, kMmaDone = 3 };
+enum MmaError { kMmaOk = 0, kMmaSingular = 1, kMmaNanStep = 2 };
+
+// Constants of a subproblem on the host side of a step (a0, a, c, d and the constraint values).
+struct MmaProblem {
+  double a0, a[kMmaMaxM], c[kMmaMaxM], d[kMmaMaxM], g[kMmaMaxM];
+};
+
+// The interior-point iteration on the device (subsolv, optimization/mmaOpt.cu:429-830): the dual and
+// slack variables, their direction and line-search base, the sums of the last trial, and what is due.
+struct MmaState {
+  int mode, err;  // first: copied to the host together
+  int parity;     // 1: the committed point is in the spare arrays
+  int ittt, itto;
+  MmaProblem pr;
+  double n, b[kMmaMaxM];
+  double y[kMmaMaxM], lam[kMmaMaxM], mu[kMmaMaxM], s[kMmaMaxM], z, zet, epsi;
+  double dy[kMmaMaxM], dl[kMmaMaxM], dmu[kMmaMaxM], ds[kMmaMaxM], dz, dzet;
+  double yo[kMmaMaxM], lo[kMmaMaxM], muo[kMmaMaxM], so[kMmaMaxM], zo, zeto;
+  double steg, residunorm, residumax;
+  // the last trial: sums and maxima over the variables (see k_mma_trial)
+  double n2, tsum, gvec[kMmaMaxM], gd[kMmaMaxM], gs[kMmaMaxM], gg[kMmaMaxM * kMmaMaxM], mrex, mab, nab;
+};
 
 template <int NM>
 __device__ __forceinline__ void block_reduce_max(double (&v)[NM], double* smem) {
@@ -67,9 +99,10 @@ __device__ __forceinline__ void block_reduce_max(double (&v)[NM], double* smem) 
   }
 }
 
-// Block partials of NS sums and NM maxima, then the last block writes result[0..NS+NM).
+// Block partials of NS sums and NM maxima, then the last block writes result[0..NS+NM); true in the
+// threads of that block, where the results can be read.
 template <int NS, int NM>
-__device__ __forceinline__ void reduce_to_result(double (&s)[NS], double (&mx)[NM], double* partials,
+__device__ __forceinline__ bool reduce_to_result(double (&s)[NS], double (&mx)[NM], double* partials,
                                                  double* result, unsigned int* counter) {
   __shared__ double smem[32 * (NS > NM ? NS : NM)];
   block_reduce_f64<NS>(s, smem);
@@ -100,24 +133,240 @@ __device__ __forceinline__ void reduce_to_result(double (&s)[NS], double (&mx)[N
     }
     __syncthreads();
     if (threadIdx.x == 0) *counter = 0;
+    return true;
   }
+  return false;
+}
+
+// std::max's rule for NaN (the second argument is taken only if it is greater).
+__device__ __forceinline__ double later_max(double a, double b) { return a < b ? b : a; }
+
+// Dense N x N solve with partial pivoting (replaces Eigen ColPivHouseholderQR, mmaOpt.cpp:48-73).
+template <int N>
+__device__ bool dense_solve(double (&A)[N][N], double (&b)[N]) {
+  for (int k = 0; k < N; k++) {
+    int p = k;
+    for (int i = k + 1; i < N; i++)
+      if (fabs(A[i][k]) > fabs(A[p][k])) p = i;
+    if (A[p][k] == 0.0) return false;
+    if (p != k) {
+      for (int j = 0; j < N; j++) {
+        const double t = A[k][j];
+        A[k][j] = A[p][j];
+        A[p][j] = t;
+      }
+      const double t = b[k];
+      b[k] = b[p];
+      b[p] = t;
+    }
+    for (int i = k + 1; i < N; i++) {
+      const double l = A[i][k] / A[k][k];
+      for (int j = k; j < N; j++) A[i][j] -= l * A[k][j];
+      b[i] -= l * b[k];
+    }
+  }
+  for (int i = N - 1; i >= 0; i--) {
+    double t = b[i];
+    for (int j = i + 1; j < N; j++) t -= A[i][j] * b[j];
+    b[i] = t / A[i][i];
+  }
+  return true;
+}
+
+// Residual norm and largest entry at the last trial's point with the current epsi: the variables' part
+// from its sums, the duals' part here.
+template <int M>
+__device__ void mma_residual(MmaState& S, double* norm, double* mx) {
+  const MmaProblem& P = S.pr;
+  double n2 = S.n2, m = later_max(later_max(S.mrex, S.mab - S.epsi), S.nab + S.epsi), ad = 0.0;
+  auto acc = [&](double r) {
+    n2 += r * r;
+    m = later_max(m, fabs(r));
+  };
+  for (int i = 0; i < M; i++) ad += P.a[i] * S.lam[i];
+  for (int i = 0; i < M; i++) acc(P.c[i] + P.d[i] * S.y[i] - S.mu[i] - S.lam[i]);
+  acc(P.a0 - S.zet - ad);
+  for (int i = 0; i < M; i++) acc(S.gvec[i] - P.a[i] * S.z - S.y[i] + S.s[i] - S.b[i]);
+  for (int i = 0; i < M; i++) acc(S.mu[i] * S.y[i] - S.epsi);
+  acc(S.zet * S.z - S.epsi);
+  for (int i = 0; i < M; i++) acc(S.lam[i] * S.s[i] - S.epsi);
+  *norm = sqrt(n2);
+  *mx = m;
+}
+
+// The sums of the last trial, from its result (see k_mma_trial).
+template <int M>
+__device__ void mma_take(MmaState& S, const double* r) {
+  S.n2 = r[0];
+  S.tsum = r[1];
+  for (int i = 0; i < M; i++) {
+    S.gvec[i] = r[2 + i];
+    S.gd[i] = r[2 + M + i];
+    S.gs[i] = r[2 + 2 * M + i];
+    for (int k = 0; k < M; k++) S.gg[i * M + k] = r[2 + 3 * M + i * M + k];
+  }
+  const double* x = r + 2 + 3 * M + M * M;
+  S.mrex = x[0];
+  S.mab = x[1];
+  S.nab = x[2];
+}
+
+// The trial point's duals for the step S.steg; the next pass is a trial there.
+template <int M>
+__device__ void mma_next_trial(MmaState& S) {
+  S.itto++;
+  for (int i = 0; i < M; i++) {
+    S.y[i] = S.yo[i] + S.steg * S.dy[i];
+    S.lam[i] = S.lo[i] + S.steg * S.dl[i];
+    S.mu[i] = S.muo[i] + S.steg * S.dmu[i];
+    S.s[i] = S.so[i] + S.steg * S.ds[i];
+  }
+  S.z = S.zo + S.steg * S.dz;
+  S.zet = S.zeto + S.steg * S.dzet;
+  S.mode = kMmaTrial;
+}
+
+// At a committed point: the next Newton direction of the duals, or the next epsi, or the end.
+template <int M>
+__device__ void mma_advance(MmaState& S) {
+  const MmaProblem& P = S.pr;
+  while (!(S.residumax > 0.9 * S.epsi && S.ittt < 200)) {
+    const double e0 = S.epsi;
+    S.epsi = 0.1 * e0;
+    if (!(S.epsi > kEpsiMin)) {
+      S.mode = kMmaDone;
+      return;
+    }
+    // the same point with the smaller epsi: the entries a - epsi and b - epsi of the residual move by
+    // de, and so does the epsi part of delx
+    const double de = e0 - S.epsi;
+    S.n2 += 2.0 * de * S.tsum + 2.0 * S.n * de * de;
+    S.tsum += 2.0 * S.n * de;
+    for (int i = 0; i < M; i++) S.gd[i] += de * S.gs[i];
+    S.ittt = 0;
+    mma_residual<M>(S, &S.residunorm, &S.residumax);
+  }
+  S.ittt++;
+  double adl = 0.0;
+  for (int i = 0; i < M; i++) adl += P.a[i] * S.lam[i];
+  const double delz = P.a0 - adl - S.epsi / S.z;
+  double AA[M + 1][M + 1], bb[M + 1], dely[M], diagy[M];
+  for (int i = 0; i < M; i++) {
+    dely[i] = P.c[i] + P.d[i] * S.y[i] - S.lam[i] - S.epsi / S.y[i];
+    const double dellam = S.gvec[i] - P.a[i] * S.z - S.y[i] - S.b[i] + S.epsi / S.lam[i];
+    diagy[i] = P.d[i] + S.mu[i] / S.y[i];
+    bb[i] = dellam + dely[i] / diagy[i] - S.gd[i];
+    for (int k = 0; k < M; k++) AA[i][k] = S.gg[i * M + k];
+    AA[i][i] += S.s[i] / S.lam[i] + 1.0 / diagy[i];
+    AA[i][M] = P.a[i];
+    AA[M][i] = P.a[i];
+  }
+  AA[M][M] = -S.zet / S.z;
+  bb[M] = delz;
+  if (!dense_solve<M + 1>(AA, bb)) {
+    S.err = kMmaSingular;
+    S.mode = kMmaDone;
+    return;
+  }
+  S.dz = bb[M];
+  for (int i = 0; i < M; i++) {
+    S.dl[i] = bb[i];
+    S.dy[i] = -dely[i] / diagy[i] + bb[i] / diagy[i];
+    S.dmu[i] = -S.mu[i] + S.epsi / S.y[i] - (S.mu[i] * S.dy[i]) / S.y[i];
+    S.ds[i] = -S.s[i] + S.epsi / S.lam[i] - (S.s[i] * bb[i]) / S.lam[i];
+    S.lo[i] = S.lam[i];
+  }
+  S.dzet = -S.zet + S.epsi / S.z - S.zet * S.dz / S.z;
+  S.mode = kMmaDirmax;
+}
+
+// After the step-bound pass: the line search's first step.
+template <int M>
+__device__ void mma_after_dirmax(MmaState& S, const double* r) {
+  double stm = later_max(r[1], r[2]);  // xsi, eta parts
+  for (int i = 0; i < M; i++) {
+    stm = later_max(stm, -1.01 * S.dy[i] / S.y[i]);
+    stm = later_max(stm, -1.01 * S.dl[i] / S.lam[i]);
+    stm = later_max(stm, -1.01 * S.dmu[i] / S.mu[i]);
+    stm = later_max(stm, -1.01 * S.ds[i] / S.s[i]);
+  }
+  stm = later_max(stm, -1.01 * S.dz / S.z);
+  stm = later_max(stm, -1.01 * S.dzet / S.zet);
+  const double stmalbe = later_max(r[3], r[4]);
+  S.steg = 1.0 / later_max(later_max(stmalbe, stm), 1.0);
+  if (isnan(S.steg)) {
+    S.err = kMmaNanStep;
+    S.mode = kMmaDone;
+    return;
+  }
+  for (int i = 0; i < M; i++) {
+    S.yo[i] = S.y[i];
+    S.muo[i] = S.mu[i];
+    S.so[i] = S.s[i];
+  }
+  S.zo = S.z;
+  S.zeto = S.zet;
+  S.itto = 0;
+  mma_next_trial<M>(S);
+}
+
+// After a trial (or the residual of the start point): accept it or halve the step.
+template <int M>
+__device__ void mma_after_trial(MmaState& S, const double* r) {
+  mma_take<M>(S, r);
+  double norm, mx;
+  mma_residual<M>(S, &norm, &mx);
+  if (S.mode == kMmaTrial) {
+    S.steg /= 2;
+    if (norm > S.residunorm && S.itto < 50) {
+      mma_next_trial<M>(S);
+      return;
+    }
+    S.parity ^= 1;  // the last point tried, as the reference commits after its line search
+  }
+  S.residunorm = norm;
+  S.residumax = mx;
+  mma_advance<M>(S);
+}
+
+// The start of a subproblem: constraint offsets sums[i] = sum_j P/ux + Q/xl from the set-up pass.
+template <int M>
+__device__ void mma_start(MmaState& S, const MmaProblem& pr, double n, const double* sums) {
+  S.mode = kMmaInit;
+  S.err = kMmaOk;
+  S.parity = S.ittt = S.itto = 0;
+  S.pr = pr;
+  S.n = n;
+  for (int i = 0; i < M; i++) {
+    S.b[i] = sums[i] - pr.g[i];
+    S.y[i] = S.lam[i] = S.s[i] = 1.0;
+    S.mu[i] = later_max(0.5 * pr.c[i], 1.0);
+    S.dl[i] = S.lo[i] = 0.0;
+  }
+  S.z = S.zet = S.epsi = 1.0;
+  S.steg = 0.0;
 }
 
 // Asymptotes, move limits, approximation coefficients p0, q0, P, Q, the constraint offsets
 // sum_j P/ux + Q/xl, and the subsolver's starting point (mmasub_ker, optimization/mmaOpt.cu:834-1019).
-template <int M>
-__global__ void __launch_bounds__(256) k_mma_setup(size_t n, int itn, const double* __restrict__ xvar,
-                                                   const double* __restrict__ xmin, const double* __restrict__ xmax,
-                                                   const double* __restrict__ xold1,
-                                                   const double* __restrict__ xold2, const double* __restrict__ df0dx,
-                                                   const double* __restrict__ dgdx, size_t ldg, double* low,
-                                                   double* upp, double move, MmaWork w) {
+// The inputs are FP64 or FP32 (T); xvar_out, if given, receives x in FP64.
+template <typename T>
+struct MmaInputs {
+  const T *x, *df0dx, *dgdx[kMmaMaxM];
+  double* xvar_out;
+};
+template <int M, typename T>
+__global__ void __launch_bounds__(256) k_mma_setup(size_t n, int itn, MmaInputs<T> in, const double* __restrict__ xmin,
+                                                   const double* __restrict__ xmax, const double* __restrict__ xold1,
+                                                   const double* __restrict__ xold2, double* low, double* upp,
+                                                   double move, MmaProblem pr, MmaWork w) {
   double bs[M];
   double dummy[1] = {-1e300};
 #pragma unroll
   for (int i = 0; i < M; i++) bs[i] = 0.0;
   for (size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += size_t(gridDim.x) * blockDim.x) {
-    const double x = xvar[j], dxr = xmax[j] - xmin[j];
+    const double x = double(in.x[j]), dxr = xmax[j] - xmin[j], df = double(in.df0dx[j]);
+    if (in.xvar_out) in.xvar_out[j] = x;
     double lo, up;
     if (itn <= 2) {
       lo = x - kAsyInit * dxr;
@@ -138,13 +387,13 @@ __global__ void __launch_bounds__(256) k_mma_setup(size_t n, int itn, const doub
     w.beta[j] = be;
     const double xmamiinv = 1.0 / fmax(dxr, 1e-5);
     const double ux1 = up - x, xl1 = x - lo, ux2 = ux1 * ux1, xl2 = xl1 * xl1;
-    const double dp = fmax(df0dx[j], 0.0), dm = fmax(-df0dx[j], 0.0);
+    const double dp = fmax(df, 0.0), dm = fmax(-df, 0.0);
     const double pq0 = 1e-3 * (dp + dm) + kRaa0 * xmamiinv;
     w.p0[j] = (dp + pq0) * ux2;
     w.q0[j] = (dm + pq0) * xl2;
 #pragma unroll
     for (int i = 0; i < M; i++) {
-      const double g = dgdx[i * ldg + j];
+      const double g = double(in.dgdx[i][j]);
       const double pp = fmax(g, 0.0), qq = fmax(-g, 0.0);
       const double pq = 1e-3 * (pp + qq) + kRaa0 * xmamiinv;
       const double Pij = (pp + pq) * ux2, Qij = (qq + pq) * xl2;
@@ -156,11 +405,9 @@ __global__ void __launch_bounds__(256) k_mma_setup(size_t n, int itn, const doub
     w.xs[j] = xs;
     w.xsi[j] = fmax(1.0 / (xs - al), 1.0);
     w.eta[j] = fmax(1.0 / (be - xs), 1.0);
-    w.dx[j] = 0.0;
-    w.dxsi[j] = 0.0;
-    w.deta[j] = 0.0;
   }
-  reduce_to_result<M, 1>(bs, dummy, w.partials, w.result, w.counter);
+  if (reduce_to_result<M, 1>(bs, dummy, w.partials, w.result, w.counter) && threadIdx.x == 0)
+    mma_start<M>(*w.state, pr, double(n), w.result);
 }
 
 // The per-variable data a subsolver pass reads: the point, its bounds and the approximation.
@@ -169,12 +416,20 @@ struct MmaElem {
   double x, xsi, eta, low, upp, al, be, p0, q0, P[M], Q[M];
 };
 
+// The committed point and the other one, by the state's parity.
+struct MmaPoint {
+  double *x, *xsi, *eta;
+};
+__device__ __forceinline__ MmaPoint mma_point(const MmaWork& w, bool spare) {
+  return spare ? MmaPoint{w.dx, w.dxsi, w.deta} : MmaPoint{w.xs, w.xsi, w.eta};
+}
+
 template <int M>
-__device__ __forceinline__ void load_elem(const MmaWork& w, const double* __restrict__ low,
+__device__ __forceinline__ void load_elem(const MmaWork& w, const MmaPoint& pt, const double* __restrict__ low,
                                           const double* __restrict__ upp, size_t j, MmaElem<M>& e) {
-  e.x = w.xs[j];
-  e.xsi = w.xsi[j];
-  e.eta = w.eta[j];
+  e.x = pt.x[j];
+  e.xsi = pt.xsi[j];
+  e.eta = pt.eta[j];
   e.low = low[j];
   e.upp = upp[j];
   e.al = w.alfa[j];
@@ -191,16 +446,16 @@ __device__ __forceinline__ void load_elem(const MmaWork& w, const double* __rest
 // Elements j and j + 1 (j even; n even and every array 16-byte aligned): one 16-byte load per
 // array, twice the bytes in flight per instruction.
 template <int M>
-__device__ __forceinline__ void load_pair(const MmaWork& w, const double* __restrict__ low,
+__device__ __forceinline__ void load_pair(const MmaWork& w, const MmaPoint& pt, const double* __restrict__ low,
                                           const double* __restrict__ upp, size_t j, MmaElem<M>& a, MmaElem<M>& b) {
   auto ld = [j](const double* p, double& u, double& v) {
     const double2 t = *reinterpret_cast<const double2*>(p + j);
     u = t.x;
     v = t.y;
   };
-  ld(w.xs, a.x, b.x);
-  ld(w.xsi, a.xsi, b.xsi);
-  ld(w.eta, a.eta, b.eta);
+  ld(pt.x, a.x, b.x);
+  ld(pt.xsi, a.xsi, b.xsi);
+  ld(pt.eta, a.eta, b.eta);
   ld(low, a.low, b.low);
   ld(upp, a.upp, b.upp);
   ld(w.alfa, a.al, b.al);
@@ -246,17 +501,27 @@ __device__ __forceinline__ void mma_dir(const MmaElem<M>& e, const MVec& lam, co
 // -1.01 dx/(x - alfa), 1.01 dx/(beta - x), without storing the direction (the trial pass
 // recomputes it). VW consecutive variables per loop step.
 template <int M, int VW>
-__global__ void __launch_bounds__(256) k_mma_dirmax(MVec lam, MVec dlam, double epsi, const double* __restrict__ low,
-                                                    const double* __restrict__ upp, MmaWork w) {
+__global__ void __launch_bounds__(256) k_mma_dirmax(const double* __restrict__ low, const double* __restrict__ upp,
+                                                    MmaWork w) {
+  const MmaState& S = *w.state;
+  if (S.mode != kMmaDirmax) return;  // another pass is due
+  MVec lam, dlam;
+#pragma unroll
+  for (int i = 0; i < M; i++) {
+    lam.v[i] = S.lo[i];
+    dlam.v[i] = S.dl[i];
+  }
+  const double epsi = S.epsi;
+  const MmaPoint pt = mma_point(w, S.parity != 0);
   double s[1] = {0.0};
   double mx[4] = {-1e300, -1e300, -1e300, -1e300};
   const size_t nq = w.n / VW;
   for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nq; q += size_t(gridDim.x) * blockDim.x) {
     MmaElem<M> e[VW];
     if (VW == 2)
-      load_pair<M>(w, low, upp, 2 * q, e[0], e[VW - 1]);
+      load_pair<M>(w, pt, low, upp, 2 * q, e[0], e[VW - 1]);
     else
-      load_elem<M>(w, low, upp, q, e[0]);
+      load_elem<M>(w, pt, low, upp, q, e[0]);
 #pragma unroll
     for (int v = 0; v < VW; v++) {
       double dx, dxsi, deta, rxa, rbx;
@@ -267,39 +532,49 @@ __global__ void __launch_bounds__(256) k_mma_dirmax(MVec lam, MVec dlam, double 
       mx[3] = fmax(mx[3], 1.01 * dx * rbx);
     }
   }
-  reduce_to_result<1, 4>(s, mx, w.partials, w.result, w.counter);
+  if (reduce_to_result<1, 4>(s, mx, w.partials, w.result, w.counter) && threadIdx.x == 0)
+    mma_after_dirmax<M>(*w.state, w.result);
 }
 
-// One pass at the trial point x + steg dx (steg = 0: the committed point, nothing written): the
-// relaxed KKT residual with the trial multiplier lam ([sum of squares, max |.|] of the n-part and
-// gvec_i = sum_j P/ux + Q/xl) and, at the same point, the pieces of the next Newton system (gvec,
-// GG delx/diagx, GG diag(1/diagx) GG^T), so an accepted step needs no further pass. The trial
-// point goes to xs_out / xsi_out / eta_out; accepting it is a pointer swap. VW consecutive
-// variables per loop step.
-// result = [resid sum of squares, resid gvec (M), newton gvec (M), GG delx/diagx (M),
-//           GG diag(1/diagx) GG^T (M*M), resid max |.|].
+// One pass at the trial point x + steg dx (start point: steg = 0, nothing written): the relaxed KKT
+// residual with the trial multiplier lam and, at the same point, the pieces of the next Newton system,
+// so an accepted step needs no further pass. The trial point goes to the arrays that do not hold the
+// committed one; accepting it flips the state's parity. VW consecutive variables per loop step.
+// result = [residual sum of squares, sum (xsi (x - alfa) - epsi) + (eta (beta - x) - epsi),
+//           gvec_i = sum P/ux + Q/xl (M), GG delx/diagx (M), GG (1/(x - alfa) - 1/(beta - x))/diagx (M),
+//           GG diag(1/diagx) GG^T (M*M), max |dL/dx|, max and -min of xsi (x - alfa), eta (beta - x)].
 template <int M, int VW>
-__global__ void __launch_bounds__(256) k_mma_trial(double steg, MVec lam, MVec lam_dir, MVec dlam, double epsi,
-                                                   double epsi_dir, const double* __restrict__ low,
-                                                   const double* __restrict__ upp, double* xs_out, double* xsi_out,
-                                                   double* eta_out, MmaWork w) {
-  constexpr int NS = 1 + M + M + M + M * M;
+__global__ void __launch_bounds__(256) k_mma_trial(const double* __restrict__ low, const double* __restrict__ upp,
+                                                   MmaWork w) {
+  const MmaState& S = *w.state;
+  const bool moved = S.mode == kMmaTrial;
+  if (!moved && S.mode != kMmaInit) return;  // another pass is due
+  MVec lam, lam_dir, dlam;
+#pragma unroll
+  for (int i = 0; i < M; i++) {
+    lam.v[i] = S.lam[i];
+    lam_dir.v[i] = S.lo[i];
+    dlam.v[i] = S.dl[i];
+  }
+  const double epsi = S.epsi, steg = S.steg;
+  const MmaPoint pt = mma_point(w, S.parity != 0), out = mma_point(w, S.parity == 0);
+  constexpr int NS = 2 + 3 * M + M * M;
   double s[NS];
-  double mx[1] = {0.0};
+  double mx[3] = {0.0, -1e300, -1e300};
 #pragma unroll
   for (int i = 0; i < NS; i++) s[i] = 0.0;
   const size_t nq = w.n / VW;
   for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nq; q += size_t(gridDim.x) * blockDim.x) {
     MmaElem<M> e[VW];
     if (VW == 2)
-      load_pair<M>(w, low, upp, 2 * q, e[0], e[VW - 1]);
+      load_pair<M>(w, pt, low, upp, 2 * q, e[0], e[VW - 1]);
     else
-      load_elem<M>(w, low, upp, q, e[0]);
+      load_elem<M>(w, pt, low, upp, q, e[0]);
 #pragma unroll
     for (int v = 0; v < VW; v++) {
-      if (steg != 0.0) {
+      if (moved) {
         double dx, dxsi, deta, r0, r1;
-        mma_dir<M>(e[v], lam_dir, dlam, epsi_dir, &dx, &dxsi, &deta, &r0, &r1);
+        mma_dir<M>(e[v], lam_dir, dlam, epsi, &dx, &dxsi, &deta, &r0, &r1);
         e[v].x = e[v].x + steg * dx;
         e[v].xsi = e[v].xsi + steg * dxsi;
         e[v].eta = e[v].eta + steg * deta;
@@ -312,13 +587,16 @@ __global__ void __launch_bounds__(256) k_mma_trial(double steg, MVec lam, MVec l
       for (int i = 0; i < M; i++) {
         plam += e[v].P[i] * lam.v[i];
         qlam += e[v].Q[i] * lam.v[i];
-        s[1 + i] += e[v].P[i] * uxi + e[v].Q[i] * xli;
+        s[2 + i] += e[v].P[i] * uxi + e[v].Q[i] * xli;
       }
       const double rex = plam * uxi * uxi - qlam * xli * xli - xsi + eta;
-      const double rexsi = xsi * (x - al) - epsi;
-      const double reeta = eta * (be - x) - epsi;
+      const double ca = xsi * (x - al), cb = eta * (be - x);
+      const double rexsi = ca - epsi, reeta = cb - epsi;
       s[0] += rex * rex + rexsi * rexsi + reeta * reeta;
-      mx[0] = fmax(mx[0], fmax(fabs(rex), fmax(fabs(rexsi), fabs(reeta))));
+      s[1] += rexsi + reeta;
+      mx[0] = fmax(mx[0], fabs(rex));
+      mx[1] = fmax(mx[1], fmax(ca, cb));
+      mx[2] = fmax(mx[2], -fmin(ca, cb));
       // Newton system pieces (its gvec is the residual's), with the reciprocals above and of
       // x - alfa, beta - x, diagx
       const double rux2 = uxi * uxi, rxl2 = xli * xli;
@@ -329,37 +607,41 @@ __global__ void __launch_bounds__(256) k_mma_trial(double steg, MVec lam, MVec l
       const double dpsidx = plam * rux2 - qlam * rxl2;
       const double delx = dpsidx - epsi * rxa + epsi * rbx;
       const double diagx = 2.0 * (plam * rux2 * uxi + qlam * rxl2 * xli) + xsi * rxa + eta * rbx;
-      const double id = 1.0 / diagx, dd = delx * id;
+      const double id = 1.0 / diagx, dd = delx * id, de = (rxa - rbx) * id;
 #pragma unroll
       for (int i = 0; i < M; i++) {
-        s[1 + 2 * M + i] += GG[i] * dd;
+        s[2 + M + i] += GG[i] * dd;
+        s[2 + 2 * M + i] += GG[i] * de;
 #pragma unroll
-        for (int k = 0; k < M; k++) s[1 + 3 * M + i * M + k] += GG[i] * GG[k] * id;
+        for (int k = 0; k < M; k++) s[2 + 3 * M + i * M + k] += GG[i] * GG[k] * id;
       }
     }
-    if (steg != 0.0) {
+    if (moved) {
       if (VW == 2) {
         const size_t j = 2 * q;
-        *reinterpret_cast<double2*>(xs_out + j) = make_double2(e[0].x, e[VW - 1].x);
-        *reinterpret_cast<double2*>(xsi_out + j) = make_double2(e[0].xsi, e[VW - 1].xsi);
-        *reinterpret_cast<double2*>(eta_out + j) = make_double2(e[0].eta, e[VW - 1].eta);
+        *reinterpret_cast<double2*>(out.x + j) = make_double2(e[0].x, e[VW - 1].x);
+        *reinterpret_cast<double2*>(out.xsi + j) = make_double2(e[0].xsi, e[VW - 1].xsi);
+        *reinterpret_cast<double2*>(out.eta + j) = make_double2(e[0].eta, e[VW - 1].eta);
       } else {
-        xs_out[q] = e[0].x;
-        xsi_out[q] = e[0].xsi;
-        eta_out[q] = e[0].eta;
+        out.x[q] = e[0].x;
+        out.xsi[q] = e[0].xsi;
+        out.eta[q] = e[0].eta;
       }
     }
   }
-#pragma unroll
-  for (int i = 0; i < M; i++) s[1 + M + i] = s[1 + i];
-  reduce_to_result<NS, 1>(s, mx, w.partials, w.result, w.counter);
+  if (reduce_to_result<NS, 3>(s, mx, w.partials, w.result, w.counter) && threadIdx.x == 0)
+    mma_after_trial<M>(*w.state, w.result);
 }
 
-__global__ void k_mma_finish(size_t n, double* xvar, double* xold1, double* xold2, const double* xs) {
+// The solution becomes x (also in FP32 to xf, if given), x and xold1 move one step back.
+__global__ void k_mma_finish(size_t n, double* xvar, double* xold1, double* xold2, float* xf, MmaWork w) {
+  const double* xs = mma_point(w, w.state->parity != 0).x;
   for (size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += size_t(gridDim.x) * blockDim.x) {
+    const double x = xs[j];
     xold2[j] = xold1[j];
     xold1[j] = xvar[j];
-    xvar[j] = xs[j];
+    xvar[j] = x;
+    if (xf) xf[j] = float(x);
   }
 }
 
@@ -368,39 +650,8 @@ __global__ void k_cast_f2d(size_t n, const float* __restrict__ a, double* b) {
     b[j] = double(a[j]);
 }
 
-__global__ void k_cast_d2f(size_t n, const double* __restrict__ a, float* b) {
-  for (size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += size_t(gridDim.x) * blockDim.x)
-    b[j] = float(a[j]);
-}
-
 __global__ void k_fill(size_t n, double v, double* a) {
   for (size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += size_t(gridDim.x) * blockDim.x) a[j] = v;
-}
-
-// Dense (m+1) x (m+1) solve with partial pivoting (replaces Eigen ColPivHouseholderQR,
-// optimization/mmaOpt.cpp:48-73).
-static bool dense_solve(int n, std::vector<double> A, std::vector<double>& b) {
-  for (int k = 0; k < n; k++) {
-    int p = k;
-    for (int i = k + 1; i < n; i++)
-      if (std::fabs(A[i * n + k]) > std::fabs(A[p * n + k])) p = i;
-    if (A[p * n + k] == 0.0) return false;
-    if (p != k) {
-      for (int j = 0; j < n; j++) std::swap(A[k * n + j], A[p * n + j]);
-      std::swap(b[k], b[p]);
-    }
-    for (int i = k + 1; i < n; i++) {
-      const double l = A[i * n + k] / A[k * n + k];
-      for (int j = k; j < n; j++) A[i * n + j] -= l * A[k * n + j];
-      b[i] -= l * b[k];
-    }
-  }
-  for (int i = n - 1; i >= 0; i--) {
-    double s = b[i];
-    for (int j = i + 1; j < n; j++) s -= A[i * n + j] * b[j];
-    b[i] = s / A[i * n + i];
-  }
-  return true;
 }
 
 static otm_status work_alloc(MmaWork& w, int m, size_t n, cudaStream_t s, bool async) {
@@ -419,7 +670,8 @@ static otm_status work_alloc(MmaWork& w, int m, size_t n, cudaStream_t s, bool a
     else
       OTM_CUDA(cudaMalloc((void**)a, size_t(m) * n * sizeof(double)));
   }
-  const size_t small = size_t(kMaxPartials) * kMmaSlots * sizeof(double) + kMmaSlots * sizeof(double) + 64;
+  const size_t small = size_t(kMaxPartials) * kMmaSlots * sizeof(double) + kMmaSlots * sizeof(double) + 64 +
+                       sizeof(MmaState);
   char* buf = nullptr;
   if (async)
     OTM_CUDA(scratch_malloc((void**)&buf, small, s));
@@ -428,8 +680,9 @@ static otm_status work_alloc(MmaWork& w, int m, size_t n, cudaStream_t s, bool a
   w.partials = (double*)buf;
   w.result = w.partials + size_t(kMaxPartials) * kMmaSlots;
   w.counter = (unsigned int*)(w.result + kMmaSlots);
+  w.state = (MmaState*)(w.result + kMmaSlots + 8);
   OTM_CUDA(cudaMemsetAsync(w.counter, 0, 64, s));
-  OTM_CUDA(cudaMallocHost((void**)&w.host, kMmaSlots * sizeof(double)));
+  OTM_CUDA(cudaMallocHost((void**)&w.host, 2 * sizeof(int)));
   return OTM_OK;
 }
 
@@ -461,210 +714,92 @@ static void dispatch_m(int m, Args&&... args) {
   }
 }
 
-template <int M>
-struct LaunchSetup {
-  static void run(int nb, cudaStream_t s, size_t n, int itn, const double* xvar, const double* xmin,
-                  const double* xmax, const double* xold1, const double* xold2, const double* df0dx,
-                  const double* dgdx, size_t ldg, double* low, double* upp, double move, MmaWork w) {
-    k_mma_setup<M><<<nb, 256, 0, s>>>(n, itn, xvar, xmin, xmax, xold1, xold2, df0dx, dgdx, ldg, low, upp, move, w);
-  }
+template <typename T>
+struct Setup {
+  template <int M>
+  struct Launch {
+    static void run(int nb, cudaStream_t s, size_t n, int itn, const MmaInputs<T>& in, const double* xmin,
+                    const double* xmax, const double* xold1, const double* xold2, double* low, double* upp, double move,
+                    const MmaProblem& pr, const MmaWork& w) {
+      k_mma_setup<M, T><<<nb, 256, 0, s>>>(n, itn, in, xmin, xmax, xold1, xold2, low, upp, move, pr, w);
+    }
+  };
 };
 
 template <int M>
 struct LaunchDirmax {
-  static void run(int nb, bool pairs, cudaStream_t s, MVec lam, MVec dlam, double epsi, const double* low,
-                  const double* upp, MmaWork w) {
+  static void run(int nb, bool pairs, cudaStream_t s, const double* low, const double* upp, const MmaWork& w) {
     if (pairs)
-      k_mma_dirmax<M, 2><<<nb, 256, 0, s>>>(lam, dlam, epsi, low, upp, w);
+      k_mma_dirmax<M, 2><<<nb, 256, 0, s>>>(low, upp, w);
     else
-      k_mma_dirmax<M, 1><<<nb, 256, 0, s>>>(lam, dlam, epsi, low, upp, w);
+      k_mma_dirmax<M, 1><<<nb, 256, 0, s>>>(low, upp, w);
   }
 };
 template <int M>
 struct LaunchTrial {
-  static void run(int nb, bool pairs, cudaStream_t s, double steg, MVec lam, MVec lam_dir, MVec dlam, double epsi,
-                  double epsi_dir, const double* low, const double* upp, double* xo, double* xsio, double* etao,
-                  MmaWork w) {
+  static void run(int nb, bool pairs, cudaStream_t s, const double* low, const double* upp, const MmaWork& w) {
     if (pairs)
-      k_mma_trial<M, 2><<<nb, 256, 0, s>>>(steg, lam, lam_dir, dlam, epsi, epsi_dir, low, upp, xo, xsio, etao, w);
+      k_mma_trial<M, 2><<<nb, 256, 0, s>>>(low, upp, w);
     else
-      k_mma_trial<M, 1><<<nb, 256, 0, s>>>(steg, lam, lam_dir, dlam, epsi, epsi_dir, low, upp, xo, xsio, etao, w);
+      k_mma_trial<M, 1><<<nb, 256, 0, s>>>(low, upp, w);
   }
 };
 
-static otm_status fetch(MmaWork& w, cudaStream_t s, int count) {
-  OTM_CUDA(cudaMemcpyAsync(w.host, w.result, count * sizeof(double), cudaMemcpyDeviceToHost, s));
-  OTM_CUDA(cudaStreamSynchronize(s));
-  return OTM_OK;
-}
+// Newton steps (a step-bound pass and a trial) queued before the host first looks, and between later
+// looks: a subproblem takes about 20 (measured on 128^3 and 384^3 design steps); a queued pair that
+// finds nothing due costs about 3 us, a look about 15.
+constexpr int kMmaFirstSteps = 16, kMmaMoreSteps = 4;
 
-// One MMA step (mmasub_g, optimization/mmaOpt.cu:1021-1062): device arrays, host-side a/c/d/gval.
-static otm_status mmasub_run(cudaStream_t s, int m, size_t n, int itn, double* xvar, const double* xmin,
-                             const double* xmax, double* xold1, double* xold2, const double* df0dx,
-                             const double* gval, const double* dgdx, size_t ldg, double* low, double* upp,
-                             double a0, const double* a, const double* c, const double* d, double move, MmaWork& w,
-                             uint64_t* launches) {
-  const int nb = int(std::min<size_t>(kMaxPartials, std::max<size_t>(1, (n + 255) / 256)));
+// Grids of the passes: the blocks that are resident at once (112 and 78 registers a thread at m = 1), so
+// that a block's reduction and the last block's sum over all blocks are paid once per resident block and
+// not once per 256 variables (at n = 2.1 M, 2048 blocks: trial 76 us, step bounds 51 us).
+constexpr int kMmaSms = 148, kMmaTrialBlocks = 2, kMmaDirmaxBlocks = 3;
+static_assert(4 * kMmaSms <= kMaxPartials, "the partial buffers hold kMaxPartials blocks");
+
+// One MMA step (mmasub_g, optimization/mmaOpt.cu:1021-1062): device arrays; a, c, d and the constraint
+// values in pr.
+template <typename T>
+static otm_status mmasub_run(cudaStream_t s, int m, size_t n, int itn, const MmaInputs<T>& in, double* xvar,
+                             const double* xmin, const double* xmax, double* xold1, double* xold2, double* low,
+                             double* upp, const MmaProblem& pr, double move, float* xf, MmaWork& w) {
+  const auto blocks = [](size_t work, int most) {
+    return int(std::min<size_t>(size_t(most), std::max<size_t>(1, (work + 255) / 256)));
+  };
+  const int nb = blocks(n, 4 * kMmaSms);
   uint64_t L = 0;
-  dispatch_m<LaunchSetup>(m, nb, s, n, itn, xvar, xmin, xmax, xold1, xold2, df0dx, dgdx, ldg, low, upp, move, w);
+  dispatch_m<Setup<T>::template Launch>(m, nb, s, n, itn, in, xmin, xmax, xold1, xold2, low, upp, move, pr, w);
   L++;
   OTM_CHECK_LAUNCH("k_mma_setup");
-  OTM_TRY(fetch(w, s, m));
-  std::vector<double> b(m);
-  for (int i = 0; i < m; i++) b[i] = w.host[i] - gval[i];
-
-  // subsolv (optimization/mmaOpt.cu:429-830): dual/slack variables of size m live on the host
-  std::vector<double> y(m, 1.0), lam(m, 1.0), mu(m), sv(m, 1.0);
-  for (int i = 0; i < m; i++) mu[i] = std::max(0.5 * c[i], 1.0);
-  double z = 1.0, zet = 1.0, epsi = 1.0;
-  MVec lamv{}, dlamv{};
-  std::vector<double> gvec(m);
-
-  auto m_residual = [&](const std::vector<double>& yy, double zz, const std::vector<double>& ll,
-                        const std::vector<double>& mm, double ze, const std::vector<double>& ss, double* n2,
-                        double* mxv) {
-    double ad = 0.0;
-    for (int i = 0; i < m; i++) ad += a[i] * ll[i];
-    auto acc = [&](double r) {
-      *n2 += r * r;
-      *mxv = std::max(*mxv, std::fabs(r));
-    };
-    for (int i = 0; i < m; i++) acc(c[i] + d[i] * yy[i] - mm[i] - ll[i]);
-    acc(a0 - ze - ad);
-    for (int i = 0; i < m; i++) acc(gvec[i] - a[i] * zz - yy[i] + ss[i] - b[i]);
-    for (int i = 0; i < m; i++) acc(mm[i] * yy[i] - epsi);
-    acc(ze * zz - epsi);
-    for (int i = 0; i < m; i++) acc(ll[i] * ss[i] - epsi);
-  };
-  // One pass at x + steg * (direction for lam_dir, dlam): residual norm / max with the trial
-  // multipliers, and the Newton pieces there (cached in newt: gvec, GG delx/diagx, GG GG^T/diagx).
-  // With steg != 0 the trial point is written to the spare arrays w.dx, w.dxsi, w.deta.
-  const int NS = 1 + 3 * m + m * m;
   // pairs of variables per loop step when every array the passes read is 16-byte aligned at
   // every row (n even; the work arrays come from the allocator, low and upp from the caller)
   // (m <= 4: beyond that the pair of elements no longer fits the registers)
   const bool pairs = m <= 4 && n % 2 == 0 && (reinterpret_cast<uintptr_t>(low) % 16) == 0 &&
                      (reinterpret_cast<uintptr_t>(upp) % 16) == 0;
-  const int nbp = int(std::min<size_t>(kMaxPartials, std::max<size_t>(1, (n / (pairs ? 2 : 1) + 255) / 256)));
-  std::vector<double> newt(size_t(2 * m + m * m));
-  auto trial = [&](double steg, const std::vector<double>& yy, double zz, const std::vector<double>& ll,
-                   const std::vector<double>& mm, double ze, const std::vector<double>& ss,
-                   const std::vector<double>& ldir, const MVec& dl, double* nrm, double* mxv) -> otm_status {
-    MVec lt{}, ld{};
-    for (int i = 0; i < m; i++) {
-      lt.v[i] = ll[i];
-      ld.v[i] = ldir[i];
-    }
-    dispatch_m<LaunchTrial>(m, nbp, pairs, s, steg, lt, ld, dl, epsi, epsi, (const double*)low, (const double*)upp,
-                            w.dx, w.dxsi, w.deta, w);
-    L++;
-    OTM_CHECK_LAUNCH("k_mma_trial");
-    OTM_TRY(fetch(w, s, NS + 1));
-    double n2 = w.host[0], mx = w.host[NS];
-    for (int i = 0; i < m; i++) gvec[i] = w.host[1 + i];
-    for (size_t i = 0; i < newt.size(); i++) newt[i] = w.host[1 + m + i];
-    m_residual(yy, zz, ll, mm, ze, ss, &n2, &mx);
-    *nrm = std::sqrt(n2);
-    *mxv = mx;
-    return OTM_OK;
-  };
-  // the trial point becomes the committed one (the work arrays keep owning both sets)
-  auto accept = [&]() {
-    std::swap(w.xs, w.dx);
-    std::swap(w.xsi, w.dxsi);
-    std::swap(w.eta, w.deta);
-  };
-
-  std::vector<double> dy(m), dmu(m), ds(m), dl(m), yo(m), lo(m), muo(m), so(m);
-  while (epsi > kEpsiMin) {
-    double residunorm, residumax;
-    OTM_TRY(trial(0.0, y, z, lam, mu, zet, sv, lam, dlamv, &residunorm, &residumax));
-    int ittt = 0;
-    while (residumax > 0.9 * epsi && ittt < 200) {
-      ittt++;
-      for (int i = 0; i < m; i++) lamv.v[i] = lam[i];
-      const double* hn = newt.data();  // Newton pieces at the committed point
-      for (int i = 0; i < m; i++) gvec[i] = hn[i];
-      double adl = 0.0;
-      for (int i = 0; i < m; i++) adl += a[i] * lam[i];
-      const double delz = a0 - adl - epsi / z;
-      std::vector<double> AA(size_t(m + 1) * (m + 1), 0.0), bb(m + 1);
-      std::vector<double> dely(m), diagy(m);
-      for (int i = 0; i < m; i++) {
-        dely[i] = c[i] + d[i] * y[i] - lam[i] - epsi / y[i];
-        const double dellam = gvec[i] - a[i] * z - y[i] - b[i] + epsi / lam[i];
-        diagy[i] = d[i] + mu[i] / y[i];
-        bb[i] = dellam + dely[i] / diagy[i] - hn[m + i];
-        for (int k = 0; k < m; k++) AA[size_t(i) * (m + 1) + k] = hn[2 * m + i * m + k];
-        AA[size_t(i) * (m + 1) + i] += sv[i] / lam[i] + 1.0 / diagy[i];
-        AA[size_t(i) * (m + 1) + m] = a[i];
-        AA[size_t(m) * (m + 1) + i] = a[i];
-      }
-      AA[size_t(m) * (m + 1) + m] = -zet / z;
-      bb[m] = delz;
-      if (!dense_solve(m + 1, AA, bb)) {
-        set_error("singular MMA Newton system");
-        return OTM_ERR_NAN;
-      }
-      for (int i = 0; i < m; i++) dl[i] = bb[i];
-      const double dz = bb[m];
-      for (int i = 0; i < m; i++) {
-        dy[i] = -dely[i] / diagy[i] + dl[i] / diagy[i];
-        dmu[i] = -mu[i] + epsi / y[i] - (mu[i] * dy[i]) / y[i];
-        ds[i] = -sv[i] + epsi / lam[i] - (sv[i] * dl[i]) / lam[i];
-        dlamv.v[i] = dl[i];
-      }
-      const double dzet = -zet + epsi / z - zet * dz / z;
-      dispatch_m<LaunchDirmax>(m, nbp, pairs, s, lamv, dlamv, epsi, (const double*)low, (const double*)upp, w);
-      L++;
-      OTM_CHECK_LAUNCH("k_mma_dirmax");
-      OTM_TRY(fetch(w, s, 5));
-      double stm = std::max(w.host[1], w.host[2]);  // xsi, eta parts
-      for (int i = 0; i < m; i++) {
-        stm = std::max(stm, -1.01 * dy[i] / y[i]);
-        stm = std::max(stm, -1.01 * dl[i] / lam[i]);
-        stm = std::max(stm, -1.01 * dmu[i] / mu[i]);
-        stm = std::max(stm, -1.01 * ds[i] / sv[i]);
-      }
-      stm = std::max(stm, -1.01 * dz / z);
-      stm = std::max(stm, -1.01 * dzet / zet);
-      const double stmalbe = std::max(w.host[3], w.host[4]);
-      double steg = 1.0 / std::max(std::max(stmalbe, stm), 1.0);
-      if (std::isnan(steg)) {
-        set_error("NaN step in the MMA subproblem");
-        return OTM_ERR_NAN;
-      }
-      yo = y;
-      lo = lam;
-      muo = mu;
-      so = sv;
-      const double zo = z, zeto = zet;
-      int itto = 0;
-      double resinew = 2 * residunorm, resimax = residumax;
-      while (resinew > residunorm && itto < 50) {
-        itto++;
-        for (int i = 0; i < m; i++) {
-          y[i] = yo[i] + steg * dy[i];
-          lam[i] = lo[i] + steg * dl[i];
-          mu[i] = muo[i] + steg * dmu[i];
-          sv[i] = so[i] + steg * ds[i];
-        }
-        z = zo + steg * dz;
-        zet = zeto + steg * dzet;
-        OTM_TRY(trial(steg, y, z, lam, mu, zet, sv, lo, dlamv, &resinew, &resimax));
-        steg /= 2;
-      }
-      accept();  // the last point tried, as the reference commits after its line search
-      residunorm = resinew;
-      residumax = resimax;
-    }
-    epsi *= 0.1;
-  }
-  k_mma_finish<<<nb, 256, 0, s>>>(n, xvar, xold1, xold2, w.xs);
+  const size_t groups = n / (pairs ? 2 : 1);
+  const int nbt = blocks(groups, kMmaTrialBlocks * kMmaSms), nbd = blocks(groups, kMmaDirmaxBlocks * kMmaSms);
+  const double *lowc = low, *uppc = upp;
+  dispatch_m<LaunchTrial>(m, nbt, pairs, s, lowc, uppc, w);
   L++;
-  OTM_CHECK_LAUNCH("k_mma_finish");
-  if (launches) *launches += L;
+  // the state machine ends: at most 200 Newton steps of at most 50 trials for each of 7 epsi
+  for (int steps = kMmaFirstSteps;; steps = kMmaMoreSteps) {
+    for (int i = 0; i < steps; i++) {
+      dispatch_m<LaunchDirmax>(m, nbd, pairs, s, lowc, uppc, w);
+      dispatch_m<LaunchTrial>(m, nbt, pairs, s, lowc, uppc, w);
+      L += 2;
+    }
+    OTM_CHECK_LAUNCH("MMA passes");
+    OTM_CUDA(cudaMemcpyAsync(w.host, w.state, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    OTM_CUDA(cudaStreamSynchronize(s));
+    if (w.host[0] == kMmaDone) break;
+  }
   count_launches(L);
+  if (w.host[1] != kMmaOk) {
+    set_error(w.host[1] == kMmaSingular ? "singular MMA Newton system" : "NaN step in the MMA subproblem");
+    return OTM_ERR_NAN;
+  }
+  k_mma_finish<<<nb, 256, 0, s>>>(n, xvar, xold1, xold2, xf, w);
+  OTM_CHECK_LAUNCH("k_mma_finish");
+  count_launches(1);
   return OTM_OK;
 }
 
@@ -679,10 +814,10 @@ struct otm_mma {
   std::vector<double> a, c, d;
   cudaStream_t stream = nullptr;
   double *xvar = nullptr, *xmin = nullptr, *xmax = nullptr, *xold1 = nullptr, *xold2 = nullptr;
-  double *low = nullptr, *upp = nullptr, *df0dx = nullptr, *dgdx = nullptr;
+  double *low = nullptr, *upp = nullptr;
   MmaWork w;
   ~otm_mma() {
-    double* arr[] = {xvar, xmin, xmax, xold1, xold2, low, upp, df0dx, dgdx};
+    double* arr[] = {xvar, xmin, xmax, xold1, xold2, low, upp};
     for (double* p : arr)
       if (p) cudaFree(p);
     work_free(w, nullptr, false);
@@ -709,14 +844,12 @@ otm_status otm_mma_create(int m, int n, double a0, double a, double c, double d,
     delete o;
     return st;
   };
-  double** arr[] = {&o->xvar, &o->xmin, &o->xmax, &o->xold1, &o->xold2, &o->low, &o->upp, &o->df0dx};
+  double** arr[] = {&o->xvar, &o->xmin, &o->xmax, &o->xold1, &o->xold2, &o->low, &o->upp};
   for (double** p : arr) {
     cudaError_t e = cudaMalloc((void**)p, o->n * sizeof(double));
     if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
     cudaMemset(*p, 0, o->n * sizeof(double));
   }
-  cudaError_t e = cudaMalloc((void**)&o->dgdx, size_t(m) * o->n * sizeof(double));
-  if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
   otm_status st = work_alloc(o->w, m, o->n, nullptr, false);
   if (st != OTM_OK) return fail(st);
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "otm_mma_create"));
@@ -762,25 +895,23 @@ otm_status otm_mma_update(otm_mma* mma, int itn, float* x_dev, const float* dfdx
   if (!mma || !x_dev || !dfdx_dev || !gval_host || !dgdx_dev) return OTM_ERR_INVALID_ARGUMENT;
   cudaStream_t s = mma->stream;
   const size_t n = mma->n;
-  const int nb = int(std::min<size_t>(kMaxPartials, (n + 255) / 256));
-  k_cast_f2d<<<nb, 256, 0, s>>>(n, x_dev, mma->xvar);
-  k_cast_f2d<<<nb, 256, 0, s>>>(n, dfdx_dev, mma->df0dx);
+  MmaInputs<float> in{};
+  in.x = x_dev;
+  in.df0dx = dfdx_dev;
+  in.xvar_out = mma->xvar;
+  MmaProblem pr{};
+  pr.a0 = mma->a0;
   for (int i = 0; i < mma->m; i++) {
     if (!dgdx_dev[i]) return OTM_ERR_INVALID_ARGUMENT;
-    k_cast_f2d<<<nb, 256, 0, s>>>(n, dgdx_dev[i], mma->dgdx + i * n);
+    in.dgdx[i] = dgdx_dev[i];
+    pr.a[i] = mma->a[i];
+    pr.c[i] = mma->c[i];
+    pr.d[i] = mma->d[i];
+    pr.g[i] = gval_host[i];
   }
-  OTM_CHECK_LAUNCH("k_cast_f2d");
-  count_launches(2 + mma->m);
-  std::vector<double> gval(mma->m);
-  for (int i = 0; i < mma->m; i++) gval[i] = gval_host[i];
   // f0val = 1 and move = 1 (optimization/mmaOptimizer.cu:69-70)
-  OTM_TRY(mmasub_run(s, mma->m, n, itn, mma->xvar, mma->xmin, mma->xmax, mma->xold1, mma->xold2, mma->df0dx,
-                     gval.data(), mma->dgdx, n, mma->low, mma->upp, mma->a0, mma->a.data(), mma->c.data(),
-                     mma->d.data(), 1.0, mma->w, nullptr));
-  k_cast_d2f<<<nb, 256, 0, s>>>(n, mma->xvar, x_dev);
-  OTM_CHECK_LAUNCH("k_cast_d2f");
-  count_launches(1);
-  return OTM_OK;
+  return mmasub_run(s, mma->m, n, itn, in, mma->xvar, mma->xmin, mma->xmax, mma->xold1, mma->xold2, mma->low, mma->upp,
+                    pr, 1.0, x_dev, mma->w);
 }
 
 otm_status otm_mmasub_device(int m, int n, int itn, double* xvar, double* xmin, double* xmax, double* xold1,
@@ -801,9 +932,21 @@ otm_status otm_mmasub_device(int m, int n, int itn, double* xvar, double* xmin, 
   OTM_CUDA(cudaStreamSynchronize(s));
   MmaWork w;
   otm_status st = work_alloc(w, m, size_t(n), s, true);
-  if (st == OTM_OK)
-    st = mmasub_run(s, m, size_t(n), itn, xvar, xmin, xmax, xold1, xold2, df0dx, hg.data(), (const double*)dgdx.ptr,
-                    dgdx.pitch / sizeof(double), low, upp, a0, ha.data(), hc.data(), hd.data(), move, w, nullptr);
+  if (st == OTM_OK) {
+    MmaInputs<double> in{};
+    in.x = xvar;
+    in.df0dx = df0dx;
+    MmaProblem pr{};
+    pr.a0 = a0;
+    for (int i = 0; i < m; i++) {
+      in.dgdx[i] = (const double*)dgdx.ptr + size_t(i) * (dgdx.pitch / sizeof(double));
+      pr.a[i] = ha[i];
+      pr.c[i] = hc[i];
+      pr.d[i] = hd[i];
+      pr.g[i] = hg[i];
+    }
+    st = mmasub_run(s, m, size_t(n), itn, in, xvar, xmin, xmax, xold1, xold2, low, upp, pr, move, (float*)nullptr, w);
+  }
   work_free(w, s, true);
   return st;
 }
