@@ -20,8 +20,6 @@
 #include "otm_solver_kernels.cuh"
 #include "otm_template.h"
 
-#include <cudaTypedefs.h>
-
 namespace otm {
 
 static thread_local std::string g_last_error;
@@ -371,48 +369,24 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
 template <typename T>
 static otm_status sweep_attributes() {
   const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromZero, false, T, T>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, false, T, T>, a, int(kTileSmemSweep)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, true, T, T>, a, int(kTileSmemSweep)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromZero, false, T, T>, a, int(kTileSmem)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, false, T, T>, a, int(kTileSmem)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromU, true, T, T>, a, int(kTileSmem)));
   OTM_CUDA(cudaFuncSetAttribute(k_tile_sweep<kFromUProlong, true, T, T>, a, int(kTileSmemProlong)));
   return OTM_OK;
 }
 
-// Dynamic shared memory of the tile kernels (a per-function attribute of the current device; set
-// at every build, which is cheap) and the TMA map of the fine right-hand side: a 4-D tensor
-// {nx, ny, nz, 3 cases} of FP32 read in boxes {8, 8, 4, 3}, eight per tile.
+// Dynamic shared memory of the tile kernels (a per-function attribute of the current device; set at
+// every build, which is cheap).
 otm_status Homo::tile_attributes() {
   const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
   OTM_TRY(sweep_attributes<float>());
   OTM_TRY(sweep_attributes<__nv_bfloat16>());
   OTM_TRY(sweep_attributes<__half>());
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_apply_dot, a, int(kTileSmemResid)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<float, float>, a, int(kTileSmemResid)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<__nv_bfloat16, __nv_bfloat16>, a, int(kTileSmemResid)));
-  OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<__half, __half>, a, int(kTileSmemResid)));
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    OTM_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-    if (q != cudaDriverEntryPointSuccess || !fn) {
-      set_error("cuTensorMapEncodeTiled is not available from the driver");
-      return OTM_ERR_UNSUPPORTED;
-    }
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
-  const Dims d = lv[0].d;
-  const cuuint64_t dims[4] = {cuuint64_t(d.nx), cuuint64_t(d.ny), cuuint64_t(d.nz), 3};
-  const cuuint64_t strides[3] = {cuuint64_t(d.nx) * 4, cuuint64_t(d.nx) * d.ny * 4, cuuint64_t(d.nv()) * 4};
-  const cuuint32_t box[4] = {cuuint32_t(kFBX), cuuint32_t(kFBY), cuuint32_t(kFBZ), 3};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = encode(&fmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, lv[0].f, dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed for the fine right-hand side");
-    return OTM_ERR_CUDA;
-  }
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_apply_dot, a, int(kTileSmem)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<float, float>, a, int(kTileSmem)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<__nv_bfloat16, __nv_bfloat16>, a, int(kTileSmem)));
+  OTM_CUDA(cudaFuncSetAttribute(k_tile_resid<__half, __half>, a, int(kTileSmem)));
   return OTM_OK;
 }
 
@@ -819,12 +793,12 @@ void Homo::vcycle_fine_tiled(const KT* k, VT* u, VT* r, const FineOp& fop, const
                shift, (const SolveScalars*)sc);
   };
   const float* none = nullptr;
-  sweep(k_tile_sweep<kFromZero, false, KT, VT>, kTileSmemSweep, nullptr, none, buf[0], 0);
+  sweep(k_tile_sweep<kFromZero, false, KT, VT>, kTileSmem, nullptr, none, buf[0], 0);
   for (int s = 1; s < npre; s++)
-    sweep(k_tile_sweep<kFromU, false, KT, VT>, kTileSmemSweep, buf[(s - 1) & 1], none, buf[s & 1], s & 1);
+    sweep(k_tile_sweep<kFromU, false, KT, VT>, kTileSmem, buf[(s - 1) & 1], none, buf[s & 1], s & 1);
   VT* pre = buf[(npre - 1) & 1];
-  launch_pdl(k_tile_resid<KT, VT>, dim3(nt), dim3(kResidThreads), kTileSmemResid, stream, fmap, L.d, k, fop,
-             (const VT*)pre, r, fs, sc);
+  launch_pdl(k_tile_resid<KT, VT>, dim3(nt), dim3(kResidThreads), kTileSmem, stream, L.d, k, fop, (const VT*)pre,
+             (const float*)L.f, r, fs, (const SolveScalars*)sc);
   launch_pdl(k_restrict<3, VT>, dim3(ceil_div(C.d.nv(), kBlock)), dim3(kBlock), 0, stream, L.d, C.d, (const VT*)r,
              C.f, (const SolveScalars*)sc, st_prefetch(1), st_prefetch_bytes(1));
   launched(npre + 2);
@@ -846,7 +820,7 @@ void Homo::vcycle_fine_tiled(const KT* k, VT* u, VT* r, const FineOp& fop, const
     if (s == 0)
       sweep(k_tile_sweep<kFromUProlong, true, KT, VT>, kTileSmemProlong, in, C.u, out, shift);
     else
-      sweep(k_tile_sweep<kFromU, true, KT, VT>, kTileSmemSweep, in, none, out, shift);
+      sweep(k_tile_sweep<kFromU, true, KT, VT>, kTileSmem, in, none, out, shift);
     in = out;
   }
   if (timed) cudaEventRecordWithFlags(prof_ev[1][prof_slot], stream, evflag);
@@ -904,7 +878,7 @@ void Homo::pcg_direction(const VT* z, const float* r, bool face, int nb) {
   launch_pdl(k_dot_rz<VT>, dim3(nb), dim3(kBlock), 0, stream, nv, r, z, partials, sc);
   // FP32 with the tile smoother: the tiled direction update (z's neighbours from shared memory)
   if (tiled && std::is_same<VT, float>::value && !face)
-    launch_pdl(k_tile_apply_dot, dim3(tile_count(d0)), dim3(kResidThreads), kTileSmemResid, stream, d0,
+    launch_pdl(k_tile_apply_dot, dim3(tile_count(d0)), dim3(kResidThreads), kTileSmem, stream, d0,
                (const float*)ks, op, (const float*)z, p, q, tile_partials, sc);
   else if (face)
     launch_pdl(k_update_p_apply_dot<true, VT>, dim3(nb), dim3(kBlock), 0, stream, d0, ks, op, z, p, q, partials, sc);
@@ -1243,10 +1217,7 @@ otm_status Homo::solve_impl(bool with_heat) {
     // retry from a zero initial guess, then give up.
   }
   otm_status st = OTM_OK;
-  if (sc_host->timeout) {
-    set_error("a tile kernel's bounded wait for its right-hand-side copy ran out");
-    st = OTM_ERR_TIMEOUT;
-  } else if (sc_host->nan) {
+  if (sc_host->nan) {
     set_error("MG numerical explode");
     st = OTM_ERR_DIVERGED;
   } else {

@@ -83,7 +83,6 @@ struct Homo {
   double* tile_partials = nullptr;  // 3 partial sums per fine tile (k_tile_apply_dot)
   std::vector<int> cl_tab_host;  // plane tables of the cluster plan (kept: the copy is asynchronous)
   int* cl_tab = nullptr;          // their device copy
-  CUtensorMap fmap{};  // TMA map of the fine right-hand side (3 cases, FP32) for the tile kernels
   int tail_l = -1;          // first level handled by the single-CTA tail kernel (-1: none)
   size_t tail_smem = 0;     // its dynamic shared memory
   int nc = 0;

@@ -35,8 +35,6 @@
 // and free the shared memory of a third CTA per SM.
 #pragma once
 
-#include <cuda.h>
-
 #include "otm_mg_kernels.cuh"
 
 namespace otm {
@@ -52,28 +50,12 @@ constexpr int kResidThreads = 256;                            // one thread per 
 constexpr int kSeg = 4;                                       // vertices per thread and pass
 constexpr int kCX = kTX / 2 + 2, kCY = kTY / 2 + 2, kCZ = kTZ / 2 + 2;  // staged coarse sites
 constexpr int kCSites = kCX * kCY * kCZ;                      // 600
-constexpr int kFElems = 3 * kTX * kTY * kTZ;                  // right-hand side of a tile (6144 floats)
-constexpr int kFBX = 8, kFBY = 8, kFBZ = 4;                   // TMA box of the right-hand side (x 3 cases)
-constexpr int kFBox = kFBX * kFBY * kFBZ * 3;                 // 768 floats per box
-constexpr int kFCase = kFBX * kFBY * kFBZ;                    // case stride inside a box (256)
 static_assert((kTX / 2) * (kTY / 2) * (kTZ / kSeg) == kSmoothThreads, "one thread per column segment");
 static_assert(kTX * kTY == kResidThreads, "one thread per column");
-static_assert(kSeg == kFBZ && kTX == 2 * kFBX && kTY == 2 * kFBY && kTZ == 2 * kFBZ,
-              "a column segment lies in one right-hand-side box along z; 2 x 2 x 2 boxes per tile");
 
-// Dynamic shared memory of a sweep: [sites][coarse block]; of the residual and the direction update:
-// [right-hand-side boxes][mbarrier][sites], after rounding the base up to 128 bytes (the TMA
-// destination's alignment).
-constexpr size_t kTileSmemSweep = size_t(kSSites) * sizeof(float4);                         // 54,720 B
-constexpr size_t kTileSmemProlong = kTileSmemSweep + size_t(kCSites) * sizeof(float4);       // 64,320 B
-constexpr size_t kOffBar = size_t(kFElems) * sizeof(float);
-constexpr size_t kOffSites = kOffBar + 128;
-constexpr size_t kTileSmemResid = kOffSites + size_t(kSSites) * sizeof(float4) + 128;        // 79,552 B
-constexpr uint32_t kFBytes = uint32_t(kFElems * sizeof(float));
-
-// Polls of the right-hand-side copy's mbarrier before a CTA gives up (each poll may suspend the
-// thread for a short hardware-defined time; together well over a second).
-constexpr int kTileWaitPolls = 1 << 20;
+// Dynamic shared memory: [sites][coarse block (prolonging sweep)].
+constexpr size_t kTileSmem = size_t(kSSites) * sizeof(float4);                        // 54,720 B
+constexpr size_t kTileSmemProlong = kTileSmem + size_t(kCSites) * sizeof(float4);      // 64,320 B
 
 // Whether a level's dimensions can be tiled.
 __host__ __device__ inline bool tile_fits(const Dims& d) {
@@ -100,72 +82,8 @@ __device__ __forceinline__ void tile_origin(const Dims& d, unsigned b, int shift
   z0 = int(q / nty) * kTZ + shift * (kTZ / 2);
 }
 
-// Position of the right-hand side of tile vertex (x, y, z) (0-based inside the tile) of case 0 in
-// the staged boxes; case c is kFCase further: box (x / 8, y / 8, z / 4), inside it x, y, z, case.
-__device__ __forceinline__ int fpos(int x, int y, int z) {
-  return ((x >> 3) + 2 * (y >> 3) + 4 * (z >> 2)) * kFBox + ((z & 3) * kFBY + (y & 7)) * kFBX + (x & 7);
-}
-
-// ---- the residual's right-hand-side copy: TMA tensor loads completing on an mbarrier -----------
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Thread 0 initialises the barrier and starts the copies of the tile's right-hand side (eight
-// boxes, their periodic origins wrapped; an origin is a multiple of 8 (x, y) or 4 (z) and the
-// level's dimensions are multiples of 16 and 8, so no box crosses the periodic boundary). The
-// barrier initialisation is published to the other threads by the __syncthreads() that precedes
-// the wait.
-__device__ __forceinline__ void tile_f_copy_start(const CUtensorMap* fmap, float* fsm, uint64_t* bar, const Dims& d,
-                                                  int x0, int y0, int z0) {
-  if (threadIdx.x == 0) {
-    const uint32_t b = smem_addr(bar);
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(1) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(kFBytes) : "memory");
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const int X = wrapm(x0 + kFBX * (q & 1), d.nx), Y = wrapm(y0 + kFBY * ((q >> 1) & 1), d.ny),
-                Z = wrapm(z0 + kFBZ * (q >> 2), d.nz);
-      asm volatile(
-          "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
-          "%4, %5}], [%6];" ::"r"(smem_addr(fsm + q * kFBox)),
-          "l"(reinterpret_cast<uint64_t>(fmap)), "r"(X), "r"(Y), "r"(Z), "r"(0), "r"(b)
-          : "memory");
-    }
-  }
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait for the copies. One thread polls the mbarrier (polls by every thread would compete
-// with the other CTA's passes for shared-memory bandwidth and issue slots); the others wait at the
-// barrier, which also makes the copied data visible to them. Returns false in every thread of the
-// CTA if the polls ran out; then the solve is flagged (timeout + done) and the polling thread waits
-// once more, again bounded, for the copies it issued before the CTA returns.
-__device__ __forceinline__ bool tile_f_copy_wait(uint64_t* bar, SolveScalars* sc) {
-  bool ok = true;
-  if (threadIdx.x == 0) {
-    ok = false;
-    for (int i = 0; i < kTileWaitPolls && !ok; i++) ok = mbar_try_wait(bar, 0);
-    if (!ok) {
-      if (sc) {
-        atomicExch(&sc->timeout, 1);
-        atomicExch(&sc->done, 1);
-      }
-      for (int i = 0; i < kTileWaitPolls && !ok; i++) ok = mbar_try_wait(bar, 0);
-      ok = false;
-    }
-  }
-  return !__syncthreads_or(!ok);
 }
 
 // ---- vector loads and stores of 4 consecutive values in the storage types --------------------
@@ -518,13 +436,6 @@ __device__ __forceinline__ void stage_tile(const Dims& d, const Dims& dc, int x0
   }
 }
 
-// Aligned base of the dynamic shared memory (128 bytes: the TMA destination).
-__device__ __forceinline__ unsigned char* tile_smem_base() {
-  extern __shared__ unsigned char tile_smem_raw[];
-  const uintptr_t a = reinterpret_cast<uintptr_t>(tile_smem_raw);
-  return reinterpret_cast<unsigned char*>((a + 127) & ~uintptr_t(127));
-}
-
 // Start of a sweep: from zero (the first pre-smoothing sweep), from u_in, or from u_in plus the
 // trilinear prolongation of the coarse correction (the first post-smoothing sweep).
 enum TileStart { kFromZero = 0, kFromU = 1, kFromUProlong = 2 };
@@ -616,33 +527,30 @@ __global__ void __launch_bounds__(kSmoothThreads, 3)
 
 // r = f - A u on the fine level for every vertex of a tile (tiling 0), from a staged tile with its
 // halo (natural site order here: lanes take consecutive sites of a row). A thread owns one column
-// of the tile and streams its 10 planes. The right-hand side (3 cases, FP32, 24 KB) arrives by TMA
-// (cp.async.bulk.tensor of eight 4-D boxes {8, 8, 4, 3}, completion on one mbarrier), issued at kernel
-// entry so that it lands while the threads stage the sites.
+// of the tile and streams its 10 planes; the right-hand side is read one plane ahead.
 template <typename KT, typename VT>
-__global__ void __launch_bounds__(kResidThreads, 2)
-    k_tile_resid(const __grid_constant__ CUtensorMap fmap, Dims d, const KT* __restrict__ ks, FineOp op,
-                 const VT* __restrict__ u, VT* __restrict__ r, const double* fscale, SolveScalars* sc) {
-  unsigned char* base = tile_smem_base();
-  float* fsm = reinterpret_cast<float*>(base);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base + kOffBar);
-  float4* sm = reinterpret_cast<float4*>(base + kOffSites);
+__global__ void __launch_bounds__(kResidThreads, 3)
+    k_tile_resid(Dims d, const KT* __restrict__ ks, FineOp op, const VT* __restrict__ u, const float* __restrict__ f,
+                 VT* __restrict__ r, const double* fscale, const SolveScalars* sc) {
+  extern __shared__ float4 resid_sm[];
+  float4* sm = resid_sm;
   pdl_wait();
   if (sc && solve_done(sc)) return;
   int x0, y0, z0;
   tile_origin(d, blockIdx.x, 0, x0, y0, z0);
   const size_t nv = d.nv();
-  tile_f_copy_start(&fmap, fsm, bar, d, x0, y0, z0);
   float fs[3] = {1.f, 1.f, 1.f};
   if (fscale)
 #pragma unroll
     for (int c = 0; c < 3; c++) fs[c] = float(fscale[c]);
+  const int lx = 1 + (int(threadIdx.x) & 15), ly = 1 + (int(threadIdx.x) >> 4);
+  const size_t pl = size_t(d.nx) * d.ny;
+  const size_t col = size_t(x0 + lx - 1) + size_t(d.nx) * size_t(y0 + ly - 1) + size_t(z0) * pl;
+  float fn[3];  // right-hand side of vertex P + 1
+#pragma unroll
+  for (int c = 0; c < 3; c++) fn[c] = __ldg(f + c * nv + col);
   stage_tile<true, kResidThreads, false>(d, d, x0, y0, z0, ks, u, (const float*)nullptr, sm, (float4*)nullptr);
   __syncthreads();
-  if (!tile_f_copy_wait(bar, sc)) return;
-  const int lx = 1 + (int(threadIdx.x) & 15), ly = 1 + (int(threadIdx.x) >> 4);
-  const size_t col = size_t(x0 + lx - 1) + size_t(d.nx) * size_t(y0 + ly - 1);
-  const size_t pl = size_t(d.nx) * d.ny;
   float Kp[4] = {0.f, 0.f, 0.f, 0.f};
   PlaneCoef Cp;
   float accA[3] = {0.f, 0.f, 0.f}, accB[3] = {0.f, 0.f, 0.f}, accC[3] = {0.f, 0.f, 0.f};
@@ -668,9 +576,11 @@ __global__ void __launch_bounds__(kResidThreads, 2)
     float dC = 0.f;
     // vertex P + 1 (interior planes 1..8): lower element plane P
     if (P + 1 <= kTZ) {
-      const float* fv = fsm + fpos(lx - 1, ly - 1, P);
 #pragma unroll
-      for (int c = 0; c < 3; c++) accC[c] = fv[c * kFCase] * fs[c];
+      for (int c = 0; c < 3; c++) accC[c] = fn[c] * fs[c];
+      if (P + 2 <= kTZ)
+#pragma unroll
+        for (int c = 0; c < 3; c++) fn[c] = __ldg(f + c * nv + col + size_t(P + 1) * pl);
       sub_plane(accC, C, nb);
       dC = sK;
     }
@@ -686,7 +596,7 @@ __global__ void __launch_bounds__(kResidThreads, 2)
     if (P >= 2) {
       sub_plane(accA, Cp, nb);
       const float diag = op.c0 * dA;
-      const size_t g = col + size_t(z0 + P - 2) * pl;
+      const size_t g = col + size_t(P - 2) * pl;
       st(r + g, accA[0] - diag * uA[0]);
       st(r + nv + g, accA[1] - diag * uA[1]);
       st(r + 2 * nv + g, accA[2] - diag * uA[2]);
@@ -711,11 +621,11 @@ __global__ void __launch_bounds__(kResidThreads, 2)
 // (p . q). z is staged like u in k_tile_resid (tiling 0, one thread per column streaming its 10
 // planes) so its 20 neighbours come from shared memory; beta == 0 (the first iteration) ignores
 // the old p and q. part: 3 doubles per tile.
-static __global__ void __launch_bounds__(kResidThreads, 2)
+static __global__ void __launch_bounds__(kResidThreads, 3)
     k_tile_apply_dot(Dims d, const float* __restrict__ ks, FineOp op, const float* __restrict__ z,
                      float* __restrict__ p, float* __restrict__ q, double* part, SolveScalars* sc) {
-  unsigned char* base = tile_smem_base();
-  float4* sm = reinterpret_cast<float4*>(base + kOffSites);
+  extern __shared__ float4 apply_sm[];
+  float4* sm = apply_sm;
   pdl_wait();
   if (solve_done(sc)) return;
   int x0, y0, z0;
