@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "otm_mg_kernels.cuh"
@@ -31,22 +32,23 @@ constexpr int kCl = 16;            // CTAs per cluster (non-portable size, opted
 constexpr int kClThreads = 512;
 constexpr int kClMaxLevels = 8;
 constexpr int kClMaxNv = 32768;    // unknowns of the first level handled by the cluster (32^3)
+constexpr int kClSlots = 256;      // stencil stride of the levels with at most that many vertices per CTA
 constexpr int kClMaxTab = 6144;    // plane-table entries over all levels (3 per plane)
 
 struct ClLevel {
   Dims d;
   int cs;      // case stride of f and r in shared memory: (planes of the fullest slab) * nx * ny
-  int urs;     // u row stride (nx, padded against shared-memory bank conflicts)
+  int uh;      // position of a row's odd sites in u: site x lies at (x odd ? uh : 0) + x / 2
+  int urs;     // u row stride (at least nx, chosen with uh against shared-memory bank conflicts)
   int ups;     // u plane stride (ny * urs, padded)
   int ucs;     // u case stride: two more planes (ghost copies of the neighbouring slabs' edge planes)
   int u_off;   // float offsets in shared memory
   int f_off;   // < 0: right-hand side read from f_in (global; first level only, when not staged)
   int r_off;   // < 0: residual in rg (global, lexicographic, case-major)
-  int st_off;  // < 0: stencils read from st (global, colour-blocked); else [vertex][27]
-  int inv_off; // inverse diagonal per own vertex (with st_off >= 0)
+  int ss;      // stencil stride: entry o of slot s at st_off + o * ss + s (kClSlots where the slots fit that)
+  int st_off;  // < 0: stencils read from st (global, colour-blocked)
+  int inv_off; // inverse diagonal per slot (with st_off >= 0)
   int tab_off; // plane tables of this level: nz ownership entries, then 2 nz ghost-push entries
-  int tw_res;  // log2 of the lanes that share one vertex's 27 products in the residual
-  int lhx, lhy;  // log2 of nx/2, ny/2 rounded up to powers of two (colour-pass enumeration)
   int lnx, lny;  // log2 of nx, ny rounded up (residual enumeration)
   int zstart[kCl + 1];  // CTA c holds planes [zstart[c], zstart[c+1])
   const float* st;
@@ -72,8 +74,40 @@ struct ClDesc {
 // an edge plane also writes the value into the copies held by its neighbours ("ghost push"),
 // so every read of a colour pass or residual is a local shared-memory load.
 
-// Plane z of f or r (in-plane stride nx) at `off` of level L, wherever it lives in the cluster
-// (case 0; case c is at + c * L.cs).
+// In-row position of site x of u: even and odd sites apart, so that the lanes of a colour pass, which
+// take every other site of a row, read consecutive words.
+__device__ __forceinline__ int cl_ux(const ClLevel& L, int x) { return ((x & 1) ? L.uh : 0) + (x >> 1); }
+
+// On a level with its stencils in shared memory a CTA orders its vertices by colour ("slots": colours
+// 0..3 of its even planes, then 4..7 of its odd planes, lexicographic inside a colour), and keeps the
+// stencils, the inverse diagonal and the right-hand side in that order: the lanes of a pass read
+// consecutive words.
+struct ClSlots {
+  int n[2], zf[2];  // vertices per colour and first plane, by plane parity
+  int npl[2];       // own planes of the parity
+  __device__ __forceinline__ ClSlots(const ClLevel& L, int rank) {
+    const int z0 = L.zstart[rank], z1 = L.zstart[rank + 1], per = (L.d.nx >> 1) * (L.d.ny >> 1);
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      zf[p] = z0 + (((z0 & 1) != p) ? 1 : 0);
+      npl[p] = zf[p] < z1 ? (z1 - zf[p] + 1) >> 1 : 0;
+      n[p] = npl[p] * per;
+    }
+  }
+  __device__ __forceinline__ int total() const { return 4 * (n[0] + n[1]); }
+  __device__ __forceinline__ int base(int color) const {
+    return (color >> 2) ? 4 * n[0] + (color & 3) * n[1] : color * n[0];
+  }
+  // slot of the own vertex (x, y, z)
+  __device__ __forceinline__ int slot(const ClLevel& L, int x, int y, int z) const {
+    const int hx = L.d.nx >> 1, hy = L.d.ny >> 1;
+    return base((x & 1) + 2 * (y & 1) + 4 * (z & 1)) +
+           ((((z - ((z & 1) ? zf[1] : zf[0])) >> 1) * hy + (y >> 1)) * hx + (x >> 1));
+  }
+};
+
+// Plane z of r, or of f on the coarsest level (in-plane stride nx), at `off` of level L, wherever it
+// lives in the cluster (case 0; case c is at + c * L.cs).
 __device__ __forceinline__ const float* cl_plane(const ClLevel& L, const int* tab, float* const* rb, int off, int z) {
   const int e = tab[L.tab_off + z];
   return rb[e >> 16] + off + (e & 0xffff) * (L.d.nx * L.d.ny);
@@ -95,160 +129,315 @@ __device__ __forceinline__ void cl_ghosts(const ClLevel& L, const int* tab, floa
   g1 = e1 >= 0 ? rb[e1 >> 16] + L.u_off + (e1 & 0xffff) * L.ups + p : nullptr;
 }
 
-// 27-point products of one vertex shared by a team of kTw lanes of one warp: lane k of the
-// team takes the offsets k, k + kTw, ... and the team sums with butterfly shuffles, so small
-// levels (a few dozen vertices per CTA) keep the latency of one vertex short. pu[0..2] are the
-// local u planes z-1, z, z+1. Returns sum_o A(v, v+o) u(v+o) over the selected offsets in
-// every lane of the team.
-template <bool kSmemSt, bool kSkipCentre, int kTw>
-__device__ __forceinline__ void cl_apply_team(const float* sp, size_t sstride, const float* const (&pu)[3], int xm,
-                                              int x, int xp, int ym, int y0, int yp, int ucs, int lane,
-                                              float (&acc)[3]) {
-  acc[0] = acc[1] = acc[2] = 0.f;
-  // fully unrolled (predicated) so that all loads of a lane are in flight together
-#pragma unroll
-  for (int k = 0; k < (27 + kTw - 1) / kTw; k++) {
-    const int o = lane + k * kTw;
-    if (o < 27 && !(kSkipCentre && o == 13)) {
-      const float s = kSmemSt ? sp[o * sstride] : __ldg(sp + o * sstride);
-      const int ox = o % 3, oy = (o / 3) % 3, oz = o / 9;
-      const int xo = ox == 0 ? xm : (ox == 1 ? x : xp);
-      const int yo = oy == 0 ? ym : (oy == 1 ? y0 : yp);
-      const float* q = (oz == 0 ? pu[0] : (oz == 1 ? pu[1] : pu[2])) + yo + xo;
-#pragma unroll
-      for (int c = 0; c < 3; c++) acc[c] += s * q[c * ucs];
-    }
-  }
-#pragma unroll
-  for (int off = kTw >> 1; off > 0; off >>= 1)
-#pragma unroll
-    for (int c = 0; c < 3; c++) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
+// A read-only load that stays where it is written (the compiler otherwise moves loads next to their use
+// to save registers, which makes a chain of L2 latencies of them).
+__device__ __forceinline__ float ld_issue(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
 }
 
-// One Gauss-Seidel colour pass over this CTA's vertices of the colour (gs_coarse_body); updated
-// edge-plane values are pushed to the ghosts. Vertices are enumerated over power-of-two index
-// ranges (shifts and masks instead of divisions); indices past nx/2 or ny/2 are idle. Only the
-// warps that hold a vertex run the body, and every load of a vertex (right-hand side, inverse
-// diagonal, ghost targets) is issued before its first store, so no store orders a reload.
-template <bool kSmemSt, int kTwl>
-__device__ __forceinline__ void cl_gs_t(const ClLevel& L, const float* __restrict__ f_glob, float* sm, const int* tab,
-                                        float* const* rb, int rank, int color) {
-  const Dims d = L.d;
-  const int nx = d.nx, ny = d.ny, hx = nx >> 1, hy = ny >> 1, plane = nx * ny;
-  const int z0 = L.zstart[rank], z1 = L.zstart[rank + 1];
-  const int zf = z0 + (((z0 & 1) != (color >> 2)) ? 1 : 0);  // first own plane of the colour's parity
-  const int npl = zf < z1 ? (z1 - zf + 1) >> 1 : 0;
-  const int lhx = L.lhx, lhy = L.lhy;
-  const int n = npl << (lhx + lhy);
-  if (n == 0) return;  // uniform over the CTA
-  const int cs = L.cs, ucs = L.ucs, urs = L.urs, ups = L.ups;
-  const int u_off = L.u_off, f_off = L.f_off, st_off = L.st_off, inv_off = L.inv_off;
-  const float* st_glob = L.st;
-  const size_t nv = d.nv();
-  // whole warps only (the team shuffles need all 32 lanes of a warp)
-  const int total = ((n << kTwl) + 31) & ~31;
-  for (int g = threadIdx.x; g < total; g += blockDim.x) {
-    const int t0 = g >> kTwl, lane = g & ((1 << kTwl) - 1);
-    const int i0 = t0 & ((1 << lhx) - 1), j0 = (t0 >> lhx) & ((1 << lhy) - 1), pk0 = t0 >> (lhx + lhy);
-    const bool active = t0 < n && i0 < hx && j0 < hy;
-    const int i = active ? i0 : 0, j = active ? j0 : 0, pk = active ? pk0 : 0;
-    const int x = 2 * i + (color & 1), y = 2 * j + ((color >> 1) & 1), z = zf + 2 * pk;
-    const int xm = wrapm(x - 1, nx), xp = wrapm(x + 1, nx);
-    const int ym = wrapm(y - 1, ny) * urs, y0 = y * urs, yp = wrapm(y + 1, ny) * urs;
-    const int zl = z - z0;
-    const float* uz = sm + u_off + zl * ups;  // local planes zl, zl+1, zl+2 = z-1, z, z+1
-    const float* const pu[3] = {uz, uz + ups, uz + 2 * ups};
-    const int lidx = zl * plane + y * nx + x;  // own-vertex index (f, r, stencils)
-    const float* sp = kSmemSt ? sm + st_off + lidx * 27 : st_glob + cb_index(d, x, y, z);
-    const size_t sstride = kSmemSt ? size_t(1) : nv;
-    float acc[3];
-    cl_apply_team<kSmemSt, true, (1 << kTwl)>(sp, sstride, pu, xm, x, xp, ym, y0, yp, ucs, lane, acc);
-    if (active && lane == 0) {
-      const float inv = kSmemSt ? sm[inv_off + lidx] : 1.0f / __ldg(sp + 13 * sstride);
-      float fv[3];
+// The colour passes (gs_coarse_body): a CTA updates its vertices of a colour and pushes updated edge-plane
+// values to the ghosts. A colour of a CTA has at most kClThreads vertices (cl_plan_try), one lane each or
+// one per load case.
+// Stencils in shared memory: one colour pass of a half sweep (colours (cx, cy) of one plane parity) by
+// one lane per vertex and load case. `V` is the lane's vertex block: what does not change over the four
+// colours of the half sweep, so that a pass is its 26 products, one store and its pushes.
+struct ClHalf {
+  const float* st;  // stencils at the slot of colour (0, 0); colour q is q * n further
+  float* up;        // u, local plane of z - 1, case of the lane
+  float *g0, *g1;   // ghost copies of plane z, same case (null: none)
+  int n;            // slots per colour
+  int ss, ups;
+  int row[4];       // offsets of the rows 2j - 1 .. 2j + 2
+  int xp[4];        // in-row positions of the sites 2i - 1 .. 2i + 2
+  float f[4], inv[4];  // right-hand side and inverse diagonal of the four colours
+  bool on;
+};
+
+template <int q, int kSS>
+__device__ __forceinline__ void cl_half_pass(const ClHalf& V) {
+  constexpr int cx = q & 1, cy = q >> 1;
+  const float* sp = V.st + q * V.n;
+  const int ss = kSS ? kSS : V.ss;
+  float st[27];
 #pragma unroll
-      for (int c = 0; c < 3; c++)
-        fv[c] = f_off >= 0 ? sm[f_off + c * cs + lidx] : __ldg(f_glob + c * nv + size_t(z) * plane + y * nx + x);
-      const int pu_idx = y0 + x;
-      float *g0, *g1;
-      cl_ghosts(L, tab, rb, z, pu_idx, g0, g1);
-      float* own = sm + u_off + (zl + 1) * ups + pu_idx;
+  for (int o = 0; o < 27; o++)
+    if (o != 13) st[o] = sp[o * ss];
+  float acc[3];  // one sum per plane: three short chains
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float v = (fv[c] - acc[c]) * inv;
-        own[c * ucs] = v;
-        if (g0) g0[c * ucs] = v;
-        if (g1) g1[c * ucs] = v;
-      }
-    }
+  for (int a = 0; a < 3; a++) {
+    const float* u = V.up + a * V.ups;
+    acc[a] = 0.f;
+#pragma unroll
+    for (int b = 0; b < 9; b++)
+      if (9 * a + b != 13) acc[a] += st[9 * a + b] * u[V.row[cy + b / 3] + V.xp[cx + b % 3]];
+  }
+  const float v = (V.f[q] - (acc[0] + acc[1] + acc[2])) * V.inv[q];
+  const int p = V.row[cy + 1] + V.xp[cx + 1];
+  if (V.on) {
+    V.up[V.ups + p] = v;
+    if (V.g0) V.g0[p] = v;
+    if (V.g1) V.g1[p] = v;
   }
 }
 
-// One lane per vertex on every level: the 27 products with compile-time offsets cost fewer
-// instructions than a lane team's shared offsets and shuffles, and on the small levels the
-// pass is bound by instruction issue, not by the latency of one vertex.
-__device__ __forceinline__ void cl_gs(const ClLevel& L, const float* f_glob, float* sm, const int* tab,
-                                      float* const* rb, int rank, int color) {
-  if (L.st_off < 0)
-    cl_gs_t<false, 0>(L, f_glob, sm, tab, rb, rank, color);
+// Colours 0..3 of the planes of parity pz (3..0 when kRev). A case's vertices are in warps of their own
+// (the 27 products of a case need no other case's: 16^3 has 64 vertices of a colour on a CTA, two warps,
+// which would each work through the three cases one after the other); the warps that hold a vertex
+// synchronise among themselves between the colours. A pass used to be a chain of index arithmetic, table
+// look-ups and conflicting reads, 2,100 cycles at 16^3 for a hundred instructions of work; the launch
+// for 16^3 and below took 77 us (32^3 cell, warm) and takes 47 us.
+template <bool kRev, int kSS>
+__device__ __forceinline__ void cl_half_run(const ClHalf& V, int nthreads) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    switch (kRev ? 3 - k : k) {
+      case 0: cl_half_pass<0, kSS>(V); break;
+      case 1: cl_half_pass<1, kSS>(V); break;
+      case 2: cl_half_pass<2, kSS>(V); break;
+      default: cl_half_pass<3, kSS>(V); break;
+    }
+    if (k < 3) asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  }
+}
+
+// As cl_half_pass by one lane per vertex with its three cases (more vertices of a colour than a third of
+// the threads): fs, is: the right-hand side and the inverse diagonal at the slot of colour (0, 0).
+template <int q>
+__device__ __forceinline__ void cl_half_pass3(const ClHalf& V, const float* fs, const float* is, int cs, int ucs) {
+  constexpr int cx = q & 1, cy = q >> 1;
+  const float* sp = V.st + q * V.n;
+  float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+  for (int o = 0; o < 27; o++) {
+    if (o == 13) continue;
+    const float st = sp[o * V.ss];
+    const float* u = V.up + (o / 9) * V.ups + V.row[cy + (o / 3) % 3] + V.xp[cx + o % 3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) acc[c] += st * u[c * ucs];
+  }
+  const float inv = is[q * V.n];
+  const int p = V.row[cy + 1] + V.xp[cx + 1];
+  float v[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) v[c] = (fs[c * cs + q * V.n] - acc[c]) * inv;
+  if (V.on) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      V.up[V.ups + p + c * ucs] = v[c];
+      if (V.g0) V.g0[p + c * ucs] = v[c];
+      if (V.g1) V.g1[p + c * ucs] = v[c];
+    }
+  }
+}
+
+template <bool kRev>
+__device__ __forceinline__ void cl_half_sweep(const ClLevel& L, float* sm, const int* tab, float* const* rb, int rank,
+                                              int pz) {
+  const ClSlots sl(L, rank);
+  const int zf = pz ? sl.zf[1] : sl.zf[0], n = pz ? sl.n[1] : sl.n[0];
+  const int nx = L.d.nx, ny = L.d.ny, hx = nx >> 1, hy = ny >> 1, z0 = L.zstart[rank];
+  const int cs = L.cs;
+  const int nw = (n + 31) & ~31;  // whole warps per case
+  const bool split = 3 * nw <= kClThreads;  // a lane per vertex and case, else per vertex
+  const int nthreads = split ? 3 * nw : nw;
+  if (int(threadIdx.x) >= nthreads) return;
+  auto vertex = [&](int t, int c) {
+    ClHalf V;
+    V.on = t < n;
+    if (!V.on) t = 0;
+    const int row = t / hx, i = t - row * hx, pk = row / hy, j = row - pk * hy;
+    const int z = zf + 2 * pk, s = (pz ? 4 * sl.n[0] : 0) + t;
+    V.n = n;
+    V.ss = L.ss;
+    V.ups = L.ups;
+    V.st = sm + L.st_off + s;
+    V.up = sm + L.u_off + c * L.ucs + (z - z0) * L.ups;  // local planes z - z0 .. + 2 are z - 1, z, z + 1
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      V.row[k] = wrapm(2 * j - 1 + k, ny) * L.urs;
+      V.xp[k] = cl_ux(L, wrapm(2 * i - 1 + k, nx));
+      V.f[k] = sm[L.f_off + c * cs + s + k * n];
+      V.inv[k] = sm[L.inv_off + s + k * n];
+    }
+    cl_ghosts(L, tab, rb, z, 0, V.g0, V.g1);
+    if (V.g0) V.g0 += c * L.ucs;
+    if (V.g1) V.g1 += c * L.ucs;
+    return V;
+  };
+  if (split) {
+    const int c = int(threadIdx.x) / nw;
+    const ClHalf V = vertex(int(threadIdx.x) - c * nw, c);
+    if (L.ss == kClSlots)
+      cl_half_run<kRev, kClSlots>(V, nthreads);
+    else
+      cl_half_run<kRev, 0>(V, nthreads);
+    return;
+  }
+  const ClHalf V = vertex(int(threadIdx.x), 0);
+  const int at = (pz ? 4 * sl.n[0] : 0) + (V.on ? int(threadIdx.x) : 0), ucs = L.ucs;
+  const float *fs = sm + L.f_off + at, *is = sm + L.inv_off + at;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    switch (kRev ? 3 - k : k) {
+      case 0: cl_half_pass3<0>(V, fs, is, cs, ucs); break;
+      case 1: cl_half_pass3<1>(V, fs, is, cs, ucs); break;
+      case 2: cl_half_pass3<2>(V, fs, is, cs, ucs); break;
+      default: cl_half_pass3<3>(V, fs, is, cs, ucs); break;
+    }
+    if (k < 3) asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  }
+}
+
+// Stencils in global memory: colours 0..3 of the planes of parity pz (3..0 when kRev), one lane per vertex
+// with its three cases, addresses and ghost targets found once for the four colours. A stencil value of the
+// next colour is loaded into its register as soon as the current colour has used it, so a pass waits on
+// shared memory and not on L2.
+template <int q, int qn>
+__device__ __forceinline__ void cl_half_pass_global(const ClHalf& V, int ucs, const float* sp, const float* f,
+                                                    int nsub, int nv, int nx, float (&st)[27], float (&fv)[3]) {
+  constexpr int cx = q & 1, cy = q >> 1;
+  const float inv = 1.0f / st[13], f0 = fv[0], f1 = fv[1], f2 = fv[2];
+  float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+  for (int o = 0; o < 27; o++) {
+    if (o != 13) {
+      const float* u = V.up + (o / 9) * V.ups + V.row[cy + (o / 3) % 3] + V.xp[cx + o % 3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) acc[c] += st[o] * u[c * ucs];
+    }
+    if (qn >= 0) st[o] = ld_issue(sp + (qn * nsub + o * nv));
+  }
+  if (qn >= 0)
+#pragma unroll
+    for (int c = 0; c < 3; c++) fv[c] = ld_issue(f + (c * nv + (qn >> 1) * nx + (qn & 1)));
+  const int p = V.row[cy + 1] + V.xp[cx + 1];
+  const float v[3] = {(f0 - acc[0]) * inv, (f1 - acc[1]) * inv, (f2 - acc[2]) * inv};
+  if (V.on) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      V.up[V.ups + p + c * ucs] = v[c];
+      if (V.g0) V.g0[p + c * ucs] = v[c];
+      if (V.g1) V.g1[p + c * ucs] = v[c];
+    }
+  }
+}
+
+template <bool kRev>
+__device__ __forceinline__ void cl_half_global(const ClLevel& L, const float* __restrict__ f_glob, float* sm,
+                                               const int* tab, float* const* rb, int rank, int pz) {
+  const ClSlots sl(L, rank);
+  const int zf = pz ? sl.zf[1] : sl.zf[0], n = pz ? sl.n[1] : sl.n[0];
+  const int nx = L.d.nx, ny = L.d.ny, hx = nx >> 1, hy = ny >> 1, z0 = L.zstart[rank];
+  const int nthreads = (n + 31) & ~31;
+  if (int(threadIdx.x) >= nthreads) return;
+  ClHalf V;
+  V.on = int(threadIdx.x) < n;
+  const int t = V.on ? int(threadIdx.x) : 0;
+  const int row = t / hx, i = t - row * hx, pk = row / hy, j = row - pk * hy, z = zf + 2 * pk;
+  V.ups = L.ups;
+  V.up = sm + L.u_off + (z - z0) * L.ups;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    V.row[k] = wrapm(2 * j - 1 + k, ny) * L.urs;
+    V.xp[k] = cl_ux(L, wrapm(2 * i - 1 + k, nx));
+  }
+  cl_ghosts(L, tab, rb, z, 0, V.g0, V.g1);
+  const int nv = int(L.d.nv()), nsub = nv >> 3;  // at most kClMaxNv
+  const float* sp = L.st + (4 * pz * nsub + (zf >> 1) * hx * hy + t);
+  const float* f = f_glob + ((z * ny + 2 * j) * nx + 2 * i);
+  const int ucs = L.ucs;
+  constexpr int q0 = kRev ? 3 : 0;
+  float st[27], fv[3];
+#pragma unroll
+  for (int o = 0; o < 27; o++) st[o] = ld_issue(sp + (q0 * nsub + o * nv));
+#pragma unroll
+  for (int c = 0; c < 3; c++) fv[c] = ld_issue(f + (c * nv + (q0 >> 1) * nx + (q0 & 1)));
+  cl_half_pass_global<(kRev ? 3 : 0), (kRev ? 2 : 1)>(V, ucs, sp, f, nsub, nv, nx, st, fv);
+  asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  cl_half_pass_global<(kRev ? 2 : 1), (kRev ? 1 : 2)>(V, ucs, sp, f, nsub, nv, nx, st, fv);
+  asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  cl_half_pass_global<(kRev ? 1 : 2), (kRev ? 0 : 3)>(V, ucs, sp, f, nsub, nv, nx, st, fv);
+  asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  cl_half_pass_global<(kRev ? 0 : 3), -1>(V, ucs, sp, f, nsub, nv, nx, st, fv);
+}
+
+// Half a sweep of a level: colours 0-3 update the even planes, 4-7 the odd ones, and a pass's changing
+// neighbours are in its own plane, so the passes of a half need only the CTA's barriers; the cluster
+// barrier after it makes the planes visible to the neighbouring CTAs.
+template <bool kRev, typename Cluster>
+__device__ __forceinline__ void cl_half(const ClLevel& L, const float* f_glob, float* sm, const int* tab,
+                                        float* const* rb, int rank, int pz, Cluster& cluster) {
+  if (L.st_off >= 0)
+    cl_half_sweep<kRev>(L, sm, tab, rb, rank, pz);
   else
-    cl_gs_t<true, 0>(L, f_glob, sm, tab, rb, rank, color);
+    cl_half_global<kRev>(L, f_glob, sm, tab, rb, rank, pz);
+  cluster.sync();
 }
 
-// r = f - A u on this CTA's vertices (resid_coarse_body, the sum formed by a lane team).
-template <bool kSmemSt, int kTwl>
-__device__ __forceinline__ void cl_resid_t(const ClLevel& L, const float* __restrict__ f_glob, float* sm,
-                                           int rank) {
+// r = f - A u on this CTA's vertices (resid_coarse_body): stencils in global memory, one lane per vertex.
+__device__ __forceinline__ void cl_resid_global(const ClLevel& L, const float* __restrict__ f_glob, float* sm,
+                                                int rank) {
   const Dims d = L.d;
   const int nx = d.nx, ny = d.ny, plane = nx * ny;
   const int z0 = L.zstart[rank], z1 = L.zstart[rank + 1];
   const int lnx = L.lnx, lny = L.lny;
   const int n = (z1 - z0) << (lnx + lny);
-  if (n == 0) return;  // uniform over the CTA
-  const int cs = L.cs, ucs = L.ucs, urs = L.urs, ups = L.ups;
-  const int u_off = L.u_off, f_off = L.f_off, r_off = L.r_off, st_off = L.st_off;
-  const float* st_glob = L.st;
-  float* rg = L.rg;
+  const int ucs = L.ucs, urs = L.urs, ups = L.ups;
   const size_t nv = d.nv();
-  const int total = ((n << kTwl) + 31) & ~31;  // whole warps only
-  for (int g = threadIdx.x; g < total; g += blockDim.x) {
-    const int t0 = g >> kTwl, lane = g & ((1 << kTwl) - 1);
-    const int x0 = t0 & ((1 << lnx) - 1), y0i = (t0 >> lnx) & ((1 << lny) - 1), zl0 = t0 >> (lnx + lny);
-    const bool active = t0 < n && x0 < nx && y0i < ny;
-    const int x = active ? x0 : 0, y = active ? y0i : 0, zl = active ? zl0 : 0;
-    const int z = z0 + zl;
-    const int xm = wrapm(x - 1, nx), xp = wrapm(x + 1, nx);
-    const int ym = wrapm(y - 1, ny) * urs, y0 = y * urs, yp = wrapm(y + 1, ny) * urs;
-    const float* uz = sm + u_off + zl * ups;
-    const float* const pu[3] = {uz, uz + ups, uz + 2 * ups};
-    const int lidx = zl * plane + y * nx + x;
-    const float* sp = kSmemSt ? sm + st_off + lidx * 27 : st_glob + cb_index(d, x, y, z);
-    const size_t sstride = kSmemSt ? size_t(1) : nv;
-    float acc[3];
-    cl_apply_team<kSmemSt, false, (1 << kTwl)>(sp, sstride, pu, xm, x, xp, ym, y0, yp, ucs, lane, acc);
-    if (active && lane == 0) {
-      const size_t gi = size_t(z) * plane + y * nx + x;
-      float fv[3];  // all loads before the first store
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const int x = t & ((1 << lnx) - 1), y = (t >> lnx) & ((1 << lny) - 1), zl = t >> (lnx + lny), z = z0 + zl;
+    if (x >= nx || y >= ny) continue;
+    const int xo[3] = {cl_ux(L, wrapm(x - 1, nx)), cl_ux(L, x), cl_ux(L, wrapm(x + 1, nx))};
+    const int yo[3] = {wrapm(y - 1, ny) * urs, y * urs, wrapm(y + 1, ny) * urs};
+    const float* u = sm + L.u_off + zl * ups;
+    const float* sp = L.st + cb_index(d, x, y, z);
+    const size_t gi = size_t(z) * plane + y * nx + x;
+    float st[27], fv[3], acc[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-      for (int c = 0; c < 3; c++) fv[c] = f_off >= 0 ? sm[f_off + c * cs + lidx] : __ldg(f_glob + c * nv + gi);
+    for (int o = 0; o < 27; o++) st[o] = ld_issue(sp + o * nv);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        if (r_off >= 0)
-          sm[r_off + c * cs + lidx] = fv[c] - acc[c];
-        else
-          rg[c * nv + gi] = fv[c] - acc[c];
-      }
+    for (int c = 0; c < 3; c++) fv[c] = ld_issue(f_glob + c * nv + gi);
+#pragma unroll
+    for (int o = 0; o < 27; o++) {
+      const float* q = u + (o / 9) * ups + yo[(o / 3) % 3] + xo[o % 3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) acc[c] += st[o] * q[c * ucs];
     }
+#pragma unroll
+    for (int c = 0; c < 3; c++) L.rg[c * nv + gi] = fv[c] - acc[c];
+  }
+}
+
+// The same with the stencils in shared memory: one lane per vertex and load case, in slot order.
+__device__ __forceinline__ void cl_resid_smem(const ClLevel& L, float* sm, int rank) {
+  const Dims d = L.d;
+  const int nx = d.nx, ny = d.ny, hx = nx >> 1, hy = ny >> 1, z0 = L.zstart[rank];
+  const ClSlots sl(L, rank);
+  const int cs = L.cs, urs = L.urs, ups = L.ups, total = sl.total();
+  for (int g = threadIdx.x; g < 3 * total; g += blockDim.x) {
+    const int c = g >= 2 * total ? 2 : (g >= total ? 1 : 0), s = g - c * total;
+    const int pz = s >= 4 * sl.n[0], q = s - (pz ? 4 * sl.n[0] : 0), n = pz ? sl.n[1] : sl.n[0];
+    const int cxy = q >= 2 * n ? (q >= 3 * n ? 3 : 2) : (q >= n ? 1 : 0), t = q - cxy * n;
+    const int row = t / hx, i = t - row * hx, pk = row / hy, j = row - pk * hy;
+    const int x = 2 * i + (cxy & 1), y = 2 * j + (cxy >> 1), zl = (pz ? sl.zf[1] : sl.zf[0]) + 2 * pk - z0;
+    const int xo[3] = {cl_ux(L, wrapm(x - 1, nx)), cl_ux(L, x), cl_ux(L, wrapm(x + 1, nx))};
+    const int yo[3] = {wrapm(y - 1, ny) * urs, y * urs, wrapm(y + 1, ny) * urs};
+    const float* u = sm + L.u_off + c * L.ucs + zl * ups;
+    const float* sp = sm + L.st_off + s;
+    float acc = 0.f;
+#pragma unroll
+    for (int o = 0; o < 27; o++) acc += sp[o * L.ss] * u[(o / 9) * ups + yo[(o / 3) % 3] + xo[o % 3]];
+    sm[L.r_off + c * cs + zl * nx * ny + y * nx + x] = sm[L.f_off + c * cs + s] - acc;
   }
 }
 
 __device__ __forceinline__ void cl_resid(const ClLevel& L, const float* f_glob, float* sm, int rank) {
   if (L.st_off < 0)
-    cl_resid_t<false, 0>(L, f_glob, sm, rank);
-  else if (L.tw_res >= 3)
-    cl_resid_t<true, 3>(L, f_glob, sm, rank);
+    cl_resid_global(L, f_glob, sm, rank);
   else
-    cl_resid_t<true, 0>(L, f_glob, sm, rank);
+    cl_resid_smem(L, sm, rank);
 }
 
 // u = 0 on this CTA's planes of a level, ghost copies included.
@@ -266,35 +455,30 @@ __device__ __forceinline__ void cl_restrict(const ClLevel& F, const ClLevel& C, 
   const Dims df = F.d, dc = C.d;
   const int pc = dc.nx * dc.ny, pf = df.nx * df.ny;
   const int Z0 = C.zstart[rank], Z1 = C.zstart[rank + 1];
+  const ClSlots sl(C, rank);
+  // one lane per coarse vertex and load case: 27 loads, most of them from other CTAs, in flight each
   const int n = (Z1 - Z0) * pc;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+  for (int g = threadIdx.x; g < 3 * n; g += blockDim.x) {
+    const int c = g / n, t = g - c * n;
     const int Zl = t / pc, rem = t - Zl * pc, Y = rem / dc.nx, X = rem - Y * dc.nx, Z = Z0 + Zl;
     const int xs[3] = {wrapm(2 * X - 1, df.nx), 2 * X, wrapm(2 * X + 1, df.nx)};
     const int ys[3] = {wrapm(2 * Y - 1, df.ny), 2 * Y, wrapm(2 * Y + 1, df.ny)};
     const int zs[3] = {wrapm(2 * Z - 1, df.nz), 2 * Z, wrapm(2 * Z + 1, df.nz)};
     const float* pr[3];
-    int cstride;
-    if (F.r_off >= 0) {
-      cstride = F.cs;
 #pragma unroll
-      for (int k = 0; k < 3; k++) pr[k] = cl_plane(F, tab, rb, F.r_off, zs[k]);
-    } else {
-      cstride = int(df.nv());
-#pragma unroll
-      for (int k = 0; k < 3; k++) pr[k] = F.rg + size_t(zs[k]) * pf;
-    }
-    float acc[3] = {0.f, 0.f, 0.f};
+    for (int k = 0; k < 3; k++)
+      pr[k] = F.r_off >= 0 ? cl_plane(F, tab, rb, F.r_off, zs[k]) + c * F.cs
+                           : F.rg + size_t(c) * df.nv() + size_t(zs[k]) * pf;
+    float acc = 0.f;
 #pragma unroll
     for (int o = 0; o < 27; o++) {
       const int ox = o % 3 - 1, oy = (o / 3) % 3 - 1, oz = o / 9 - 1;
       const float w = (ox ? 0.5f : 1.f) * (oy ? 0.5f : 1.f) * (oz ? 0.5f : 1.f);
       const float* q = pr[oz + 1] + ys[oy + 1] * df.nx + xs[ox + 1];
       // a global residual was written by other CTAs of this launch: read it past L1
-#pragma unroll
-      for (int c = 0; c < 3; c++) acc[c] += w * (F.r_off >= 0 ? q[c * cstride] : __ldcg(q + c * cstride));
+      acc += w * (F.r_off >= 0 ? *q : __ldcg(q));
     }
-#pragma unroll
-    for (int c = 0; c < 3; c++) sm[C.f_off + c * C.cs + t] = acc[c];
+    sm[C.f_off + c * C.cs + (C.st_off >= 0 ? sl.slot(C, X, Y, Z) : t)] = acc;
   }
   cl_zero_u(C, sm, rank);
 }
@@ -326,6 +510,7 @@ __device__ __forceinline__ void cl_coarsest(const ClDesc& cd, float* sm, const i
   for (int t = warp; t < nown; t += int(blockDim.x >> 5)) {
     const int i = z0 * pc + t;  // lexicographic coarsest index
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+#pragma unroll 4
     for (int j = lane; j < n; j += 32) {
       const double m = __ldg(cd.Ainv + size_t(i) * n + j);  // symmetric: row i == column i
       a0 += m * (double(g[j]) - m0);
@@ -340,7 +525,7 @@ __device__ __forceinline__ void cl_coarsest(const ClDesc& cd, float* sm, const i
     }
     if (lane == 0) {
       const int zl = t / pc, rem = t - zl * pc, y = rem / C.d.nx, x = rem - y * C.d.nx;
-      float* u = sm + C.u_off + (zl + 1) * C.ups + y * C.urs + x;  // own planes start at local plane 1
+      float* u = sm + C.u_off + (zl + 1) * C.ups + y * C.urs + cl_ux(C, x);  // own planes start at local plane 1
       u[0] = float(a0);
       u[C.ucs] = float(a1);
       u[2 * C.ucs] = float(a2);
@@ -354,8 +539,10 @@ __device__ __forceinline__ void cl_prolong(const ClLevel& F, const ClLevel& C, f
   const Dims df = F.d, dc = C.d;
   const int pf = df.nx * df.ny;
   const int z0 = F.zstart[rank], z1 = F.zstart[rank + 1];
+  // one lane per fine vertex and load case
   const int n = (z1 - z0) * pf;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+  for (int g = threadIdx.x; g < 3 * n; g += blockDim.x) {
+    const int c = g >= 2 * n ? 2 : (g >= n ? 1 : 0), t = g - c * n;
     const int zl = t / pf, rem = t - zl * pf, y = rem / df.nx, x = rem - y * df.nx, z = z0 + zl;
     const int X0 = x >> 1, Y0 = y >> 1, Z0 = z >> 1;
     const int X1 = (x & 1) ? wrapm(X0 + 1, dc.nx) : X0;
@@ -363,49 +550,24 @@ __device__ __forceinline__ void cl_prolong(const ClLevel& F, const ClLevel& C, f
     const int Z1 = (z & 1) ? wrapm(Z0 + 1, dc.nz) : Z0;
     const float wx1 = (x & 1) ? 0.5f : 0.f, wy1 = (y & 1) ? 0.5f : 0.f, wz1 = (z & 1) ? 0.5f : 0.f;
     const float wx0 = 1.f - wx1, wy0 = 1.f - wy1, wz0 = 1.f - wz1;
-    const float* p0 = cl_uplane(C, tab, rb, Z0);
-    const float* p1 = cl_uplane(C, tab, rb, Z1);
+    const float* u0 = cl_uplane(C, tab, rb, Z0) + c * C.ucs;
+    const float* u1 = cl_uplane(C, tab, rb, Z1) + c * C.ucs;
     const int r0 = Y0 * C.urs, r1 = Y1 * C.urs;
-    const int pu_idx = y * F.urs + x;
-    // every load (coarse values, possibly in other CTAs, the old fine values and the ghost
+    const int pu_idx = y * F.urs + cl_ux(F, x), p0 = cl_ux(C, X0), p1 = cl_ux(C, X1);
+    // every load (coarse values, possibly in other CTAs, the old fine value and the ghost
     // targets) before the first store
-    float a[3], uo[3];
-    float* uf = sm + F.u_off + (zl + 1) * F.ups + pu_idx;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float* u0 = p0 + c * C.ucs;
-      const float* u1 = p1 + c * C.ucs;
-      a[c] = wz0 * (wy0 * (wx0 * u0[r0 + X0] + wx1 * u0[r0 + X1]) +
-                    wy1 * (wx0 * u0[r1 + X0] + wx1 * u0[r1 + X1])) +
-             wz1 * (wy0 * (wx0 * u1[r0 + X0] + wx1 * u1[r0 + X1]) +
-                    wy1 * (wx0 * u1[r1 + X0] + wx1 * u1[r1 + X1]));
-      uo[c] = uf[c * F.ucs];
-    }
+    float* uf = sm + F.u_off + c * F.ucs + (zl + 1) * F.ups + pu_idx;
+    const float a = wz0 * (wy0 * (wx0 * u0[r0 + p0] + wx1 * u0[r0 + p1]) +
+                           wy1 * (wx0 * u0[r1 + p0] + wx1 * u0[r1 + p1])) +
+                    wz1 * (wy0 * (wx0 * u1[r0 + p0] + wx1 * u1[r0 + p1]) +
+                           wy1 * (wx0 * u1[r1 + p0] + wx1 * u1[r1 + p1]));
     float *g0, *g1;
     cl_ghosts(F, tab, rb, z, pu_idx, g0, g1);
-    const int fucs = F.ucs;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float v = uo[c] + a[c];
-      uf[c * fucs] = v;
-      if (g0) g0[c * fucs] = v;
-      if (g1) g1[c * fucs] = v;
-    }
+    const float v = *uf + a;
+    *uf = v;
+    if (g0) g0[c * F.ucs] = v;
+    if (g1) g1[c * F.ucs] = v;
   }
-}
-
-// One colour pass (cl_gs) followed by the barrier that its successor in the sweep needs:
-// colours 0-3 update the even planes, 4-7 the odd ones, and a pass's changing neighbours are in
-// its own plane unless it ends a half (colour 3 or 4 last, going up or down), after which the
-// neighbouring CTAs' planes must be visible.
-template <typename Cluster>
-__device__ __forceinline__ void cl_gs_sync(const ClLevel& L, const float* f_glob, float* sm, const int* tab,
-                                           float* const* rb, int rank, int color, bool half_end, Cluster& cluster) {
-  cl_gs(L, f_glob, sm, tab, rb, rank, color);
-  if (half_end)
-    cluster.sync();
-  else
-    __syncthreads();
 }
 
 static __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
@@ -440,43 +602,40 @@ static __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
   // stencils of the other smoothed levels. One thread per own vertex, all of its loads in flight
   // before its stores (a copy of one element per round trip made this a chain of L2 latencies).
   cl_zero_u(cd.lv[0], sm, rank);
-  if (cd.lv[0].f_off >= 0) {
-    const ClLevel& V = cd.lv[0];
-    const int pl = V.d.nx * V.d.ny, z0 = V.zstart[rank];
-    const int n = (V.zstart[rank + 1] - z0) * pl;
-    const size_t nv = V.d.nv();
-    const float* fz = cd.f_in + size_t(z0) * pl;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      float v[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) v[c] = __ldg(fz + c * nv + t);
-#pragma unroll
-      for (int c = 0; c < 3; c++) sm[V.f_off + c * V.cs + t] = v[c];
-    }
-  }
   for (int l = 0; l < L - 1; l++) {
     const ClLevel& V = cd.lv[l];
     if (V.st_off < 0) continue;
-    const int nx = V.d.nx, pl = nx * V.d.ny, z0 = V.zstart[rank];
-    const int n = (V.zstart[rank + 1] - z0) * pl;
+    const ClSlots sl(V, rank);
+    const int hx = V.d.nx >> 1, hy = V.d.ny >> 1, per = hx * hy, cs = V.cs;
     const size_t nv = V.d.nv();
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      const int zl = t / pl, rem = t - zl * pl, y = rem / nx, x = rem - y * nx;
-      const float* src = V.st + cb_index(V.d, x, y, z0 + zl);
-      float a[27];
+    for (int s = threadIdx.x; s < sl.total(); s += blockDim.x) {
+      const int pz = s >= 4 * sl.n[0], q = s - (pz ? 4 * sl.n[0] : 0), n = pz ? sl.n[1] : sl.n[0];
+      const int cxy = q >= 2 * n ? (q >= 3 * n ? 3 : 2) : (q >= n ? 1 : 0), t = q - cxy * n;
+      const int zf = pz ? sl.zf[1] : sl.zf[0];
+      // a colour's vertices of the CTA's planes are consecutive in the global colour-blocked order too
+      const float* src = V.st + size_t(cxy + 4 * pz) * (nv >> 3) + size_t(zf >> 1) * per + t;
+      float a[27], f[3] = {0.f, 0.f, 0.f};
 #pragma unroll
       for (int o = 0; o < 27; o++) a[o] = __ldg(src + size_t(o) * nv);
-      float* dst = sm + V.st_off + t * 27;
+      if (l == 0) {
+        const int row = t / hx, i = t - row * hx, pk = row / hy, j = row - pk * hy;
+        const size_t gi = (size_t(zf + 2 * pk) * V.d.ny + 2 * j + (cxy >> 1)) * V.d.nx + 2 * i + (cxy & 1);
 #pragma unroll
-      for (int o = 0; o < 27; o++) dst[o] = a[o];
-      sm[V.inv_off + t] = 1.0f / a[13];
+        for (int c = 0; c < 3; c++) f[c] = __ldg(cd.f_in + c * nv + gi);
+      }
+      float* dst = sm + V.st_off + s;
+#pragma unroll
+      for (int o = 0; o < 27; o++) dst[o * V.ss] = a[o];
+      sm[V.inv_off + s] = 1.0f / a[13];
+      if (l == 0)
+#pragma unroll
+        for (int c = 0; c < 3; c++) sm[V.f_off + c * cs + s] = f[c];
     }
   }
   cluster.sync();
   for (int l = 0; l < L - 1; l++) {
     const ClLevel& F = cd.lv[l];
-    for (int s = 0; s < cd.pre; s++)
-      for (int c = 0; c < 8; c++) cl_gs_sync(F, cd.f_in, sm, tab, rb, rank, c, c == 3 || c == 7, cluster);
+    for (int s = 0; s < 2 * cd.pre; s++) cl_half<false>(F, cd.f_in, sm, tab, rb, rank, s & 1, cluster);
     cl_resid(F, cd.f_in, sm, rank);
     cluster.sync();
     cl_restrict(F, cd.lv[l + 1], sm, tab, rb, rank);
@@ -488,8 +647,7 @@ static __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
     const ClLevel& F = cd.lv[l];
     cl_prolong(F, cd.lv[l + 1], sm, tab, rb, rank);
     cluster.sync();
-    for (int s = 0; s < cd.post; s++)
-      for (int c = 7; c >= 0; c--) cl_gs_sync(F, cd.f_in, sm, tab, rb, rank, c, c == 4 || c == 0, cluster);
+    for (int s = 0; s < 2 * cd.post; s++) cl_half<true>(F, cd.f_in, sm, tab, rb, rank, 1 - (s & 1), cluster);
   }
   // no distributed access after the last barrier: write this CTA's planes of the correction
   {
@@ -501,7 +659,7 @@ static __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
       const size_t g = size_t(z0) * pl + t;
       const int zl = t / pl, rem = t - zl * pl, y = rem / T.d.nx, x = rem - y * T.d.nx;
 #pragma unroll
-      for (int c = 0; c < 3; c++) cd.u_out[c * nv + g] = sm[T.u_off + c * T.ucs + (zl + 1) * T.ups + y * T.urs + x];
+      for (int c = 0; c < 3; c++) cd.u_out[c * nv + g] = sm[T.u_off + c * T.ucs + (zl + 1) * T.ups + y * T.urs + cl_ux(T, x)];
     }
   }
 }
@@ -509,29 +667,37 @@ static __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
 // Host-side layout of the cluster part for the level dimensions dims[0..n-1] (the last one is
 // the coarsest). Returns the dynamic shared memory in bytes, or 0 when the levels do not fit
 // one cluster (then the per-level kernels are used).
-// Worst number of distinct shared-memory words per bank over the lane-team reads of u (teams of
-// 8 lanes at vertices x, x+2, x+4, x+6; lane k reads offset k + 8 round) for row stride rs
-// and plane stride ps.
-inline int cl_team_conflicts(int rs, int ps) {
-  int worst = 1;
-  for (int round = 0; round < 4; round++) {
-    int addr[32], na = 0;
-    for (int j = 0; j < 4; j++)
-      for (int lane = 0; lane < 8; lane++) {
-        const int o = lane + 8 * round;
-        if (o >= 27) continue;
-        const int a = 2 * j + (o / 9) * ps + ((o / 3) % 3) * rs + o % 3;
-        bool dup = false;
-        for (int q = 0; q < na; q++) dup = dup || addr[q] == a;
-        if (!dup) addr[na++] = a;
-      }
-    for (int b = 0; b < 32; b++) {
-      int cnt = 0;
-      for (int q = 0; q < na; q++) cnt += (addr[q] % 32) == b;
-      worst = std::max(worst, cnt);
-    }
+// Worst number of distinct shared-memory words per bank over the u reads of a warp: of a colour pass
+// (lanes over (x/2, y/2, plane/2); row stride rs, plane stride ps), and of the
+// residual's and the prolongation's natural order.
+inline int cl_worst_bank(const int* addr, int n) {
+  int in_bank[32][32], cnt[32] = {}, worst = 1;  // distinct words seen per bank
+  for (int q = 0; q < n; q++) {
+    const int b = addr[q] & 31;
+    bool dup = false;
+    for (int r = 0; r < cnt[b]; r++) dup = dup || in_bank[b][r] == addr[q];
+    if (dup) continue;
+    in_bank[b][cnt[b]++] = addr[q];
+    worst = std::max(worst, cnt[b]);
   }
   return worst;
+}
+inline int cl_pass_conflicts(const Dims& d, int rs, int ps) {
+  const int hx = d.nx / 2, hy = d.ny / 2;
+  int addr[32];
+  for (int t = 0; t < 32; t++) {
+    const int row = t / hx, i = t % hx, k = row / hy, j = row % hy;
+    addr[t] = i + 2 * j * rs + 2 * k * ps;
+  }
+  return cl_worst_bank(addr, 32);
+}
+inline int cl_row_conflicts(const Dims& d, int uh, int rs) {
+  int addr[32];
+  for (int t = 0; t < 32; t++) {
+    const int x = t % d.nx, y = t / d.nx;
+    addr[t] = ((x & 1) ? uh : 0) + (x >> 1) + y * rs;
+  }
+  return cl_worst_bank(addr, 32);
 }
 
 inline int cl_log2_ceil(int v) {
@@ -556,24 +722,40 @@ inline size_t cl_plan_try(const Dims* dims, int n, ClDesc* cd, bool first_smem) 
     for (int c = 0; c <= kCl; c++) V.zstart[c] = int((long long)c * d.nz / kCl);
     for (int c = 0; c < kCl; c++) maxpl = std::max(maxpl, V.zstart[c + 1] - V.zstart[c]);
     const int plane = d.nx * d.ny;
+    if (l < n - 1 && ((maxpl + 1) / 2) * (plane / 4) > kClThreads) return 0;  // a colour's lanes
     V.cs = maxpl * plane;
-    // u strides: padded on the lane-team levels so that a round of team reads is free of bank
-    // conflicts (smallest plane stride among the best), plain on the first level
+    V.lnx = cl_log2_ceil(d.nx);
+    V.lny = cl_log2_ceil(d.ny);
+    // u rows: the odd sites' place, row and plane strides with the fewest bank conflicts of a colour pass,
+    // then of the natural order (the smallest such strides); plain on the coarsest level
     const bool smem_st = l < n - 1 && (l > 0 || first_smem);
+    const int evens = (d.nx + 1) / 2;
+    V.uh = evens;
     V.urs = d.nx;
-    V.ups = plane;
-    if (smem_st) {
-      int best = cl_team_conflicts(V.urs, V.ups);
-      for (int px = 0; px <= 32 && best > 1; px++)
-        for (int py = 0; py < 64; py++) {
-          const int rs = d.nx + px, ps = rs * d.ny + py;
-          const int w = cl_team_conflicts(rs, ps);
-          if (w < best || (w == best && ps < V.ups)) {
+    if (l < n - 1) {
+      int best = INT_MAX;
+      for (int rs = d.nx; rs <= d.nx + 16 && best > 9; rs++) {
+        const int pass = 8 * cl_pass_conflicts(d, rs, rs * d.ny);
+        for (int uh = evens; uh <= rs - d.nx / 2 && best > 9 && pass < best; uh++) {
+          const int w = pass + cl_row_conflicts(d, uh, rs);
+          if (w < best) {
             best = w;
+            V.uh = uh;
             V.urs = rs;
-            V.ups = ps;
           }
         }
+      }
+    }
+    V.ups = V.urs * d.ny;
+    if (l < n - 1 && plane / 4 < 32) {  // a warp spans planes
+      int best = cl_pass_conflicts(d, V.urs, V.ups);
+      for (int py = 1; py < 32 && best > 1; py++) {
+        const int w = cl_pass_conflicts(d, V.urs, V.urs * d.ny + py);
+        if (w < best) {
+          best = w;
+          V.ups = V.urs * d.ny + py;
+        }
+      }
     }
     V.ucs = (maxpl + 2) * V.ups;
     V.u_off = off;
@@ -587,19 +769,14 @@ inline size_t cl_plan_try(const Dims* dims, int n, ClDesc* cd, bool first_smem) 
     if (smem_st) {
       V.r_off = off;
       off += 3 * V.cs;
+      V.ss = std::max(V.cs, V.cs <= kClSlots ? kClSlots : 0);
       V.st_off = off;
-      off += 27 * V.cs;
+      off += 27 * V.ss;
       V.inv_off = off;
       off += V.cs;
     }
     V.tab_off = tab;
     tab += 3 * d.nz;
-    V.lhx = cl_log2_ceil(std::max(1, d.nx / 2));
-    V.lhy = cl_log2_ceil(std::max(1, d.ny / 2));
-    V.lnx = cl_log2_ceil(d.nx);
-    V.lny = cl_log2_ceil(d.ny);
-    // residual: 8 lanes per vertex where that fills about one round of the CTA's threads
-    V.tw_res = (((maxpl << (V.lnx + V.lny)) << 3) <= 2 * kClThreads) ? 3 : 0;
   }
   cd->nlev = n;
   cd->nc = int(dims[n - 1].nv());
