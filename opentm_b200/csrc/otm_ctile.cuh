@@ -273,4 +273,168 @@ __global__ void __launch_bounds__(kCThreads)
   }
 }
 
+// ---- few tiles: stencils in shared memory, a lane per vertex and load case --------------------------
+// With at most one tile per SM the sweep above is bound by the length of a warp's instruction chain (one
+// warp per scheduler stages 14 sites and takes eight passes of three cases) and by eight L2 latencies. Here
+// a CTA has 384 threads, one per vertex of a colour and load case; it first starts the copies of the
+// stencils of all eight colours (108 KB, cp.async of 16 bytes: a row of 8 vertices of a colour is 32
+// contiguous bytes of the colour-blocked array, in two halves because a shifted tile may wrap between
+// them), one group per colour in the order of the passes, and the staging of u and the earlier passes run
+// while they land. The sites are kept case by case with rows of 20 words, even and odd sites apart: the
+// lanes of a pass (8 sites of 4 rows two apart) read 32 different banks. Arithmetic and order are those of
+// k_ctile_sweep.
+constexpr int kCSmallThreads = 3 * kCThreads;
+constexpr int kCSmallRow = 20, kCSmallPlane = kCSmallRow * kCSY, kCSmallCase = kCSmallPlane * kCSZ;  // 2000 floats
+constexpr int kCSmallStencils = 8 * 27 * kCThreads;
+constexpr size_t kCSmallSmem = size_t(kCSmallStencils + 3 * kCSmallCase) * sizeof(float);  // 134,592 B
+constexpr size_t kCSmallSmemProlong = kCSmallSmem + size_t(3 * kCCSites) * sizeof(float);
+constexpr unsigned kCSmallTiles = 148;
+
+__device__ __forceinline__ int cspos(int lx, int ly, int lz) {
+  return lz * kCSmallPlane + ly * kCSmallRow + ((lx & 1) ? kCSHalf + (lx >> 1) : (lx >> 1));
+}
+
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// Pass number P of the sweep: the lane's vertex (i, j, k) of the pass's colour, case plane u of the sites,
+// stencils at st (27 x 128 per colour), its right-hand side f. Waits for its colour's copies.
+template <int P, bool kReverse>
+__device__ __forceinline__ void ctile_small_pass(float* u, const float* st, float f, int i, int j, int k) {
+  constexpr int C = kReverse ? 7 - P : P, CX = C & 1, CY = (C >> 1) & 1, CZ = C >> 2;
+  constexpr int oL = (CX == 0) ? -kCSHalf : kCSHalf - 1, oR = (CX == 0) ? -kCSHalf + 1 : kCSHalf;
+  asm volatile("cp.async.wait_group %0;" ::"n"(7 - P) : "memory");
+  __syncthreads();  // the copies of every thread, and the previous pass
+  const float* sp = st + C * 27 * kCThreads + i + 8 * j + 32 * k;
+  float* b = u + cspos(1 + 2 * i + CX, 1 + 2 * j + CY, 1 + 2 * k + CZ);
+  float acc = f;
+#pragma unroll
+  for (int o = 0; o < 27; o++) {
+    if (o == 13) continue;
+    const int ox = o % 3 - 1, oy = (o / 3) % 3 - 1, oz = o / 9 - 1;
+    acc -= sp[o * kCThreads] * b[(ox < 0 ? oL : (ox > 0 ? oR : 0)) + oy * kCSmallRow + oz * kCSmallPlane];
+  }
+  *b = acc * (1.0f / sp[13 * kCThreads]);
+}
+
+template <int kStart, bool kReverse>
+__global__ void __launch_bounds__(kCSmallThreads, 1)
+    k_ctile_sweep_small(Dims d, Dims dc, const float* __restrict__ st, const float* __restrict__ u_in,
+                        const float* __restrict__ uc, float* __restrict__ u_out, const float* __restrict__ f, int shift,
+                        const SolveScalars* sc) {
+  extern __shared__ float4 csm_small[];
+  float* st_sm = reinterpret_cast<float*>(csm_small);
+  float* sites = st_sm + kCSmallStencils;
+  float* cb = sites + 3 * kCSmallCase;
+  const int t = int(threadIdx.x), warp = t >> 5, lane = t & 31;
+  int x0, y0, z0;
+  ctile_origin(d, blockIdx.x, shift, x0, y0, z0);
+  const size_t nv = d.nv(), nsub = nv >> 3;
+  pdl_wait();
+  if (sc && solve_done(sc)) return;
+  {
+    // lane: row r = j + 4 k of a colour's 8 x 4 x 4 vertices and half h of the row; the 12 warps take the
+    // (pass, offset) pairs q = 27 p + o in turn
+    const int h = lane & 1, r = lane >> 1;
+    const int hx = d.nx >> 1, hy = d.ny >> 1, hz = d.nz >> 1;
+    const int X = wrapm(x0 / 2 + 4 * h, hx), Y = wrapm(y0 / 2 + (r & 3), hy), Z = wrapm(z0 / 2 + (r >> 2), hz);
+    const float* src = st + (size_t(X) + size_t(hx) * (size_t(Y) + size_t(hy) * Z));
+    float* dst = st_sm + r * 8 + h * 4;
+    int q = warp;
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+      const int c = kReverse ? 7 - p : p;
+#pragma unroll
+      for (int e = 0; e < 3; e++)
+        if (q < 27 * (p + 1)) {
+          const int o = q - 27 * p;
+          cp_async16(dst + (c * 27 + o) * kCThreads, src + size_t(o) * nv + c * nsub);
+          q += kCSmallThreads / 32;
+        }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+  }
+  // this lane's vertex (i, j, k) of a colour and its case; its right-hand side of every colour
+  const int i = lane & 7, j = lane >> 3, k = warp & 3, cs = warp >> 2;
+  float fr[8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const int X = wrapm(x0 + 2 * i + (c & 1), d.nx), Y = wrapm(y0 + 2 * j + ((c >> 1) & 1), d.ny),
+              Z = wrapm(z0 + 2 * k + (c >> 2), d.nz);
+    fr[c] = __ldg(f + cs * nv + size_t(X) + size_t(d.nx) * (size_t(Y) + size_t(d.ny) * Z));
+  }
+  // staging: all loads first, then the prolongation and the stores
+  constexpr int kSites = kCSX * kCSY * kCSZ, kItems = 3 * kSites, kSI = (kItems + kCSmallThreads - 1) / kCSmallThreads;
+  constexpr int kCI = (3 * kCCSites + kCSmallThreads - 1) / kCSmallThreads;
+  const int c0x = x0 / 2 - 1, c0y = y0 / 2 - 1, c0z = z0 / 2 - 1;
+  float uv[kSI];
+  if (kStart == kFromUProlong) {
+    const size_t nvc = dc.nv();
+    float cv[kCI];
+#pragma unroll
+    for (int it = 0; it < kCI; it++) {
+      const int q = t + it * kCSmallThreads, c = q / kCCSites, s = q - c * kCCSites;
+      const int ax = s % kCCX, ay = (s / kCCX) % kCCY, az = s / (kCCX * kCCY);
+      const int X = wrapm(c0x + ax, dc.nx), Y = wrapm(c0y + ay, dc.ny), Z = wrapm(c0z + az, dc.nz);
+      if (q < 3 * kCCSites) cv[it] = __ldg(uc + c * nvc + size_t(X) + size_t(dc.nx) * (size_t(Y) + size_t(dc.ny) * Z));
+    }
+#pragma unroll
+    for (int it = 0; it < kCI; it++) {
+      const int q = t + it * kCSmallThreads;
+      if (q < 3 * kCCSites) cb[q] = cv[it];
+    }
+  }
+#pragma unroll
+  for (int it = 0; it < kSI; it++) {
+    const int q = t + it * kCSmallThreads, c = q / kSites, s = q - c * kSites;
+    const int lx = s % kCSX, ly = (s / kCSX) % kCSY, lz = s / (kCSX * kCSY);
+    const size_t g = size_t(wrapm(x0 - 1 + lx, d.nx)) +
+                     size_t(d.nx) * (size_t(wrapm(y0 - 1 + ly, d.ny)) + size_t(d.ny) * wrapm(z0 - 1 + lz, d.nz));
+    uv[it] = kStart != kFromZero && q < kItems ? __ldg(u_in + c * nv + g) : 0.f;
+  }
+  if (kStart == kFromUProlong) __syncthreads();  // the coarser block
+#pragma unroll
+  for (int it = 0; it < kSI; it++) {
+    const int q = t + it * kCSmallThreads, c = q / kSites, s = q - c * kSites;
+    if (q >= kItems) continue;
+    const int lx = s % kCSX, ly = (s / kCSX) % kCSY, lz = s / (kCSX * kCSY);
+    float v = uv[it];
+    if (kStart == kFromUProlong) {
+      // the expression and weights of cprolong_site, one case
+      const int ux = x0 - 1 + lx, uy = y0 - 1 + ly, uz = z0 - 1 + lz;
+      const int ax0 = (ux >> 1) - c0x, ay0 = (uy >> 1) - c0y, az0 = (uz >> 1) - c0z;
+      const int ax1 = ax0 + (ux & 1), ay1 = ay0 + (uy & 1), az1 = az0 + (uz & 1);
+      const float wx1 = (ux & 1) ? 0.5f : 0.f, wy1 = (uy & 1) ? 0.5f : 0.f, wz1 = (uz & 1) ? 0.5f : 0.f;
+      const float wx0 = 1.f - wx1, wy0 = 1.f - wy1, wz0 = 1.f - wz1;
+      const float* b = cb + c * kCCSites;
+      const float* r00 = b + (ay0 + kCCY * az0) * kCCX;
+      const float* r10 = b + (ay1 + kCCY * az0) * kCCX;
+      const float* r01 = b + (ay0 + kCCY * az1) * kCCX;
+      const float* r11 = b + (ay1 + kCCY * az1) * kCCX;
+      v += wz0 * (wy0 * (wx0 * r00[ax0] + wx1 * r00[ax1]) + wy1 * (wx0 * r10[ax0] + wx1 * r10[ax1])) +
+           wz1 * (wy0 * (wx0 * r01[ax0] + wx1 * r01[ax1]) + wy1 * (wx0 * r11[ax0] + wx1 * r11[ax1]));
+    }
+    sites[c * kCSmallCase + cspos(lx, ly, lz)] = v;
+  }
+  float* u = sites + cs * kCSmallCase;
+  ctile_small_pass<0, kReverse>(u, st_sm, fr[kReverse ? 7 : 0], i, j, k);
+  ctile_small_pass<1, kReverse>(u, st_sm, fr[kReverse ? 6 : 1], i, j, k);
+  ctile_small_pass<2, kReverse>(u, st_sm, fr[kReverse ? 5 : 2], i, j, k);
+  ctile_small_pass<3, kReverse>(u, st_sm, fr[kReverse ? 4 : 3], i, j, k);
+  ctile_small_pass<4, kReverse>(u, st_sm, fr[kReverse ? 3 : 4], i, j, k);
+  ctile_small_pass<5, kReverse>(u, st_sm, fr[kReverse ? 2 : 5], i, j, k);
+  ctile_small_pass<6, kReverse>(u, st_sm, fr[kReverse ? 1 : 6], i, j, k);
+  ctile_small_pass<7, kReverse>(u, st_sm, fr[kReverse ? 0 : 7], i, j, k);
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < kCTX * kCTY * kCTZ / kCThreads; it++) {
+    const int s = (t - cs * kCThreads) + it * kCThreads;  // the lane's case
+    const int lx = 1 + s % kCTX, ly = 1 + (s / kCTX) % kCTY, lz = 1 + s / (kCTX * kCTY);
+    u_out[cs * nv + size_t(wrapm(x0 + lx - 1, d.nx)) +
+          size_t(d.nx) * (size_t(wrapm(y0 + ly - 1, d.ny)) + size_t(d.ny) * wrapm(z0 + lz - 1, d.nz))] =
+        u[cspos(lx, ly, lz)];
+  }
+}
+
 }  // namespace otm

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "otm_common.cuh"
@@ -354,6 +355,14 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
       if (!ctile_fits(lv[l].d)) continue;
       OTM_TRY(alloc((void**)&lv[l].u2, 3 * lv[l].d.nv() * sizeof(float)));
       lv[l].ctiled = true;
+      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromZero, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(kCSmallSmem)));
+      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromU, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(kCSmallSmem)));
+      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromU, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(kCSmallSmem)));
+      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromUProlong, true>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCSmallSmemProlong)));
     }
   }
   stats.levels = int(lv.size());
@@ -835,17 +844,43 @@ void Homo::vcycle_coarse_tiled(int l) {
   Level& L = lv[l];
   Level& C = lv[l + 1];
   const unsigned nt = ctile_count(L.d);
+  const bool small = nt <= kCSmallTiles;
   const int npre = cfg.pre_smooth, npost = cfg.post_smooth;
   const float* none = nullptr;
+  // one sweep, forward or reverse (`rev`), on tiling `shift`
+  auto sweep = [&](auto start, const float* in, const float* uc, float* out, int shift, bool rev) {
+    constexpr int kStart = decltype(start)::value;
+    constexpr size_t smem = kStart == kFromUProlong ? kCTileSmemProlong : kCTileSmem;
+    constexpr size_t smem_small = kStart == kFromUProlong ? kCSmallSmemProlong : kCSmallSmem;
+    const float *st = L.st, *f = L.f;
+    const SolveScalars* s = sc;
+    auto run_small = [&](auto kern) {
+      launch_pdl(kern, dim3(nt), dim3(kCSmallThreads), smem_small, stream, L.d, C.d, st, in, uc, out, f, shift, s);
+    };
+    if (!small) {
+      launch_pdl(k_ctile_sweep<kStart>, dim3(nt), dim3(kCThreads), smem, stream, L.d, C.d, st, in, uc, out, f, shift,
+                 rev ? 1 : 0, s);
+    } else if constexpr (kStart == kFromZero) {
+      run_small(k_ctile_sweep_small<kFromZero, false>);
+    } else if constexpr (kStart == kFromUProlong) {
+      run_small(k_ctile_sweep_small<kFromUProlong, true>);
+    } else {
+      if (rev)
+        run_small(k_ctile_sweep_small<kFromU, true>);
+      else
+        run_small(k_ctile_sweep_small<kFromU, false>);
+    }
+  };
+  constexpr std::integral_constant<int, kFromZero> from_zero{};
+  constexpr std::integral_constant<int, kFromU> from_u{};
+  constexpr std::integral_constant<int, kFromUProlong> from_prolong{};
   float* in = nullptr;
   for (int s = 0; s < npre; s++) {
     float* out = ((npre - 1 - s) % 2 == 0) ? L.u2 : L.u;
     if (s == 0)
-      launch_pdl(k_ctile_sweep<kFromZero>, dim3(nt), dim3(kCThreads), kCTileSmem, stream, L.d, C.d,
-                 (const float*)L.st, none, none, out, (const float*)L.f, 0, 0, (const SolveScalars*)sc);
+      sweep(from_zero, none, none, out, 0, false);
     else
-      launch_pdl(k_ctile_sweep<kFromU>, dim3(nt), dim3(kCThreads), kCTileSmem, stream, L.d, C.d, (const float*)L.st,
-                 (const float*)in, none, out, (const float*)L.f, s & 1, 0, (const SolveScalars*)sc);
+      sweep(from_u, in, none, out, s & 1, false);
     in = out;
   }
   const float* pre = in;
@@ -860,11 +895,9 @@ void Homo::vcycle_coarse_tiled(int l) {
     float* out = (s == npost - 1) ? L.u : (pin == L.r ? L.u2 : L.r);
     const int shift = (npost - 1 - s) & 1;
     if (s == 0)
-      launch_pdl(k_ctile_sweep<kFromUProlong>, dim3(nt), dim3(kCThreads), kCTileSmemProlong, stream, L.d, C.d,
-                 (const float*)L.st, pin, (const float*)C.u, out, (const float*)L.f, shift, 1, (const SolveScalars*)sc);
+      sweep(from_prolong, pin, C.u, out, shift, true);
     else
-      launch_pdl(k_ctile_sweep<kFromU>, dim3(nt), dim3(kCThreads), kCTileSmem, stream, L.d, C.d, (const float*)L.st,
-                 pin, none, out, (const float*)L.f, shift, 1, (const SolveScalars*)sc);
+      sweep(from_u, pin, none, out, shift, true);
     pin = out;
   }
   launched(npost);
