@@ -55,9 +55,21 @@ float objective(const float K[9], const double t[6], float dK[9]) {
 struct DeviceFields {
   float *rho = nullptr, *rho_f = nullptr, *k = nullptr, *dk = nullptr, *wsum = nullptr, *g_k = nullptr,
         *g_rho = nullptr, *dvdx = nullptr;
+  void* block = nullptr;  // one allocation for all of them
+  cudaError_t allocate(size_t ne, bool with_dvdx) {
+    const size_t n = (ne + 63) & ~size_t(63);  // 256-byte aligned fields
+    const cudaError_t e = cudaMalloc(&block, n * (with_dvdx ? 8 : 7) * sizeof(float));
+    if (e != cudaSuccess) return e;
+    float* p = static_cast<float*>(block);
+    for (float** f : {&rho, &rho_f, &k, &dk, &wsum, &g_k, &g_rho}) {
+      *f = p;
+      p += n;
+    }
+    if (with_dvdx) dvdx = p;
+    return e;
+  }
   ~DeviceFields() {
-    for (float* p : {rho, rho_f, k, dk, wsum, g_k, g_rho, dvdx})
-      if (p) cudaFree(p);
+    if (block) cudaFree(block);
   }
 };
 
@@ -307,8 +319,7 @@ otm_status otm_run_custom(const otm_driver_config* cfg, const float* rho0_host, 
     }
   } guard{s};
   DeviceFields F;
-  for (float** p : {&F.rho, &F.rho_f, &F.k, &F.dk, &F.wsum, &F.g_k, &F.g_rho})
-    OTM_CUDA(cudaMalloc((void**)p, ne * sizeof(float)));
+  OTM_CUDA(F.allocate(ne, cfg->model == OTM_MODEL_MMA));
 
   // Homogenization_H hom_H(config) with the run's solve tolerance
   otm_config hc;
@@ -386,7 +397,6 @@ otm_status otm_run_custom(const otm_driver_config* cfg, const float* rho0_host, 
     } mg{mma};
     OTM_TRY(otm_mma_set_stream(mma, s));
     OTM_TRY(otm_mma_set_bound_scalar(mma, 0.0001f, 1.0f));
-    OTM_CUDA(cudaMalloc((void**)&F.dvdx, ne * sizeof(float)));
     k_fill<<<ceil_div(ne, 256), 256, 0, s>>>(ne, float(1.0 / (double(n) * n * n)), F.dvdx);
     count_launches(1);
     for (int itn = 0; itn < cfg->max_iter; itn++) {

@@ -98,6 +98,8 @@ struct Homo {
   bool external = false;
   cudaMemPool_t pool = nullptr;
   std::vector<void*> allocations;
+  unsigned char* arena = nullptr;  // rest of the reserved block
+  size_t arena_left = 0;
   // the first iteration of a device-loop solve runs outside the loop graph and waits for the
   // side stream's coarse chain only before its first coarse level (set while it is launched)
   bool join_in_cycle = false;
@@ -120,6 +122,7 @@ struct Homo {
   otm_solve_stats stats{};
 
   ~Homo();
+  otm_status reserve(size_t bytes);
   otm_status alloc(void** p, size_t bytes);
   otm_status build(const otm_config& c, cudaStream_t ext_stream = nullptr, cudaMemPool_t ext_pool = nullptr,
                    bool external_mode = false);

@@ -405,9 +405,8 @@ otm_status field_means(const int reso[3], const float* a, const float* b, int pi
                        double out[2]) {
   const Dims d{reso[0], reso[1], reso[2]};
   double* dev = nullptr;
-  double* host = nullptr;
+  double host[2] = {0.0, 0.0};  // pageable: pinning 16 bytes costs more than their copy
   cudaError_t e = scratch_malloc((void**)&dev, (2 * kSumBlocks + 2) * sizeof(double), s);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&host, 2 * sizeof(double));
   if (e == cudaSuccess) {
     launch_mean(d, pitchT, a, 0, 0.f, 0.f, 0.f, dev, dev + 2 * kSumBlocks, s);
     launch_mean(d, pitchT, b, 0, 0.f, 0.f, 0.f, dev + kSumBlocks, dev + 2 * kSumBlocks + 1, s);
@@ -419,7 +418,6 @@ otm_status field_means(const int reso[3], const float* a, const float* b, int pi
     out[0] = host[0];
     out[1] = host[1];
   }
-  if (host) cudaFreeHost(host);
   if (e != cudaSuccess) return cuda_fail(e, "field mean");
   if (e2 != cudaSuccess) return cuda_fail(e2, "field mean");
   return OTM_OK;

@@ -38,6 +38,7 @@ struct MVec {
 struct MmaWork {
   size_t n = 0;
   int m = 0;
+  bool carved = false;  // the arrays lie in the owner's block
   double *alfa = nullptr, *beta = nullptr, *p0 = nullptr, *q0 = nullptr, *P = nullptr, *Q = nullptr;
   double *xs = nullptr, *xsi = nullptr, *eta = nullptr, *dx = nullptr, *dxsi = nullptr, *deta = nullptr;
   double* partials = nullptr;  // kMaxPartials * 96
@@ -654,30 +655,34 @@ __global__ void k_fill(size_t n, double v, double* a) {
   for (size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += size_t(gridDim.x) * blockDim.x) a[j] = v;
 }
 
-static otm_status work_alloc(MmaWork& w, int m, size_t n, cudaStream_t s, bool async) {
+// Device bytes of a subsolve's work arrays, every array 256-byte aligned.
+static size_t mma_padded(size_t doubles) { return (doubles * sizeof(double) + 255) & ~size_t(255); }
+static size_t mma_small_bytes() {
+  return size_t(kMaxPartials) * kMmaSlots * sizeof(double) + kMmaSlots * sizeof(double) + 64 + sizeof(MmaState);
+}
+static size_t work_bytes(int m, size_t n) {
+  return 10 * mma_padded(n) + 2 * mma_padded(size_t(m) * n) + mma_padded(mma_small_bytes() / sizeof(double) + 1);
+}
+
+// The work arrays carved out of `block` (work_bytes of it), or allocated one by one: from the scratch pool
+// when async, else with cudaMalloc.
+static otm_status work_alloc(MmaWork& w, int m, size_t n, cudaStream_t s, bool async, char* block = nullptr) {
   w.m = m;
   w.n = n;
+  w.carved = block != nullptr;
+  auto take = [&](void** p, size_t doubles) -> cudaError_t {
+    if (block) {
+      *p = block;
+      block += mma_padded(doubles);
+      return cudaSuccess;
+    }
+    const size_t bytes = doubles * sizeof(double);
+    return async ? scratch_malloc(p, bytes, s) : cudaMalloc(p, bytes);
+  };
   double** arr[] = {&w.alfa, &w.beta, &w.p0, &w.q0, &w.xs, &w.xsi, &w.eta, &w.dx, &w.dxsi, &w.deta};
-  for (double** a : arr) {
-    if (async)
-      OTM_CUDA(scratch_malloc((void**)a, n * sizeof(double), s));
-    else
-      OTM_CUDA(cudaMalloc((void**)a, n * sizeof(double)));
-  }
-  for (double** a : {&w.P, &w.Q}) {
-    if (async)
-      OTM_CUDA(scratch_malloc((void**)a, size_t(m) * n * sizeof(double), s));
-    else
-      OTM_CUDA(cudaMalloc((void**)a, size_t(m) * n * sizeof(double)));
-  }
-  const size_t small = size_t(kMaxPartials) * kMmaSlots * sizeof(double) + kMmaSlots * sizeof(double) + 64 +
-                       sizeof(MmaState);
-  char* buf = nullptr;
-  if (async)
-    OTM_CUDA(scratch_malloc((void**)&buf, small, s));
-  else
-    OTM_CUDA(cudaMalloc((void**)&buf, small));
-  w.partials = (double*)buf;
+  for (double** a : arr) OTM_CUDA(take((void**)a, n));
+  for (double** a : {&w.P, &w.Q}) OTM_CUDA(take((void**)a, size_t(m) * n));
+  OTM_CUDA(take((void**)&w.partials, mma_small_bytes() / sizeof(double) + 1));
   w.result = w.partials + size_t(kMaxPartials) * kMmaSlots;
   w.counter = (unsigned int*)(w.result + kMmaSlots);
   w.state = (MmaState*)(w.result + kMmaSlots + 8);
@@ -689,7 +694,7 @@ static otm_status work_alloc(MmaWork& w, int m, size_t n, cudaStream_t s, bool a
 static void work_free(MmaWork& w, cudaStream_t s, bool async) {
   double* arr[] = {w.alfa, w.beta, w.p0, w.q0, w.xs, w.xsi, w.eta, w.dx, w.dxsi, w.deta, w.P, w.Q, w.partials};
   for (double* a : arr)
-    if (a) {
+    if (a && !w.carved) {
       if (async)
         cudaFreeAsync(a, s);
       else
@@ -816,11 +821,13 @@ struct otm_mma {
   double *xvar = nullptr, *xmin = nullptr, *xmax = nullptr, *xold1 = nullptr, *xold2 = nullptr;
   double *low = nullptr, *upp = nullptr;
   MmaWork w;
+  char* block = nullptr;  // one allocation for all arrays, where it could be had
   ~otm_mma() {
     double* arr[] = {xvar, xmin, xmax, xold1, xold2, low, upp};
     for (double* p : arr)
-      if (p) cudaFree(p);
+      if (p && !block) cudaFree(p);
     work_free(w, nullptr, false);
+    if (block) cudaFree(block);
   }
 };
 
@@ -845,12 +852,23 @@ otm_status otm_mma_create(int m, int n, double a0, double a, double c, double d,
     return st;
   };
   double** arr[] = {&o->xvar, &o->xmin, &o->xmax, &o->xold1, &o->xold2, &o->low, &o->upp};
+  const size_t each = mma_padded(o->n);
+  if (cudaMalloc((void**)&o->block, 7 * each + work_bytes(m, o->n)) != cudaSuccess) {
+    cudaGetLastError();  // the arrays may still fit one by one
+    o->block = nullptr;
+  }
+  char* at = o->block;
   for (double** p : arr) {
-    cudaError_t e = cudaMalloc((void**)p, o->n * sizeof(double));
-    if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
+    if (at) {
+      *p = (double*)at;
+      at += each;
+    } else {
+      const cudaError_t e = cudaMalloc((void**)p, o->n * sizeof(double));
+      if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
+    }
     cudaMemset(*p, 0, o->n * sizeof(double));
   }
-  otm_status st = work_alloc(o->w, m, o->n, nullptr, false);
+  otm_status st = work_alloc(o->w, m, o->n, nullptr, false, at);
   if (st != OTM_OK) return fail(st);
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "otm_mma_create"));
   *out = o;
