@@ -1057,7 +1057,8 @@ void Homo::launch_solve_init() {
   k_rhs_mean<<<nb, kBlock, 0, stream>>>(d0, ks, ef, b, partials, means, &sc->counter[T_MEAN]);
   sc_host->tol = cfg.fem_rel_thres;
   cudaMemcpyAsync(&sc->tol, &sc_host->tol, sizeof(double), cudaMemcpyHostToDevice, stream);
-  k_init_residual<false><<<nb, kBlock, 0, stream>>>(d0, ks, op, x, b, means, lv[0].f, partials, sc);
+  k_init_residual<false, true><<<nb, kBlock, 0, stream>>>(d0, ks, op, x, b, means, lv[0].f, partials, sc);
+  x_zero = false;  // the solve that follows writes x
   launched(2);
 }
 
@@ -1183,11 +1184,11 @@ void Homo::launch_solve_start() {
     else
       k_resid64<false><<<nb, kBlock, 0, stream>>>(d0, ks, op, x64, b, lv[0].f, partials, sc, kmax_bits,
                                                   cfg.max_iter, 1);
-  } else if (face) {
-    k_init_residual<true><<<nb, kBlock, 0, stream>>>(d0, ks, op, x, b, means, lv[0].f, partials, sc);
   } else {
-    k_init_residual<false><<<nb, kBlock, 0, stream>>>(d0, ks, op, x, b, means, lv[0].f, partials, sc);
+    auto* kern = x_zero ? k_init_residual<false, true> : (face ? k_init_residual<true, false> : k_init_residual<false, false>);
+    kern<<<nb, kBlock, 0, stream>>>(d0, ks, op, x, b, means, lv[0].f, partials, sc);
   }
+  x_zero = false;  // the solve that follows writes x
   launched(mixed ? 3 : 2);
 }
 
@@ -1240,6 +1241,7 @@ otm_status Homo::solve_impl(bool with_heat) {
     if (!cfg.warm_start || attempt > 0) {
       OTM_CUDA(cudaMemsetAsync(x, 0, 3 * nv * sizeof(float), stream));
       if (mixed) OTM_CUDA(cudaMemsetAsync(x64, 0, 3 * nv * sizeof(double), stream));
+      x_zero = true;
     }
     if (device_loop) {
       OTM_TRY(launch_device_solve(with_heat));
@@ -1619,6 +1621,7 @@ otm_status otm_homo_set_solution(otm_homo* h, int lcase, const float* src_dev) {
   const size_t nv = H.lv[0].d.nv();
   OTM_TRY(H.enter());
   OTM_CUDA(cudaMemcpyAsync(H.x + lcase * nv, src_dev, nv * sizeof(float), cudaMemcpyDeviceToDevice, H.stream));
+  H.x_zero = false;
   if (H.mixed) {
     otm::k_x_to_x64<<<otm::ceil_div(nv, otm::kBlock), otm::kBlock, 0, H.stream>>>(nv, H.x + lcase * nv,
                                                                                  H.x64 + lcase * nv);
@@ -1633,6 +1636,7 @@ otm_status otm_homo_reset_displacement(otm_homo* h) {
   OTM_TRY(H.enter());
   OTM_CUDA(cudaMemsetAsync(H.x, 0, 3 * H.lv[0].d.nv() * sizeof(float), H.stream));
   if (H.mixed) OTM_CUDA(cudaMemsetAsync(H.x64, 0, 3 * H.lv[0].d.nv() * sizeof(double), H.stream));
+  H.x_zero = true;
   H.solved = false;
   return H.leave();
 }

@@ -71,6 +71,7 @@ struct Homo {
   float* kraw = nullptr;  // conductivity as imported
   float* b = nullptr;     // right-hand sides
   float* x = nullptr;     // solutions chi (kept for warm starts)
+  bool x_zero = false;    // x has been set to zero and not written since (in stream order)
   float* p = nullptr;
   float* q = nullptr;
   double* Ainv = nullptr;

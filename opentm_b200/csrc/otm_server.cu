@@ -684,6 +684,7 @@ static otm_status launch_on_lane(otm_server* s, Request& r, Lane& ln, size_t ci)
   OTM_CUDA(cudaMemcpyAsync(H.b, src, nv * sizeof(float), cudaMemcpyHostToDevice, ln.stream));
   OTM_TRY(H.update(H.b, r.reso[0]));
   OTM_CUDA(cudaMemsetAsync(H.x, 0, 3 * nv * sizeof(float), ln.stream));
+  H.x_zero = true;
   OTM_TRY(H.launch_device_solve(true));
   OTM_CUDA(cudaEventRecord(ln.done, ln.stream));
   ln.req = r.id;
