@@ -29,7 +29,7 @@ namespace otm {
 
 constexpr int kCl = 16;            // CTAs per cluster (non-portable size, opted in at set-up): one
                                    // 32^3 colour pass at 16 CTAs loads half the stencils per SM of 8
-constexpr int kClThreads = 512;
+constexpr int kClThreads = 512;    // 640: 2% slower on 32^3 and 40 x 56 x 72 solves, 4% faster on 96 x 128 x 64 V(1,1)
 constexpr int kClMaxLevels = 8;
 constexpr int kClMaxNv = 32768;    // unknowns of the first level handled by the cluster (32^3)
 constexpr int kClSlots = 256;      // stencil stride of the levels with at most that many vertices per CTA

@@ -283,6 +283,9 @@ __global__ void __launch_bounds__(kCThreads)
 // while they land. The sites are kept case by case with rows of 20 words, even and odd sites apart: the
 // lanes of a pass (8 sites of 4 rows two apart) read 32 different banks. Arithmetic and order are those of
 // k_ctile_sweep.
+// The four sweeps of a 32^3 level (32 tiles; from zero, from u, prolonging, reverse): 64.6 -> 47.7 us. Its
+// shared memory leaves one CTA per SM, so the line is at one tile per SM: a 64^3 level (256 tiles) takes
+// 91 us this way, as two rounds of CTAs, and 64 with k_ctile_sweep.
 constexpr int kCSmallThreads = 3 * kCThreads;
 constexpr int kCSmallRow = 20, kCSmallPlane = kCSmallRow * kCSY, kCSmallCase = kCSmallPlane * kCSZ;  // 2000 floats
 constexpr int kCSmallStencils = 8 * 27 * kCThreads;

@@ -303,7 +303,8 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
 }
 
 // Blocks of a launch with ny rows per thread and z chunks of zc planes, and the chunk to use: the longest
-// (least work on the 2H planes around it) that still gives the GPU enough blocks, at least 4.
+// (least work on the 2H planes around it) that still gives the GPU enough blocks, at least 4: eight of
+// 128 threads per SM, about what is resident at the kernel's registers.
 constexpr long long kConvFill = 8 * 148;
 static long long conv_blocks(const Dims& d, int ny, int zc) {
   return (long long)((d.nx + kTX - 1) / kTX) * ((d.ny + kTYT * ny - 1) / (kTYT * ny)) * ((d.nz + zc - 1) / zc);
@@ -402,8 +403,8 @@ __global__ void __launch_bounds__(256) k_product(Dims d, const float* __restrict
 
 // OCOptimizer::filterSens (optimization/OCOptimizer.cu:76-152): s_e <- sum w s_n rho_n / (sum w * rho_e)
 // over the periodic Linear neighbourhood, in place. The products s rho go to tmp (d.nv() floats)
-// first, so that the convolution can write s; at 128^3, radius 2: 1457 us with every tap read and
-// wrapped from global memory by each voxel and a copy back.
+// first, so that the convolution can write s. At 128^3, radius 2: products 9.5 us and convolution 25 us,
+// against 1457 us with every tap read and wrapped from global memory by each voxel and a copy back.
 otm_status oc_filter_run(const Dims& d, float* sens, const float* rho, size_t pitch, float* tmp, float radius,
                          cudaStream_t s) {
   ConvWeights cw;
