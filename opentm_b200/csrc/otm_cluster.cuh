@@ -15,6 +15,11 @@
 // neighbours lie in its own plane, held by its own CTA (CTA barriers between those passes). The arithmetic is that of the
 // per-level kernels in otm_mg_kernels.cuh except for the summation order of the 27-point
 // products; the coarsest solve is u = Ainv (f - mean f) as in k_coarsest_solve.
+//
+// The order of a vertex's 27 products is part of the results: a design run whose solves stop at a relative
+// residual of 0.01 carries a last-bit change of one cycle into densities that differ by 1e-4 after ten
+// steps. A colour pass sums the offsets 0..26 one after the other (three sums by plane, a shorter chain:
+// 128^3 OC steps 0.7 % faster, 32^3 solves not), a residual as cl_resid_smem says.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -50,6 +55,7 @@ struct ClLevel {
   int inv_off; // inverse diagonal per slot (with st_off >= 0)
   int tab_off; // plane tables of this level: nz ownership entries, then 2 nz ghost-push entries
   int lnx, lny;  // log2 of nx, ny rounded up (residual enumeration)
+  int res8;    // the residual's 27 products in eight sums (levels of few vertices per CTA), else in one
   int zstart[kCl + 1];  // CTA c holds planes [zstart[c], zstart[c+1])
   const float* st;
   float* rg;
@@ -164,16 +170,11 @@ __device__ __forceinline__ void cl_half_pass(const ClHalf& V) {
 #pragma unroll
   for (int o = 0; o < 27; o++)
     if (o != 13) st[o] = sp[o * ss];
-  float acc[3];  // one sum per plane: three short chains
+  float acc = 0.f;
 #pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const float* u = V.up + a * V.ups;
-    acc[a] = 0.f;
-#pragma unroll
-    for (int b = 0; b < 9; b++)
-      if (9 * a + b != 13) acc[a] += st[9 * a + b] * u[V.row[cy + b / 3] + V.xp[cx + b % 3]];
-  }
-  const float v = (V.f[q] - (acc[0] + acc[1] + acc[2])) * V.inv[q];
+  for (int o = 0; o < 27; o++)
+    if (o != 13) acc += st[o] * V.up[(o / 9) * V.ups + V.row[cy + (o / 3) % 3] + V.xp[cx + o % 3]];
+  const float v = (V.f[q] - acc) * V.inv[q];
   const int p = V.row[cy + 1] + V.xp[cx + 1];
   if (V.on) {
     V.up[V.ups + p] = v;
@@ -410,7 +411,9 @@ __device__ __forceinline__ void cl_resid_global(const ClLevel& L, const float* _
   }
 }
 
-// The same with the stencils in shared memory: one lane per vertex and load case, in slot order.
+// The same with the stencils in shared memory: one lane per vertex and load case, in slot order. kStride
+// sums, of the offsets k, k + kStride, ..., added pairwise at half the distance each time.
+template <int kStride>
 __device__ __forceinline__ void cl_resid_smem(const ClLevel& L, float* sm, int rank) {
   const Dims d = L.d;
   const int nx = d.nx, ny = d.ny, hx = nx >> 1, hy = ny >> 1, z0 = L.zstart[rank];
@@ -426,18 +429,26 @@ __device__ __forceinline__ void cl_resid_smem(const ClLevel& L, float* sm, int r
     const int yo[3] = {wrapm(y - 1, ny) * urs, y * urs, wrapm(y + 1, ny) * urs};
     const float* u = sm + L.u_off + c * L.ucs + zl * ups;
     const float* sp = sm + L.st_off + s;
-    float acc = 0.f;
+    float acc[kStride];
 #pragma unroll
-    for (int o = 0; o < 27; o++) acc += sp[o * L.ss] * u[(o / 9) * ups + yo[(o / 3) % 3] + xo[o % 3]];
-    sm[L.r_off + c * cs + zl * nx * ny + y * nx + x] = sm[L.f_off + c * cs + s] - acc;
+    for (int k = 0; k < kStride; k++) acc[k] = 0.f;
+#pragma unroll
+    for (int o = 0; o < 27; o++) acc[o % kStride] += sp[o * L.ss] * u[(o / 9) * ups + yo[(o / 3) % 3] + xo[o % 3]];
+#pragma unroll
+    for (int h = kStride >> 1; h > 0; h >>= 1)
+#pragma unroll
+      for (int k = 0; k < h; k++) acc[k] += acc[k + h];
+    sm[L.r_off + c * cs + zl * nx * ny + y * nx + x] = sm[L.f_off + c * cs + s] - acc[0];
   }
 }
 
 __device__ __forceinline__ void cl_resid(const ClLevel& L, const float* f_glob, float* sm, int rank) {
   if (L.st_off < 0)
     cl_resid_global(L, f_glob, sm, rank);
+  else if (L.res8)
+    cl_resid_smem<8>(L, sm, rank);
   else
-    cl_resid_smem(L, sm, rank);
+    cl_resid_smem<1>(L, sm, rank);
 }
 
 // u = 0 on this CTA's planes of a level, ghost copies included.
@@ -726,6 +737,7 @@ inline size_t cl_plan_try(const Dims* dims, int n, ClDesc* cd, bool first_smem) 
     V.cs = maxpl * plane;
     V.lnx = cl_log2_ceil(d.nx);
     V.lny = cl_log2_ceil(d.ny);
+    V.res8 = (maxpl << (V.lnx + V.lny)) <= kClThreads / 4;
     // u rows: the odd sites' place, row and plane strides with the fewest bank conflicts of a colour pass,
     // then of the natural order (the smallest such strides); plain on the coarsest level
     const bool smem_st = l < n - 1 && (l > 0 || first_smem);
