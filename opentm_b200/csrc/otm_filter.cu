@@ -67,7 +67,8 @@ static otm_status make_weights(int type, float radius, ConvWeights* cw) {
 // four, where a read per tap takes 27 and 93. The weight depends on the squared distance only, and with the
 // loops unrolled its place in the parameter bank is a constant, so a tap is one FMA. The radii in common
 // use (1.5 to 2, 2.5, 3, 3.5, 4) have their set of taps compiled in; others skip the zero weights by
-// branches that all threads take alike. An output's taps are summed in the reference's order (x fastest, z slowest; the adjoint streams z downwards for that).
+// branches that all threads take alike. An output's taps are summed in the reference's order (x fastest, z
+// slowest; the adjoint streams z downwards for that).
 //   MODE 0: forward            out = sum w src / sum_valid w
 //   MODE 1: forward + SIMP     also k = (k0 - kmin) out^p + kmin and dk = dk/dout
 //   MODE 2: adjoint            out = sum_off w g(i - off) / ws(i - off)
@@ -78,13 +79,11 @@ static otm_status make_weights(int type, float radius, ConvWeights* cw) {
 //   MODE 5: OC sensitivity     out = sum w src / (sum w * rho), rho (ws_in) pitched like out
 constexpr int kTX = 32, kTYT = 4, kConvThreads = kTX * kTYT;
 
-// A radial filter: weight by squared distance, zero from smax on; the sums of a whole z plane of weights
-// by |oz| (for the valid weight of voxels cut along z only).
+// A radial filter: weight by squared distance, zero from smax on.
 template <int H>
 struct Radial {
   float w[3 * H * H + 1];
   int smax;
-  float plane[H + 1];
 };
 
 template <int H>
@@ -92,15 +91,48 @@ static void make_radial(const ConvWeights& cw, Radial<H>* r) {
   constexpr int W1 = 2 * H + 1;
   for (float& w : r->w) w = 0.f;
   r->smax = 0;
-  for (int k = 0; k <= H; k++) {
-    r->plane[k] = 0.f;
+  for (int k = 0; k <= H; k++)
     for (int oy = -H; oy <= H; oy++)
       for (int ox = -H; ox <= H; ox++) {
         const int s = ox * ox + oy * oy + k * k;
         r->w[s] = cw.w[(ox + H) + W1 * ((oy + H) + W1 * (k + H))];
         if (r->w[s] != 0.f && s >= r->smax) r->smax = s + 1;
-        r->plane[k] += r->w[s];
       }
+}
+
+// Zero padding: the valid weight of a voxel is the sum of its in-bounds taps in the reference's order (x
+// fastest, z slowest), one after the other. A column's taps are in bounds for offsets xlo..xhi, ylo..yhi in
+// its planes; along z a voxel may be cut above (its sum is an intermediate value of the whole column's) or
+// below (its sum starts at a later plane). up[m]: planes -H..m; low[g]: planes -g..H, g < H, with kLow.
+// kS as in k_conv_stream; taps past the filter's reach add a weight of zero. (Summed plane by plane first,
+// the weights of boundary voxels differed in the last bits from those of the reference's order, and with them
+// every density of a zero-padded design run.)
+template <int H, int kS, bool kLow>
+__device__ __forceinline__ void valid_weights(const Radial<H>& rw, int xlo, int xhi, int ylo, int yhi,
+                                              float (&up)[H + 1], float (&low)[H + 1]) {
+  float a = 0.f;
+#pragma unroll
+  for (int g = 0; g <= H; g++) low[g] = 0.f;
+#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
+  for (int ez = -H; ez <= H; ez++) {
+#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
+    for (int ey = -H; ey <= H; ey++) {
+      if (ey < ylo || ey > yhi) continue;  // the same for all lanes of a warp
+#pragma unroll
+      for (int ex = -H; ex <= H; ex++) {
+        const int q = ex * ex + ey * ey + ez * ez;
+        if (q >= (kS > 0 ? kS : H * H + H + 1)) continue;  // radius < H + 0.5
+        const float w = ex >= xlo && ex <= xhi ? rw.w[q] : 0.f;
+        a += w;
+        if (kLow)
+#pragma unroll
+          for (int g = 0; g < H; g++)
+            if (ez >= -g) low[g] += w;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m <= H; m++)
+      if (ez == m) up[m] = a;
   }
 }
 
@@ -120,35 +152,41 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
   constexpr bool kFwd = MODE < 2 || MODE >= 4, kValid = kFwd && MODE != 5;
   constexpr int W1 = 2 * H + 1;
   __shared__ float buf[2][SN];
-  __shared__ float wplane[kValid ? H + 1 : 1][kTY][kTX];  // zero padding: valid weights of a column by |oz|
+  // zero padding: valid weights of a column's voxels m = 0..H - 1 planes from its upper end, of those farther
+  // from both ends (H) and of plane g (H + 1 + g); of plane g (g) where there are at most 2H planes
+  __shared__ float wcol[kValid ? 2 * H + 1 : 1][kTY][kTX];
   const int tid = threadIdx.x + kTX * threadIdx.y;
   const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * zchunk;
   const int z1 = min(z0 + zchunk, d.nz), planes = z1 - z0 + 2 * H;
   const int ox = x0 + int(threadIdx.x), oyr = int(threadIdx.y) * kNY, oy0 = y0 + oyr;  // own outputs
+  const int xlo = max(-H, -ox), xhi = min(H, d.nx - 1 - ox);  // own taps in bounds along x
   if (kValid && !periodic) {
-    // in x, this thread's taps are inside from ex = xlo to xhi
-    const int xlo = max(-H, -ox), xhi = min(H, d.nx - 1 - ox);
-#pragma unroll
+    const bool cut_z = z0 < H || z1 > d.nz - H;
+#pragma unroll 1
     for (int j = 0; j < kNY; j++) {
-      const int oy = oy0 + j;
-      float t[H + 1];
-#pragma unroll
-      for (int k = 0; k <= H; k++) t[k] = rw.plane[k];
-      if (xlo > -H || xhi < H || oy < H || oy >= d.ny - H) {
-#pragma unroll
-        for (int k = 0; k <= H; k++) t[k] = 0.f;
-#pragma unroll(H <= 3 ? 2 * H + 1 : 1)
-        for (int ey = -H; ey <= H; ey++)
-          if (oy + ey >= 0 && oy + ey < d.ny)
-#pragma unroll
-            for (int ex = -H; ex <= H; ex++) {
-              const bool in = ex >= xlo && ex <= xhi;
-#pragma unroll
-              for (int k = 0; k <= H; k++) t[k] += in ? rw.w[ex * ex + ey * ey + k * k] : 0.f;
-            }
+      const int ylo = max(-H, -(oy0 + j)), yhi = min(H, d.ny - 1 - (oy0 + j));
+      const bool cut = cut_z || ylo > -H || yhi < H || xlo > -H || xhi < H;
+      if (!__any_sync(0xffffffffu, cut)) continue;
+      if (d.nz <= 2 * H) {
+        for (int g = 0; g < d.nz; g++) {
+          float a = 0.f;
+          for (int ez = -min(g, H); ez <= min(H, d.nz - 1 - g); ez++)
+            for (int ey = ylo; ey <= yhi; ey++)
+              for (int ex = xlo; ex <= xhi; ex++) a += rw.w[ex * ex + ey * ey + ez * ez];
+          wcol[kValid ? g : 0][oyr + j][threadIdx.x] = a;
+        }
+        continue;
       }
+      float up[H + 1], low[H + 1];
+      if (z0 < H)
+        valid_weights<H, kS, true>(rw, xlo, xhi, ylo, yhi, up, low);
+      else
+        valid_weights<H, kS, false>(rw, xlo, xhi, ylo, yhi, up, low);
 #pragma unroll
-      for (int k = 0; k <= H; k++) wplane[k][oyr + j][threadIdx.x] = t[k];
+      for (int m = 0; m <= H; m++) wcol[m][oyr + j][threadIdx.x] = up[m];
+      if (z0 < H)
+#pragma unroll
+        for (int g = 0; g < H; g++) wcol[kValid ? H + 1 + g : 0][oyr + j][threadIdx.x] = low[g];
     }
   }
   // this thread's staged positions (the same in every plane): offsets in a plane of src and of the
@@ -270,9 +308,8 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
         } else {
           float ws = wsum_all;
           if (!periodic && (ox < H || ox >= d.nx - H || oy < H || oy >= d.ny - H || gz < H || gz >= d.nz - H)) {
-            ws = 0.f;
-            for (int k = -H; k <= H; k++)
-              if (gz + k >= 0 && gz + k < d.nz) ws += wplane[k < 0 ? -k : k][oyr + j][threadIdx.x];
+            const int m = d.nz <= 2 * H ? gz : (gz < H ? H + 1 + gz : min(d.nz - 1 - gz, H));
+            ws = wcol[kValid ? m : 0][oyr + j][threadIdx.x];
           }
           const float out = sumv / ws;
           if (dst) dst[row * dst_pitch + ox] = out;
