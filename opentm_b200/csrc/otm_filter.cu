@@ -6,6 +6,8 @@
 // warp), so no device allocation or global state is used.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <type_traits>
 
@@ -66,8 +68,11 @@ static otm_status make_weights(int type, float radius, ConvWeights* cw) {
 // is a tap of (rolling accumulators): 9 reads per output at radius 2 with one row, 17.5 at radius 3 with
 // four, where a read per tap takes 27 and 93. The weight depends on the squared distance only, and with the
 // loops unrolled its place in the parameter bank is a constant, so a tap is one FMA. The radii in common
-// use (1.5 to 2, 2.5, 3, 3.5, 4) have their set of taps compiled in; others skip the zero weights by
-// branches that all threads take alike. An output's taps are summed in the reference's order (x fastest, z
+// use (1.5 to 2, 2.5 to 3, 3.5 to 3.6, 3.75 to 4) have their set of taps compiled in; the other radii of a half
+// width H share the taps within H - 1/2, and those from there to H + 1/2 are predicated on the radius. (With a
+// branch per tap, and from half width 5 on with weights looked up by a run-time index and four rows a thread,
+// these radii took up to four times the time of a kernel that reads every tap's value for itself: 128^3,
+// radius 4.4, 5 and 6: 194, 333 and 845 us against 140, 189 and 297; now 92, 127 and 187.) An output's taps are summed in the reference's order (x fastest, z
 // slowest; the adjoint streams z downwards for that).
 //   MODE 0: forward            out = sum w src / sum_valid w
 //   MODE 1: forward + SIMP     also k = (k0 - kmin) out^p + kmin and dk = dk/dout
@@ -103,13 +108,15 @@ static void make_radial(const ConvWeights& cw, Radial<H>* r) {
 // Zero padding: the valid weight of a voxel is the sum of its in-bounds taps in the reference's order (x
 // fastest, z slowest), one after the other. A column's taps are in bounds for offsets xlo..xhi, ylo..yhi in
 // its planes; along z a voxel may be cut above (its sum is an intermediate value of the whole column's) or
-// below (its sum starts at a later plane). up[m]: planes -H..m; low[g]: planes -g..H, g < H, with kLow.
-// kS as in k_conv_stream; taps past the filter's reach add a weight of zero. (Summed plane by plane first,
+// below (its sum starts at a later plane). up[m]: planes -H..m; low[g]: planes -g..H, g < H, with kLow
+// (from half width 5 on only those the block needs, g0 <= g < g1, and up only where it reaches plane H).
+// Taps past the filter's reach add a weight of zero. (Summed plane by plane first,
 // the weights of boundary voxels differed in the last bits from those of the reference's order, and with them
 // every density of a zero-padded design run.)
 template <int H, int kS, bool kLow>
-__device__ __forceinline__ void valid_weights(const Radial<H>& rw, int xlo, int xhi, int ylo, int yhi,
+__device__ __forceinline__ void valid_weights(const Radial<H>& rw, int xlo, int xhi, int ylo, int yhi, int g0, int g1,
                                               float (&up)[H + 1], float (&low)[H + 1]) {
+  constexpr int kReach = kS > 0 ? kS : H * H + H + 1;
   float a = 0.f;
 #pragma unroll
   for (int g = 0; g <= H; g++) low[g] = 0.f;
@@ -117,18 +124,23 @@ __device__ __forceinline__ void valid_weights(const Radial<H>& rw, int xlo, int 
   for (int ez = -H; ez <= H; ez++) {
 #pragma unroll(H <= 4 ? 2 * H + 1 : 1)
     for (int ey = -H; ey <= H; ey++) {
-      if (ey < ylo || ey > yhi) continue;  // the same for all lanes of a warp
+      if (ey < ylo || ey > yhi || ey * ey + ez * ez >= rw.smax) continue;  // the same for all lanes of a warp
+      float w[2 * H + 1];
+      auto beyond = [&](int ex) { return H <= 4 && ex * ex + ey * ey + ez * ez >= kReach; };  // of every radius
 #pragma unroll
-      for (int ex = -H; ex <= H; ex++) {
-        const int q = ex * ex + ey * ey + ez * ez;
-        if (q >= (kS > 0 ? kS : H * H + H + 1)) continue;  // radius < H + 0.5
-        const float w = ex >= xlo && ex <= xhi ? rw.w[q] : 0.f;
-        a += w;
-        if (kLow)
+      for (int ex = -H; ex <= H; ex++)
+        if (!beyond(ex)) w[ex + H] = ex >= xlo && ex <= xhi ? rw.w[ex * ex + ey * ey + ez * ez] : 0.f;
+      if (H <= 4 || !kLow || g1 >= H)
 #pragma unroll
-          for (int g = 0; g < H; g++)
-            if (ez >= -g) low[g] += w;
-      }
+        for (int ex = -H; ex <= H; ex++)
+          if (!beyond(ex)) a += w[ex + H];
+      if (kLow)
+#pragma unroll
+        for (int g = 0; g < H; g++)
+          if (ez >= -g && (H <= 4 || (g >= g0 && g < g1)))
+#pragma unroll
+            for (int ex = -H; ex <= H; ex++)
+              if (!beyond(ex)) low[g] += w[ex + H];
     }
 #pragma unroll
     for (int m = 0; m <= H; m++)
@@ -151,6 +163,9 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
   constexpr int SX = kTX + 2 * H, SY = kTY + 2 * H, SN = SX * SY, NL = (SN + kConvThreads - 1) / kConvThreads;
   constexpr bool kFwd = MODE < 2 || MODE >= 4, kValid = kFwd && MODE != 5;
   constexpr int W1 = 2 * H + 1;
+  // squared distances below kSure are taps of every radius of this half width (at least H - 1/2), those from
+  // kReach on of none
+  constexpr int kSure = kS > 0 ? kS : (H == 0 ? 1 : H * H - H + 1), kReach = kS > 0 ? kS : H * H + H + 1;
   __shared__ float buf[2][SN];
   // zero padding: valid weights of a column's voxels m = 0..H - 1 planes from its upper end, of those farther
   // from both ends (H) and of plane g (H + 1 + g); of plane g (g) where there are at most 2H planes
@@ -179,9 +194,9 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
       }
       float up[H + 1], low[H + 1];
       if (z0 < H)
-        valid_weights<H, kS, true>(rw, xlo, xhi, ylo, yhi, up, low);
+        valid_weights<H, kS, true>(rw, xlo, xhi, ylo, yhi, z0, min(z1, H), up, low);
       else
-        valid_weights<H, kS, false>(rw, xlo, xhi, ylo, yhi, up, low);
+        valid_weights<H, kS, false>(rw, xlo, xhi, ylo, yhi, 0, 0, up, low);
 #pragma unroll
       for (int m = 0; m <= H; m++) wcol[m][oyr + j][threadIdx.x] = up[m];
       if (z0 < H)
@@ -245,51 +260,30 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
   for (int pl = 0; pl < planes; pl++) {
     if (pl + 1 < planes) fetch(pl + 1);
     const float* b = buf[pl & 1] + base;
-    if (kS > 0) {
-      // row by row of the window, every value read once; an output meets its taps (oy, ox) in the
-      // reference's order (the adjoint's offsets are negated, so it takes the rows downwards)
+    // row by row of the window, every value read once; an output meets its taps (oy, ox) in the
+    // reference's order (the adjoint's offsets are negated, so it takes the rows downwards)
 #pragma unroll
-      for (int i = 0; i < kNY + 2 * H; i++) {
-        const int r = kFwd ? i - H : kNY - 1 + H - i;
+    for (int i = 0; i < kNY + 2 * H; i++) {
+      const int r = kFwd ? i - H : kNY - 1 + H - i;
 #pragma unroll
-        for (int ex = -H; ex <= H; ex++) {
-          if (ex * ex >= kS) continue;
-          const float t = b[r * SX + (kFwd ? ex : -ex)];
+      for (int ex = -H; ex <= H; ex++) {
+        if (ex * ex >= kReach) continue;
+        const float t = b[r * SX + (kFwd ? ex : -ex)];
 #pragma unroll
-          for (int j = 0; j < kNY; j++) {
-            const int ey = kFwd ? r - j : j - r;
-            if (ey < -H || ey > H) continue;
+        for (int j = 0; j < kNY; j++) {
+          const int ey = kFwd ? r - j : j - r;
+          if (ey < -H || ey > H) continue;
 #pragma unroll
-            for (int k = 0; k <= H; k++) {
-              const int q = ex * ex + ey * ey + k * k;
-              if (q >= kS) continue;
+          for (int k = 0; k <= H; k++) {
+            const int q = ex * ex + ey * ey + k * k;
+            if (q >= kReach) continue;
+            if (q < kSure || q < rw.smax) {
               acc[H - k][j] += rw.w[q] * t;
               if (k > 0) acc[H + k][j] += rw.w[q] * t;
             }
           }
         }
       }
-    } else {
-#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
-      for (int ey = -H; ey <= H; ey++)
-#pragma unroll
-        for (int ex = -H; ex <= H; ex++) {
-          const int d2 = ex * ex + ey * ey, off = kFwd ? ey * SX + ex : -(ey * SX + ex);
-          if (d2 >= rw.smax) continue;
-          float t[kNY];
-#pragma unroll
-          for (int j = 0; j < kNY; j++) t[j] = b[off + j * SX];
-#pragma unroll
-          for (int k = 0; k <= H; k++) {
-            if (d2 + k * k >= rw.smax) break;
-            const float w = rw.w[d2 + k * k];
-#pragma unroll
-            for (int j = 0; j < kNY; j++) {
-              acc[H - k][j] += w * t[j];
-              if (k > 0) acc[H + k][j] += w * t[j];
-            }
-          }
-        }
     }
     if (pl >= 2 * H) {
       const int gz = kFwd ? z0 + pl - 2 * H : z1 - 1 - (pl - 2 * H);
@@ -339,17 +333,30 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
   }
 }
 
-// Blocks of a launch with ny rows per thread and z chunks of zc planes, and the chunk to use: the longest
-// (least work on the 2H planes around it) that still gives the GPU enough blocks, at least 4: eight of
-// 128 threads per SM, about what is resident at the kernel's registers.
-constexpr long long kConvFill = 8 * 148;
+// Blocks of a launch with ny rows per thread and z chunks of zc planes.
+constexpr long long kConvSms = 148;
 static long long conv_blocks(const Dims& d, int ny, int zc) {
   return (long long)((d.nx + kTX - 1) / kTX) * ((d.ny + kTYT * ny - 1) / (kTYT * ny)) * ((d.nz + zc - 1) / zc);
 }
+// The z chunk: a block works through its planes and 2 H more, and the blocks of an SM share it once there are
+// more than kShare, so the chunk with the least planes x max(kShare, blocks per SM). Within 3 % of the best
+// of 2 to 64 planes on average over 16^3 to 256^3 and radii 1.2 to 6. The longest chunk that leaves eight
+// blocks per SM, as it was, costs 25 % more at radius 6 (96^3: 249 against 140 us) and 2 to 4 % at radius 1.2
+// to 2.2.
+template <int H>
 static int conv_zchunk(const Dims& d, int ny) {
-  int zc = 32;
-  while (zc > 4 && conv_blocks(d, ny, zc) < kConvFill) zc /= 2;
-  return zc;
+  constexpr long long kShare = H <= 2 ? 4 : 3;
+  int best = 32;
+  long long least = LLONG_MAX;
+  for (int zc = 32; zc >= 4; zc /= 2) {
+    const long long per_sm = (conv_blocks(d, ny, zc) + kConvSms - 1) / kConvSms;
+    const long long cost = (std::min(zc, d.nz) + 2 * H) * std::max(kShare, per_sm);
+    if (cost < least) {
+      least = cost;
+      best = zc;
+    }
+  }
+  return best;
 }
 
 template <int H, int MODE>
@@ -361,7 +368,7 @@ static otm_status launch_stream(const Dims& d, const float* src, size_t src_pitc
   make_radial<H>(cw, &rw);
   auto run = [&](auto ny_tag) {
     constexpr int kNY = decltype(ny_tag)::value;
-    const int zchunk = conv_zchunk(d, kNY);
+    const int zchunk = conv_zchunk<H>(d, kNY);
     dim3 grid((d.nx + kTX - 1) / kTX, (d.ny + kTYT * kNY - 1) / (kTYT * kNY), (d.nz + zchunk - 1) / zchunk);
     auto launch = [&](auto kern) {
       kern<<<grid, dim3(kTX, kTYT), 0, s>>>(d, src, src_pitch, dk_in, ws_in, dst, dst_pitch, ws_out, periodic, zchunk,
@@ -382,10 +389,11 @@ static otm_status launch_stream(const Dims& d, const float* src, size_t src_pitc
     else
       launch(k_conv_stream<H, 0, kNY, MODE>);
   };
-  // rows per thread: 4 where the window's values are shared by enough taps and the cell fills the GPU
-  // with the fewer threads, else 1
-  constexpr int kFew = H >= 5 ? 4 : 1, kMany = H >= 3 ? 4 : 1;
-  if (kFew != kMany && conv_blocks(d, kMany, 16) < kConvFill)
+  // rows per thread: 4 where shared-memory reads bound a single row (half widths 3 and 4: about one read per
+  // three multiply-adds; five and more from half width 5 on) and the cell fills the GPU with the fewer
+  // threads, else 1
+  constexpr int kFew = 1, kMany = H == 3 || H == 4 ? 4 : 1;
+  if (kFew != kMany && conv_blocks(d, kMany, 16) < 8 * kConvSms)
     run(std::integral_constant<int, kFew>{});
   else
     run(std::integral_constant<int, kMany>{});
