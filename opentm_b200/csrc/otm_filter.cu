@@ -171,7 +171,9 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_stream(Dims d, const floa
   // from both ends (H) and of plane g (H + 1 + g); of plane g (g) where there are at most 2H planes
   __shared__ float wcol[kValid ? 2 * H + 1 : 1][kTY][kTX];
   const int tid = threadIdx.x + kTX * threadIdx.y;
-  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * zchunk;
+  // blocks in one dimension, x tiles fastest: a launch's y and z extents end at 65,535
+  const unsigned tx = unsigned(d.nx + kTX - 1) / kTX, ty = unsigned(d.ny + kTY - 1) / kTY, bq = blockIdx.x / tx;
+  const int x0 = int(blockIdx.x - bq * tx) * kTX, y0 = int(bq % ty) * kTY, z0 = int(bq / ty) * zchunk;
   const int z1 = min(z0 + zchunk, d.nz), planes = z1 - z0 + 2 * H;
   const int ox = x0 + int(threadIdx.x), oyr = int(threadIdx.y) * kNY, oy0 = y0 + oyr;  // own outputs
   const int xlo = max(-H, -ox), xhi = min(H, d.nx - 1 - ox);  // own taps in bounds along x
@@ -369,7 +371,7 @@ static otm_status launch_stream(const Dims& d, const float* src, size_t src_pitc
   auto run = [&](auto ny_tag) {
     constexpr int kNY = decltype(ny_tag)::value;
     const int zchunk = conv_zchunk<H>(d, kNY);
-    dim3 grid((d.nx + kTX - 1) / kTX, (d.ny + kTYT * kNY - 1) / (kTYT * kNY), (d.nz + zchunk - 1) / zchunk);
+    const unsigned grid = unsigned(conv_blocks(d, kNY, zchunk));
     auto launch = [&](auto kern) {
       kern<<<grid, dim3(kTX, kTYT), 0, s>>>(d, src, src_pitch, dk_in, ws_in, dst, dst_pitch, ws_out, periodic, zchunk,
                                             rw, wsum_all, p, k0, kmin, kout, dkout, ksout, pp, bad);

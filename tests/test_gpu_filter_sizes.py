@@ -54,3 +54,18 @@ def test_oc_filter_sizes(shape, radius):
     OCOptimizer(n).filterSens(st, rt, nx + 5, (nx, ny, nz), radius)
     assert rel_field(st.cpu().numpy()[:, :, :nx], ora.oc_filter_sens(s, rho, radius))[0] <= FILTER_TOL
     assert bool((st[:, :, nx:] == 0).all())
+
+
+@pytest.mark.parametrize("shape", [(2, 300000, 2), (300000, 1, 3), (2, 3, 300000)])
+def test_filter_long_axis(shape):
+    """An axis of more tiles than a launch has blocks along y or z."""
+    from opentm_b200 import OCOptimizer, filter_forward
+    n = int(np.prod(shape))
+    nz, ny, nx = shape
+    src = wl.uniform(n + 5, n).reshape(shape).astype(np.float32)
+    dst, _ = filter_forward(torch.from_numpy(src).cuda(), (nx, ny, nz), 1.5, 1, False)
+    assert rel_field(dst.cpu().numpy(), ora.conv_forward(src, 1, 1.5, False)[0])[0] <= FILTER_TOL
+    rho = (0.1 + 0.9 * wl.uniform(n + 6, n)).reshape(shape).astype(np.float32)
+    st = torch.from_numpy(-src).cuda()
+    OCOptimizer(n).filterSens(st, torch.from_numpy(rho).cuda(), nx, (nx, ny, nz), 2.0)
+    assert rel_field(st.cpu().numpy(), ora.oc_filter_sens(-src, rho, 2.0))[0] <= FILTER_TOL
