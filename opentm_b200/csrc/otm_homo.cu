@@ -92,9 +92,11 @@ static void launch_galerkin_coarse(Dims df, Dims dc, const float* stf, float* st
 static bool mixed_supported() { return true; }
 
 // Device memory of the handle. A handle of its own carves its buffers out of one allocation of the size
-// they are expected to take (build() reserves it; creating and destroying a handle was mostly some 45
-// allocations and as many frees: 4.4 + 1.6 ms at 32^3, 9 + 5.6 ms at 128^3), with single allocations for
-// what does not fit it. The server's handles take theirs from its stream-ordered pool.
+// that they take together (build() reserves it; creating and destroying a handle was mostly some 45
+// allocations and as many frees: 4.4 + 1.6 ms at 32^3, 9 + 5.6 ms at 128^3), or allocates them one by one
+// where a block of that size is not to be had. The server's handles take theirs from its stream-ordered pool.
+static size_t padded(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+
 otm_status Homo::reserve(size_t bytes) {
   if (pool) return OTM_OK;
   if (cudaMalloc((void**)&arena, bytes) != cudaSuccess) {
@@ -108,11 +110,10 @@ otm_status Homo::reserve(size_t bytes) {
 }
 
 otm_status Homo::alloc(void** p, size_t bytes) {
-  const size_t padded = (bytes + 255) & ~size_t(255);
-  if (padded <= arena_left) {
+  if (padded(bytes) <= arena_left) {
     *p = arena;
-    arena += padded;
-    arena_left -= padded;
+    arena += padded(bytes);
+    arena_left -= padded(bytes);
     bytes_allocated += bytes;
     return OTM_OK;
   }
@@ -148,42 +149,47 @@ Homo::~Homo() {
   if (sc_host) cudaFreeHost(sc_host);
 }
 
-otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool_t ext_pool, bool external_mode) {
+// What a handle of configuration c consists of: its levels, which kernels smooth them, and the sizes of its
+// plans. Without on_device no device is asked and no error returned (device_bytes): then the cluster cycle is
+// taken to be refused, and the inverse to run on the cluster size that needs more.
+otm_status Homo::plan(const otm_config& c, bool on_device) {
   cfg = c;
-  external = external_mode;
-  pool = ext_pool;
-  for (int i = 0; i < 3; i++) {
-    if (cfg.reso[i] < 2) return invalid("resolution must be >= 2 per axis");
-    if (cfg.reso[i] > 1024) {
-      set_error("axis resolution cannot exceed 1024");  // homogenization/grid.cpp:23-25
-      return OTM_ERR_UNSUPPORTED;
+  if (on_device) {
+    for (int i = 0; i < 3; i++) {
+      if (cfg.reso[i] < 2) return invalid("resolution must be >= 2 per axis");
+      if (cfg.reso[i] > 1024) {
+        set_error("axis resolution cannot exceed 1024");  // homogenization/grid.cpp:23-25
+        return OTM_ERR_UNSUPPORTED;
+      }
     }
+    if (cfg.pre_smooth < 0 || cfg.post_smooth < 0 || cfg.pre_smooth + cfg.post_smooth == 0)
+      return invalid("need at least one smoothing sweep");
+    if (cfg.max_iter < 1) return invalid("max_iter must be >= 1");
   }
-  if (cfg.pre_smooth < 0 || cfg.post_smooth < 0 || cfg.pre_smooth + cfg.post_smooth == 0)
-    return invalid("need at least one smoothing sweep");
-  if (cfg.max_iter < 1) return invalid("max_iter must be >= 1");
   if (cfg.check_every < 1) cfg.check_every = 1;
   if (cfg.check_every > kMaxChunk) cfg.check_every = kMaxChunk;
   if (cfg.coarsest_max_dof < 8) cfg.coarsest_max_dof = 8;
-  if (cfg.solver != OTM_SOLVER_PCG && cfg.solver != OTM_SOLVER_VCYCLE) return invalid("unknown solver");
-  if (cfg.smoother != OTM_SMOOTHER_COLOR && cfg.smoother != OTM_SMOOTHER_TILED) return invalid("unknown smoother");
-  if (cfg.precision < OTM_PRECISION_FP32 || cfg.precision > OTM_PRECISION_MIXED_FP16)
-    return invalid("unknown precision");
-  if (cfg.precision != OTM_PRECISION_FP32 && !mixed_supported()) {
-    set_error("mixed-precision storage is not available in this build");
-    return OTM_ERR_UNSUPPORTED;
+  if (on_device) {
+    if (cfg.solver != OTM_SOLVER_PCG && cfg.solver != OTM_SOLVER_VCYCLE) return invalid("unknown solver");
+    if (cfg.smoother != OTM_SMOOTHER_COLOR && cfg.smoother != OTM_SMOOTHER_TILED) return invalid("unknown smoother");
+    if (cfg.precision < OTM_PRECISION_FP32 || cfg.precision > OTM_PRECISION_MIXED_FP16)
+      return invalid("unknown precision");
+    if (cfg.precision != OTM_PRECISION_FP32 && !mixed_supported()) {
+      set_error("mixed-precision storage is not available in this build");
+      return OTM_ERR_UNSUPPORTED;
+    }
+    if (cfg.solver == OTM_SOLVER_PCG && cfg.pre_smooth != cfg.post_smooth)
+      return invalid("PCG needs a symmetric V-cycle (pre_smooth == post_smooth)");
   }
-  if (cfg.solver == OTM_SOLVER_PCG && cfg.pre_smooth != cfg.post_smooth)
-    return invalid("PCG needs a symmetric V-cycle (pre_smooth == post_smooth)");
 
-  std::vector<Dims> dims = level_dims(cfg.reso, cfg.coarsest_max_dof);
-  if (dims.back().nv() > size_t(kMaxCoarsest)) {
+  const std::vector<Dims> dims = level_dims(cfg.reso, cfg.coarsest_max_dof);
+  if (on_device && dims.back().nv() > size_t(kMaxCoarsest)) {
     set_error("coarsest level too large for the dense direct solve (aspect ratio too extreme)");
     return OTM_ERR_UNSUPPORTED;
   }
   // template matrices, element size 1/reso_x (homogenization/homogenization.cpp:211)
   template_matrices(1.0 / cfg.reso[0] / 2.0, &tm);
-  if (tm.structure_error > 1e-9) {
+  if (on_device && tm.structure_error > 1e-9) {
     set_error("element matrix does not have the cube-Laplacian structure");
     return OTM_ERR_UNSUPPORTED;
   }
@@ -196,6 +202,154 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
       ef.disp[j][cc] = float(tm.disp[j][cc]);
       ef.feMu[j][cc] = float(tm.feMu[j][cc]);
     }
+  const int L = int(dims.size());
+  if (on_device && mixed && L == 1) {
+    set_error("mixed precision needs at least two multigrid levels");
+    return OTM_ERR_UNSUPPORTED;
+  }
+  lv.resize(dims.size());
+  for (int l = 0; l < L; l++) lv[l].d = dims[l];
+  nc = int(dims.back().nv());
+  // small levels (<= 16^3 unknowns) and the coarsest solve run in one single-CTA kernel
+  {
+    int t = -1;
+    for (int l = 1; l < L; l++)
+      if (dims[l].nv() <= size_t(kTailMaxNv)) {
+        t = l;
+        break;
+      }
+    if (t > 0 && t < L - 1 && L - t <= kTailMaxLevels) {
+      size_t floats = 0;
+      for (int l = t; l < L; l++) floats += 9 * dims[l].nv();
+      if (floats * sizeof(float) <= size_t(kMaxDynSmem)) {
+        tail_l = t;
+        tail_smem = floats * sizeof(float);
+        if (on_device)
+          OTM_CUDA(cudaFuncSetAttribute(k_vcycle_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+      }
+    }
+  }
+  // the levels from the first with <= 32^3 unknowns (cluster_cycle 3) or <= 16^3 (cluster_cycle 2)
+  // and the coarsest solve in one thread-block-cluster launch; cluster_cycle 1 takes <= 16^3 when
+  // the level above that is smoothed by the coarse tile kernels (a sweep there is one launch, and
+  // the cluster's passes cost a cluster barrier per half sweep), else <= 32^3
+  const bool tiles = cfg.smoother == OTM_SMOOTHER_TILED && cfg.solver == OTM_SOLVER_PCG && cfg.pre_smooth > 1 &&
+                     cfg.post_smooth > 1;
+  if (cfg.cluster_cycle) {
+    size_t cl_max = cfg.cluster_cycle == 2 ? size_t(kClMaxNv / 8) : size_t(kClMaxNv);
+    if (cfg.cluster_cycle == 1)
+      for (int l = 2; l < L - 1; l++)
+        if (dims[l].nv() <= size_t(kClMaxNv / 8)) {
+          if (tiles && dims[l - 1].nv() <= size_t(kClMaxNv) && ctile_fits(dims[l - 1])) cl_max = kClMaxNv / 8;
+          break;
+        }
+    int t = -1;
+    for (int l = 1; l < L - 1; l++)
+      if (dims[l].nv() <= cl_max) {
+        t = l;
+        break;
+      }
+    if (t > 0 && !on_device) {
+      for (int l = t; l < L; l++) cl_entries += 3 * size_t(dims[l].nz);
+    } else if (t > 0) {
+      ClDesc cd{};
+      const size_t bytes = cl_plan(dims.data() + t, L - t, &cd);
+      if (bytes > 0 &&
+          cudaFuncSetAttribute(k_vcycle_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem) ==
+              cudaSuccess &&
+          cudaFuncSetAttribute(k_vcycle_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3(kCl);
+        lc.blockDim = dim3(kClThreads);
+        lc.dynamicSmemBytes = bytes;
+        int ncl = 0;
+        if (cudaOccupancyMaxActiveClusters(&ncl, (void*)k_vcycle_cluster, &lc) == cudaSuccess && ncl >= 1) {
+          cd.pre = cfg.pre_smooth;
+          cd.post = cfg.post_smooth;
+          cl_tables(&cd, cl_tab_host);
+          cl_entries = cl_tab_host.size();
+          cl_desc = cd;
+          cluster_l = t;
+          cluster_smem = bytes;
+        }
+      }
+      cudaGetLastError();  // a refused attribute or occupancy query leaves no error behind
+    }
+  }
+  // the tile-staged fine smoother: cube elements (no face couplings), every axis a multiple of the
+  // tile, a coarser level to correct from, at least two sweeps in each leg (consecutive sweeps move
+  // the tile faces by half a tile; with one sweep per leg both legs would keep the faces of one
+  // tiling, and the 128^3 design loop at V(1,1) ran 354 against 389 iterations/s with the colour
+  // passes), and the PCG solver. Block
+  // Jacobi across the tile faces leaves the mode that is constant inside each tile and alternates in
+  // sign from tile to tile almost undamped (a smoother factor near -1): preconditioned CG is not
+  // affected by that (the preconditioner stays symmetric positive definite), but stationary V-cycles
+  // would stall on it, so they keep the global colour passes.
+  tiled = tiles && !face && L > 1 && tile_fits(dims[0]);
+  // coarse levels smoothed by the tile kernels: the levels between the fine level and the cluster
+  // or single-CTA cycle (or the coarsest level) whose axes are multiples of the coarse tile, under
+  // the same conditions as the fine level's tiles
+  if (tiles) {
+    int last = L - 1;  // first level not smoothed by regular passes
+    if (cluster_l > 0) last = std::min(last, cluster_l);
+    if (tail_l > 0) last = std::min(last, tail_l);
+    for (int l = 1; l < last; l++) lv[l].ctiled = ctile_fits(dims[l]);
+  }
+  if (on_device) return plan_direct_inverse();
+  if (dims.back().nv() <= size_t(kMaxCoarsest)) {
+    const DirPlan wide = dir_plan(nc, kDirCl), narrow = dir_plan(nc, 8);
+    dir = wide.work > narrow.work ? wide : narrow;
+  }
+  return OTM_OK;
+}
+
+// Every device buffer of the planned handle: take(pointer, bytes) for each, in the order in which they lie.
+template <typename F>
+otm_status Homo::buffers(F&& take) {
+  auto floats = [&](float** p, size_t n) { return take((void**)p, n * sizeof(float)); };
+  for (size_t l = 0; l < lv.size(); l++) {
+    Level& V = lv[l];
+    const size_t n = V.d.nv();
+    // the mixed form keeps the fine-level correction and residual in 16-bit buffers instead
+    if (!(mixed && l == 0 && lv.size() > 1)) {
+      OTM_TRY(floats(&V.u, 3 * n));
+      OTM_TRY(floats(&V.r, 3 * n));
+    }
+    OTM_TRY(floats(&V.f, 3 * n));
+    if (l > 0 || lv.size() == 1) OTM_TRY(floats(&V.st, 27 * n));
+  }
+  const size_t nv = lv[0].d.nv();
+  for (float** p : {&ks, &kraw}) OTM_TRY(floats(p, nv));
+  for (float** p : {&b, &x}) OTM_TRY(floats(p, 3 * nv));
+  if (mixed) {
+    OTM_TRY(take((void**)&x64, 3 * nv * sizeof(double)));
+    OTM_TRY(take(&k16, nv * 2));
+    for (void** p : {&u16, &r16}) OTM_TRY(take(p, 3 * nv * 2));
+  }
+  for (float** pp : {&p, &q}) OTM_TRY(floats(pp, 3 * nv));
+  OTM_TRY(take((void**)&Ainv, size_t(nc) * nc * sizeof(double)));
+  if (dir.work) OTM_TRY(take((void**)&dir_work, dir.work * sizeof(double)));
+  OTM_TRY(floats(&table, 64 * 27));
+  OTM_TRY(take((void**)&sc, sizeof(SolveScalars)));
+  OTM_TRY(take((void**)&partials, size_t(kMaxPartials) * 16 * sizeof(double)));
+  OTM_TRY(take((void**)&means, 8 * sizeof(double)));
+  OTM_TRY(take((void**)&flags, 4 * sizeof(int)));
+  if (cl_entries) OTM_TRY(take((void**)&cl_tab, cl_entries * sizeof(int)));
+  if (tiled) {
+    // the second buffer of the sweep ping-pong (the fine correction's storage type)
+    OTM_TRY(take(&u2, 3 * nv * (mixed ? 2 : sizeof(float))));
+    // per-tile partial sums of the tiled direction update (p . q)
+    OTM_TRY(take((void**)&tile_partials, size_t(tile_count(lv[0].d)) * 3 * sizeof(double)));
+  }
+  for (Level& V : lv)
+    if (V.ctiled) OTM_TRY(floats(&V.u2, 3 * V.d.nv()));
+  return OTM_OK;
+}
+
+otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool_t ext_pool, bool external_mode) {
+  external = external_mode;
+  pool = ext_pool;
+  OTM_TRY(plan(c, true));
 
   if (external) {
     stream = ext_stream;
@@ -216,61 +370,26 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
     for (int a = 0; a < 2; a++)
       for (int j = 0; j < kMaxChunk; j++) OTM_CUDA(cudaEventCreate(&prof_ev[a][j]));
 
-  // what the buffers below take (with some room for the small ones)
-  const bool tiles = cfg.smoother == OTM_SMOOTHER_TILED && cfg.solver == OTM_SOLVER_PCG && cfg.pre_smooth > 1 &&
-                     cfg.post_smooth > 1;
-  const size_t nc0 = dims.back().nv();
-  size_t expected = (size_t(4) << 20) + 2 * nc0 * nc0 * sizeof(double) + dims[0].nv() * (mixed ? 100 : 80);
-  if (tiles && !face && tile_fits(dims[0])) expected += dims[0].nv() * 12;
-  for (size_t l = 1; l < dims.size(); l++)
-    expected += dims[l].nv() * sizeof(float) * (9 + 27 + (tiles && ctile_fits(dims[l]) ? 3 : 0));
-  OTM_TRY(reserve(expected));
-  lv.resize(dims.size());
-  for (size_t l = 0; l < dims.size(); l++) {
-    Level& L = lv[l];
-    L.d = dims[l];
-    const size_t nv = L.d.nv();
-    // the mixed form keeps the fine-level correction and residual in 16-bit buffers instead
-    const bool fp32_fine = !(mixed && l == 0 && dims.size() > 1);
-    if (fp32_fine) {
-      OTM_TRY(alloc((void**)&L.u, 3 * nv * sizeof(float)));
-      OTM_TRY(alloc((void**)&L.r, 3 * nv * sizeof(float)));
-      OTM_CUDA(cudaMemsetAsync(L.u, 0, 3 * nv * sizeof(float), stream));
-      OTM_CUDA(cudaMemsetAsync(L.r, 0, 3 * nv * sizeof(float), stream));
-    }
-    OTM_TRY(alloc((void**)&L.f, 3 * nv * sizeof(float)));
-    OTM_CUDA(cudaMemsetAsync(L.f, 0, 3 * nv * sizeof(float), stream));
-    if (l > 0 || dims.size() == 1) OTM_TRY(alloc((void**)&L.st, 27 * nv * sizeof(float)));
-  }
+  size_t need = 0;
+  buffers([&](void**, size_t bytes) {
+    need += padded(bytes);
+    return OTM_OK;
+  });
+  OTM_TRY(reserve(need));
+  OTM_TRY(buffers([&](void** p, size_t bytes) { return alloc(p, bytes); }));
   const size_t nv = lv[0].d.nv();
-  OTM_TRY(alloc((void**)&ks, nv * sizeof(float)));
-  OTM_TRY(alloc((void**)&kraw, nv * sizeof(float)));
-  OTM_TRY(alloc((void**)&b, 3 * nv * sizeof(float)));
-  OTM_TRY(alloc((void**)&x, 3 * nv * sizeof(float)));
+  for (Level& V : lv) {
+    const size_t bytes = 3 * V.d.nv() * sizeof(float);
+    if (V.u) OTM_CUDA(cudaMemsetAsync(V.u, 0, bytes, stream));
+    if (V.r) OTM_CUDA(cudaMemsetAsync(V.r, 0, bytes, stream));
+    OTM_CUDA(cudaMemsetAsync(V.f, 0, bytes, stream));
+  }
   OTM_CUDA(cudaMemsetAsync(x, 0, 3 * nv * sizeof(float), stream));
   if (mixed) {
-    if (lv.size() == 1) {
-      set_error("mixed precision needs at least two multigrid levels");
-      return OTM_ERR_UNSUPPORTED;
-    }
-    OTM_TRY(alloc((void**)&x64, 3 * nv * sizeof(double)));
-    OTM_TRY(alloc(&k16, nv * 2));
-    OTM_TRY(alloc(&u16, 3 * nv * 2));
-    OTM_TRY(alloc(&r16, 3 * nv * 2));
     OTM_CUDA(cudaMemsetAsync(x64, 0, 3 * nv * sizeof(double), stream));
     OTM_CUDA(cudaMemsetAsync(u16, 0, 3 * nv * 2, stream));
   }
-  OTM_TRY(alloc((void**)&p, 3 * nv * sizeof(float)));
-  OTM_TRY(alloc((void**)&q, 3 * nv * sizeof(float)));
   OTM_CUDA(cudaMemsetAsync(p, 0, 3 * nv * sizeof(float), stream));
-  nc = int(lv.back().d.nv());
-  OTM_TRY(alloc((void**)&Ainv, size_t(nc) * nc * sizeof(double)));
-  OTM_TRY(plan_direct_inverse());
-  OTM_TRY(alloc((void**)&table, 64 * 27 * sizeof(float)));
-  OTM_TRY(alloc((void**)&sc, sizeof(SolveScalars)));
-  OTM_TRY(alloc((void**)&partials, size_t(kMaxPartials) * 16 * sizeof(double)));
-  OTM_TRY(alloc((void**)&means, 8 * sizeof(double)));
-  OTM_TRY(alloc((void**)&flags, 4 * sizeof(int)));
   OTM_CUDA(cudaMemsetAsync(sc, 0, sizeof(SolveScalars), stream));
   OTM_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(int), stream));
   // pinned block: solve scalars, then the level-1 Galerkin table (uploaded from pinned memory
@@ -282,121 +401,24 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
   galerkin_level1_table(tm, tab);
   OTM_CUDA(cudaMemcpyAsync(table, tab, 64 * 27 * sizeof(float), cudaMemcpyHostToDevice, stream));
   if (!external) OTM_CUDA(cudaStreamSynchronize(stream));
-  // small levels (<= 16^3 unknowns) and the coarsest solve run in one single-CTA kernel
-  {
-    const int L = int(lv.size());
-    int t = -1;
-    for (int l = 1; l < L; l++)
-      if (lv[l].d.nv() <= size_t(kTailMaxNv)) {
-        t = l;
-        break;
-      }
-    if (t > 0 && t < L - 1 && L - t <= kTailMaxLevels) {
-      size_t floats = 0;
-      for (int l = t; l < L; l++) floats += 9 * lv[l].d.nv();
-      if (floats * sizeof(float) <= size_t(kMaxDynSmem)) {
-        tail_l = t;
-        tail_smem = floats * sizeof(float);
-        OTM_CUDA(cudaFuncSetAttribute(k_vcycle_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
-      }
+  if (cluster_l > 0) {
+    for (int i = 0; i < cl_desc.nlev; i++) {
+      cl_desc.lv[i].st = lv[cluster_l + i].st;
+      cl_desc.lv[i].rg = lv[cluster_l + i].r;
     }
+    cl_desc.Ainv = Ainv;
+    cl_desc.tab_g = cl_tab;
+    OTM_CUDA(cudaMemcpyAsync(cl_tab, cl_tab_host.data(), cl_entries * sizeof(int), cudaMemcpyHostToDevice, stream));
   }
-  // the levels from the first with <= 32^3 unknowns (cluster_cycle 3) or <= 16^3 (cluster_cycle 2)
-  // and the coarsest solve in one thread-block-cluster launch; cluster_cycle 1 takes <= 16^3 when
-  // the level above that is smoothed by the coarse tile kernels (a sweep there is one launch, and
-  // the cluster's passes cost a cluster barrier per half sweep), else <= 32^3
-  if (cfg.cluster_cycle) {
-    const int L = int(lv.size());
-    size_t cl_max = cfg.cluster_cycle == 2 ? size_t(kClMaxNv / 8) : size_t(kClMaxNv);
-    if (cfg.cluster_cycle == 1) {
-      const bool ctiles = cfg.smoother == OTM_SMOOTHER_TILED && cfg.solver == OTM_SOLVER_PCG && cfg.pre_smooth > 1 &&
-                          cfg.post_smooth > 1;
-      for (int l = 2; l < L - 1; l++)
-        if (lv[l].d.nv() <= size_t(kClMaxNv / 8)) {
-          if (ctiles && lv[l - 1].d.nv() <= size_t(kClMaxNv) && ctile_fits(lv[l - 1].d)) cl_max = kClMaxNv / 8;
-          break;
-        }
-    }
-    int t = -1;
-    for (int l = 1; l < L - 1; l++)
-      if (lv[l].d.nv() <= cl_max) {
-        t = l;
-        break;
-      }
-    if (t > 0) {
-      std::vector<Dims> dims;
-      for (int l = t; l < L; l++) dims.push_back(lv[l].d);
-      ClDesc cd{};
-      const size_t bytes = cl_plan(dims.data(), int(dims.size()), &cd);
-      if (bytes > 0 &&
-          cudaFuncSetAttribute(k_vcycle_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem) ==
-              cudaSuccess &&
-          cudaFuncSetAttribute(k_vcycle_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-        cudaLaunchConfig_t lc{};
-        lc.gridDim = dim3(kCl);
-        lc.blockDim = dim3(kClThreads);
-        lc.dynamicSmemBytes = bytes;
-        int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, (void*)k_vcycle_cluster, &lc) == cudaSuccess && ncl >= 1) {
-          cd.pre = cfg.pre_smooth;
-          cd.post = cfg.post_smooth;
-          for (int i = 0; i < cd.nlev; i++) {
-            cd.lv[i].st = lv[t + i].st;
-            cd.lv[i].rg = lv[t + i].r;
-          }
-          cd.Ainv = Ainv;
-          cl_tables(&cd, cl_tab_host);
-          OTM_TRY(alloc((void**)&cl_tab, cl_tab_host.size() * sizeof(int)));
-          OTM_CUDA(cudaMemcpyAsync(cl_tab, cl_tab_host.data(), cl_tab_host.size() * sizeof(int),
-                                   cudaMemcpyHostToDevice, stream));
-          cd.tab_g = cl_tab;
-          cl_desc = cd;
-          cluster_l = t;
-          cluster_smem = bytes;
-        }
-      }
-      cudaGetLastError();  // a refused attribute or occupancy query leaves no error behind
-    }
-  }
-  // the tile-staged fine smoother: cube elements (no face couplings), every axis a multiple of the
-  // tile, a coarser level to correct from, at least two sweeps in each leg (consecutive sweeps move
-  // the tile faces by half a tile; with one sweep per leg both legs would keep the faces of one
-  // tiling, and the 128^3 design loop at V(1,1) ran 354 against 389 iterations/s with the colour
-  // passes), and the PCG solver. Block
-  // Jacobi across the tile faces leaves the mode that is constant inside each tile and alternates in
-  // sign from tile to tile almost undamped (a smoother factor near -1): preconditioned CG is not
-  // affected by that (the preconditioner stays symmetric positive definite), but stationary V-cycles
-  // would stall on it, so they keep the global colour passes.
-  if (cfg.smoother == OTM_SMOOTHER_TILED && cfg.solver == OTM_SOLVER_PCG && !face && lv.size() > 1 &&
-      tile_fits(lv[0].d) && cfg.pre_smooth > 1 && cfg.post_smooth > 1) {
-    OTM_TRY(tile_attributes());
-    // the second buffer of the sweep ping-pong (the fine correction's storage type)
-    OTM_TRY(alloc(&u2, 3 * lv[0].d.nv() * (mixed ? 2 : sizeof(float))));
-    // per-tile partial sums of the tiled direction update (p . q)
-    OTM_TRY(alloc((void**)&tile_partials, size_t(tile_count(lv[0].d)) * 3 * sizeof(double)));
-    tiled = true;
-  }
-  // coarse levels smoothed by the tile kernels: the levels between the fine level and the cluster
-  // or single-CTA cycle (or the coarsest level) whose axes are multiples of the coarse tile, under
-  // the same conditions as the fine level's tiles
-  if (cfg.smoother == OTM_SMOOTHER_TILED && cfg.solver == OTM_SOLVER_PCG && cfg.pre_smooth > 1 && cfg.post_smooth > 1) {
-    const int L = int(lv.size());
-    int last = L - 1;  // first level not smoothed by regular passes
-    if (cluster_l > 0) last = std::min(last, cluster_l);
-    if (tail_l > 0) last = std::min(last, tail_l);
-    for (int l = 1; l < last; l++) {
-      if (!ctile_fits(lv[l].d)) continue;
-      OTM_TRY(alloc((void**)&lv[l].u2, 3 * lv[l].d.nv() * sizeof(float)));
-      lv[l].ctiled = true;
-      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromZero, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(kCSmallSmem)));
-      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromU, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(kCSmallSmem)));
-      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromU, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(kCSmallSmem)));
-      OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromUProlong, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCSmallSmemProlong)));
-    }
+  if (tiled) OTM_TRY(tile_attributes());
+  bool ctiled = false;
+  for (const Level& V : lv) ctiled |= V.ctiled;
+  if (ctiled) {
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromZero, false>, a, int(kCSmallSmem)));
+    OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromU, false>, a, int(kCSmallSmem)));
+    OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromU, true>, a, int(kCSmallSmem)));
+    OTM_CUDA(cudaFuncSetAttribute(k_ctile_sweep_small<kFromUProlong, true>, a, int(kCSmallSmemProlong)));
   }
   stats.levels = int(lv.size());
   stats.cluster_level = cluster_l;
@@ -488,7 +510,7 @@ otm_status Homo::plan_direct_inverse() {
     return OTM_ERR_UNSUPPORTED;
   }
   dir = dir_plan(nc, ncl);
-  return alloc((void**)&dir_work, dir.work * sizeof(double));
+  return OTM_OK;
 }
 
 otm_status Homo::launch_direct_inverse(cudaStream_t cs) {

@@ -83,7 +83,8 @@ struct Homo {
   bool tiled = false;
   double* tile_partials = nullptr;  // 3 partial sums per fine tile (k_tile_apply_dot)
   std::vector<int> cl_tab_host;  // plane tables of the cluster plan (kept: the copy is asynchronous)
-  int* cl_tab = nullptr;          // their device copy
+  size_t cl_entries = 0;         // their count
+  int* cl_tab = nullptr;         // their device copy
   int tail_l = -1;          // first level handled by the single-CTA tail kernel (-1: none)
   size_t tail_smem = 0;     // its dynamic shared memory
   int nc = 0;
@@ -123,6 +124,9 @@ struct Homo {
   otm_solve_stats stats{};
 
   ~Homo();
+  otm_status plan(const otm_config& c, bool on_device);
+  template <typename F>
+  otm_status buffers(F&& take);
   otm_status reserve(size_t bytes);
   otm_status alloc(void** p, size_t bytes);
   otm_status build(const otm_config& c, cudaStream_t ext_stream = nullptr, cudaMemPool_t ext_pool = nullptr,
