@@ -77,7 +77,8 @@ OTM_API otm_status otm_server_poll(otm_server* s, int64_t request_id, double C[9
 /* Cancel a queued request, or a running one: the batched form drops it at the next step and
  * releases its memory; the handle form lets its solve finish, then reports it cancelled. */
 OTM_API otm_status otm_server_cancel(otm_server* s, int64_t request_id);
-/* Bytes of device memory a request of this size keeps resident while it runs. */
+/* Bytes of device memory a request of this size keeps resident while it runs, on a server with the
+ * default smoothing (one with pre_smooth = 1 keeps the same or less). */
 OTM_API size_t otm_server_request_bytes(const int reso[3]);
 /* Device bytes currently held by running requests. */
 OTM_API size_t otm_server_bytes_in_use(const otm_server* s);

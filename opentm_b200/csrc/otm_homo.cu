@@ -346,6 +346,17 @@ otm_status Homo::buffers(F&& take) {
   return OTM_OK;
 }
 
+size_t Homo::device_bytes(const otm_config& c) {
+  Homo h;
+  h.plan(c, false);
+  size_t total = 0;
+  h.buffers([&](void**, size_t bytes) {
+    total += padded(bytes);
+    return OTM_OK;
+  });
+  return total;
+}
+
 otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool_t ext_pool, bool external_mode) {
   external = external_mode;
   pool = ext_pool;

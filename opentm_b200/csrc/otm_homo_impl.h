@@ -127,6 +127,9 @@ struct Homo {
   otm_status plan(const otm_config& c, bool on_device);
   template <typename F>
   otm_status buffers(F&& take);
+  // Device bytes of a handle of configuration c, padded as in its block (an upper bound where that hangs on
+  // the device: see plan()). No device needed.
+  static size_t device_bytes(const otm_config& c);
   otm_status reserve(size_t bytes);
   otm_status alloc(void** p, size_t bytes);
   otm_status build(const otm_config& c, cudaStream_t ext_stream = nullptr, cudaMemPool_t ext_pool = nullptr,

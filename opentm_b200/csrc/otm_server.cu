@@ -254,29 +254,12 @@ static void homo_config(const otm_server_config& sc, const int reso[3], otm_conf
   c->use_graphs = 0;
 }
 
-// Device bytes of one request's resident state (the allocations of Homo::build for an FP32
-// PCG solve).
-static size_t request_bytes(const int reso[3]) {
-  size_t total = 0;
-  Dims d{reso[0], reso[1], reso[2]};
-  int L = 0;
-  while (true) {
-    const size_t nv = d.nv();
-    total += 9 * nv * sizeof(float);  // u, f, r
-    if (L > 0) total += 27 * nv * sizeof(float);
-    L++;
-    const bool can = d.nx % 2 == 0 && d.ny % 2 == 0 && d.nz % 2 == 0 && d.nx >= 8 && d.ny >= 8 && d.nz >= 8 &&
-                     nv > 64;
-    if (!can) break;
-    d = Dims{d.nx / 2, d.ny / 2, d.nz / 2};
-  }
-  const size_t nv0 = size_t(reso[0]) * reso[1] * reso[2];
-  const size_t nc = d.nv();
-  total += nv0 * sizeof(float) * (2 + 4 * 3);  // ks, kraw, b, x, p, q
-  total += nc * nc * sizeof(double) + 64 * 27 * sizeof(float);
-  total += sizeof(SolveScalars) + size_t(kMaxPartials) * 16 * sizeof(double) + 8 * sizeof(double) + 16;
-  total += nv0 * sizeof(float);  // the imported field while it is being set up
-  return total;
+// Device bytes of one request's resident state: its handle's buffers, and the imported field while it is
+// being set up.
+static size_t request_bytes(const otm_server_config& sc, const int reso[3]) {
+  otm_config c;
+  homo_config(sc, reso, &c);
+  return Homo::device_bytes(c) + size_t(reso[0]) * reso[1] * reso[2] * sizeof(float);
 }
 
 }  // namespace otm
@@ -804,7 +787,9 @@ otm_status otm_server_config_init(otm_server_config* cfg) {
 
 size_t otm_server_request_bytes(const int reso[3]) {
   if (!reso) return 0;
-  return otm::request_bytes(reso);
+  otm_server_config c;
+  otm_server_config_init(&c);
+  return otm::request_bytes(c, reso);
 }
 
 otm_status otm_server_create(const otm_server_config* cfg, void* stream, otm_server** out) {
@@ -858,7 +843,7 @@ otm_status otm_server_submit(otm_server* s, const int reso[3], const float* k_ho
       set_error("serving supports 8 to 1024 cells per axis");
       return OTM_ERR_UNSUPPORTED;
     }
-  const size_t bytes = request_bytes(reso);
+  const size_t bytes = request_bytes(s->cfg, reso);
   if (bytes > s->cfg.hbm_budget_bytes) {
     set_error("request larger than the serving memory budget");
     return OTM_ERR_BUDGET;

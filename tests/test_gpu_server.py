@@ -146,3 +146,23 @@ def test_requests_arriving_while_others_run(batched):
         C, info = s.poll(rid)
         assert np.array_equal(C, _solve_alone(k, batched)[0])
     assert all(s.poll(r) is not None for r in first)
+
+
+def test_resident_memory_within_budget():
+    """Cells whose coarsest level is large (990 unknowns: the inverse's scratch is half of the handle) on many
+    lanes: what the device gives up stays within the budget that admitted them."""
+    from opentm_b200 import Server
+    shape = (20, 22, 18)
+    budget = 16 * Server.request_bytes((18, 22, 20))
+    ks = [random_k(shape, seed=140 + i)[0] for i in range(32)]
+    # the library's kernels are loaded first: their memory is not the requests'
+    _solve_alone(ks[0], False)
+    torch.cuda.synchronize()
+    s = Server(hbm_budget_bytes=budget, max_active=32, streams=32, host_stage_bytes=RING)
+    free0 = torch.cuda.mem_get_info()[0]
+    ids = [s.submit(k) for k in ks]
+    s.run_until_idle()
+    used = free0 - torch.cuda.mem_get_info()[0]
+    assert s.bytes_resident() <= budget
+    assert used <= budget + (64 << 20), (used, budget)  # the pool grows in steps of 32 MB
+    assert all(max(s.poll(i)[1].stats.rel_res) <= 1e-6 for i in ids)

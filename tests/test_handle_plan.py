@@ -1,5 +1,5 @@
 """CPU check of a handle's device memory (tests/cpp/handle_plan_check.cu): one allocation per handle, sized
-by the buffers that the handle then takes from it. Host code linked with the library's objects and a CUDA
+by the buffers that the handle then takes from it, and a serving request counted with all of them. Host code linked with the library's objects and a CUDA
 runtime that only counts; no GPU needed."""
 import glob
 import os
@@ -15,7 +15,7 @@ NVCC = shutil.which("nvcc") or ("/usr/local/cuda/bin/nvcc" if os.path.exists("/u
 
 
 @pytest.mark.skipif(NVCC is None, reason="needs nvcc")
-def test_handle_takes_one_allocation(tmp_path):
+def test_handle_memory(tmp_path):
     build.build()  # the library's objects, where they are not there yet
     exe = tmp_path / "handle_plan_check"
     subprocess.run([NVCC, *build.host_compiler(), *build.ARCH, "-std=c++17", "-O1", "--expt-relaxed-constexpr",
