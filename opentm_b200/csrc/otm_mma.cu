@@ -731,6 +731,7 @@ struct Setup {
   };
 };
 
+// The two passes of a Newton step; blocks_per_sm: how many of an instance's blocks are resident on an SM.
 template <int M>
 struct LaunchDirmax {
   static void run(int nb, bool pairs, cudaStream_t s, const double* low, const double* upp, const MmaWork& w) {
@@ -749,17 +750,20 @@ struct LaunchTrial {
       k_mma_trial<M, 1><<<nb, 256, 0, s>>>(low, upp, w);
   }
 };
+template <int M>
+struct ResidentBlocks {
+  static void run(bool pairs, int* dirmax, int* trial, cudaError_t* e) {
+    const void* d = pairs ? (const void*)k_mma_dirmax<M, 2> : (const void*)k_mma_dirmax<M, 1>;
+    const void* t = pairs ? (const void*)k_mma_trial<M, 2> : (const void*)k_mma_trial<M, 1>;
+    *e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(dirmax, d, 256, 0);
+    if (*e == cudaSuccess) *e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(trial, t, 256, 0);
+  }
+};
 
 // Newton steps (a step-bound pass and a trial) queued before the host first looks, and between later
 // looks: a subproblem takes about 20 (measured on 128^3 and 384^3 design steps); a queued pair that
 // finds nothing due costs about 3 us, a look about 15.
 constexpr int kMmaFirstSteps = 16, kMmaMoreSteps = 4;
-
-// Grids of the passes: the blocks that are resident at once (112 and 78 registers a thread at m = 1), so
-// that a block's reduction and the last block's sum over all blocks are paid once per resident block and
-// not once per 256 variables (n = 2.1 M: trial 51 us and step bounds 44 us, 76 and 51 with 2048 blocks).
-constexpr int kMmaSms = 148, kMmaTrialBlocks = 2, kMmaDirmaxBlocks = 3;
-static_assert(4 * kMmaSms <= kMaxPartials, "the partial buffers hold kMaxPartials blocks");
 
 // One MMA step (mmasub_g, optimization/mmaOpt.cu:1021-1062): device arrays; a, c, d and the constraint
 // values in pr.
@@ -770,7 +774,10 @@ static otm_status mmasub_run(cudaStream_t s, int m, size_t n, int itn, const Mma
   const auto blocks = [](size_t work, int most) {
     return int(std::min<size_t>(size_t(most), std::max<size_t>(1, (work + 255) / 256)));
   };
-  const int nb = blocks(n, 4 * kMmaSms);
+  int dev = 0, sms = 0;
+  OTM_CUDA(cudaGetDevice(&dev));
+  OTM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int nb = blocks(n, std::min(4 * sms, kMaxPartials));
   uint64_t L = 0;
   dispatch_m<Setup<T>::template Launch>(m, nb, s, n, itn, in, xmin, xmax, xold1, xold2, low, upp, move, pr, w);
   L++;
@@ -781,7 +788,17 @@ static otm_status mmasub_run(cudaStream_t s, int m, size_t n, int itn, const Mma
   const bool pairs = m <= 4 && n % 2 == 0 && (reinterpret_cast<uintptr_t>(low) % 16) == 0 &&
                      (reinterpret_cast<uintptr_t>(upp) % 16) == 0;
   const size_t groups = n / (pairs ? 2 : 1);
-  const int nbt = blocks(groups, kMmaTrialBlocks * kMmaSms), nbd = blocks(groups, kMmaDirmaxBlocks * kMmaSms);
+  // grids of the blocks that are resident at once, so that a block's reduction and the last block's sum over
+  // all blocks are paid once per resident block (m = 1, n = 2.1 M: trial 51 us and step bounds 44 us, 76 and
+  // 51 with 2048 blocks) and no second wave fills a part of the GPU: registers allow two and three blocks an SM
+  // at m = 1, fewer from m = 2 on (three updates at n = 2.1 M with two and three blocks and with what fits:
+  // m = 2 9.93 and 9.13 ms, m = 4 12.7 and 11.9, m = 8 30.5 and 28.9)
+  int rd = 0, rt = 0;
+  cudaError_t e = cudaSuccess;
+  dispatch_m<ResidentBlocks>(m, pairs, &rd, &rt, &e);
+  OTM_CUDA(e);
+  const int nbt = blocks(groups, std::min(std::max(rt, 1) * sms, kMaxPartials)),
+            nbd = blocks(groups, std::min(std::max(rd, 1) * sms, kMaxPartials));
   const double *lowc = low, *uppc = upp;
   dispatch_m<LaunchTrial>(m, nbt, pairs, s, lowc, uppc, w);
   L++;
