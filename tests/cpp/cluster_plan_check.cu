@@ -3,7 +3,8 @@
 // CTA lies inside the planned bytes and no two overlap, the z-slabs cover every plane once, the
 // plane tables fit, and the ghost-copy rule of the kernel (a plane is the lower ghost of the CTA
 // whose slab starts after it and the upper ghost of the CTA whose slab ends before it; at most two
-// pushes per plane) feeds every ghost copy a CTA with planes reads. Host code only; prints "ok".
+// pushes per plane) feeds every ghost copy a CTA with planes reads; and a CTA's vertices have slots of their
+// own. Host code only; prints "ok".
 #include <algorithm>
 #include <cstdio>
 #include <utility>
@@ -24,6 +25,35 @@ static int fails = 0;
   } while (0)
 
 static int wrapz(int z, int n) { return ((z % n) + n) % n; }
+
+// The slots of a CTA's vertices (ClSlots, restated): every vertex its own, below the stencil stride; a
+// colour's slots consecutive and in the order in which the half sweeps and the global colour-blocked array
+// enumerate it; at most a lane per vertex of a colour.
+static void check_slots(const ClLevel& V, int l) {
+  const int nx = V.d.nx, ny = V.d.ny, hx = nx / 2, hy = ny / 2;
+  for (int c = 0; c < kCl; c++) {
+    const int z0 = V.zstart[c], z1 = V.zstart[c + 1];
+    std::vector<char> seen(size_t(V.ss), 0);
+    int n[2], zf[2];
+    for (int p = 0; p < 2; p++) {
+      zf[p] = z0 + ((z0 & 1) != p);
+      n[p] = (zf[p] < z1 ? (z1 - zf[p] + 1) / 2 : 0) * hx * hy;
+      CHECK(n[p] <= kClThreads, "level %d CTA %d: %d vertices of a colour", l, c, n[p]);
+    }
+    for (int z = z0; z < z1; z++)
+      for (int y = 0; y < ny; y++)
+        for (int x = 0; x < nx; x++) {
+          const int p = z & 1, cxy = (x & 1) + 2 * (y & 1);
+          const int t = ((z - zf[p]) / 2 * hy + y / 2) * hx + x / 2;  // place in the colour
+          const int slot = (p ? 4 * n[0] : 0) + cxy * n[p] + t;
+          const bool ok = t < n[p] && slot >= 0 && slot < V.ss && !seen[size_t(slot)];
+          CHECK(ok, "level %d CTA %d: slot %d of (%d, %d, %d)", l, c, slot, x, y, z);
+          if (ok) seen[size_t(slot)] = 1;
+          // the same order as the global colour-blocked array from the colour's first own plane on
+          CHECK((zf[p] / 2) * hx * hy + t == ((z / 2) * hy + y / 2) * hx + x / 2, "level %d: colour-blocked order", l);
+        }
+  }
+}
 
 static void check_stack(Dims d0) {
   // the levels of the cluster part: halve while every axis is even, >= 8 and above 64 unknowns
@@ -60,10 +90,16 @@ static void check_stack(Dims d0) {
     }
     CHECK(V.cs >= maxpl * V.d.nx * V.d.ny, "level %d: case stride too small", l);
     CHECK(V.urs >= V.d.nx && V.ups >= V.urs * V.d.ny && V.ucs >= (maxpl + 2) * V.ups, "level %d: u strides", l);
+    // odd sites of a row behind its even ones (cl_ux)
+    CHECK(V.uh >= (V.d.nx + 1) / 2 && V.uh + V.d.nx / 2 <= V.urs, "level %d: odd sites at %d of %d", l, V.uh, V.urs);
+    if (V.st_off >= 0) {
+      CHECK(V.ss >= V.cs, "level %d: stencil stride %d for %d vertices", l, V.ss, V.cs);
+      check_slots(V, l);
+    }
     add(V.u_off, 3L * V.ucs, "u", l);
     add(V.f_off, 3L * V.cs, "f", l);
     add(V.r_off, 3L * V.cs, "r", l);
-    add(V.st_off, 27L * V.cs, "stencils", l);
+    add(V.st_off, 27L * V.ss, "stencils", l);
     add(V.inv_off, long(V.cs), "inverse diagonal", l);
     CHECK(V.tab_off == tab_total, "level %d: plane table offset", l);
     tab_total += 3 * nz;

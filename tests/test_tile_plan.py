@@ -1,9 +1,10 @@
-"""CPU emulation of the tile-staged fine smoother and residual (opentm_b200/csrc/otm_tile.cuh).
+"""CPU emulation of the tile-staged smoothers and residual (opentm_b200/csrc/otm_tile.cuh, otm_ctile.cuh).
 
 The kernels' index arithmetic is restated here line by line (tile origins of both tilings, the
 periodic wrap of shifted tiles, the parity-split and padded shared-memory site order, the thread ->
-column-segment mapping, the six-plane streaming of a pass, the right-hand-side boxes the TMA copies
-deliver, the staged coarse block and the quad-wise prolongation, the write-back) and every
+register-block mapping and which of a pass's neighbours come from the block, the six-plane streaming of
+a pass, the right-hand side's two-wide loads, the staged coarse block and the quad-wise prolongation, the
+write-back from registers; on coarse levels also the copies of the stencils into shared memory) and every
 shared-memory and global access is checked to stay in bounds before the kernels run on a GPU.
 Within a pass no thread may read the values (.xyz) of a site that another thread writes in the
 same pass, and the write-back must cover each vertex once. The emulated arithmetic is then compared
@@ -21,9 +22,6 @@ SPLANE, SSITES = SROW * SY, SROW * SY * SZ
 THREADS, SEG, RTHREADS = 128, 4, 256
 CX, CY, CZ = TX // 2 + 2, TY // 2 + 2, TZ // 2 + 2
 CSITES = CX * CY * CZ
-FBX, FBY, FBZ = 8, 8, 4
-FBOX = FBX * FBY * FBZ * 3
-FCASE = FBX * FBY * FBZ
 OP = dict(c0=0.35, c2=-0.08, c3=-0.095)  # distinct c2 / c3 so that a mix-up shows
 NBR = [(-1, -1), (0, -1), (1, -1), (-1, 0), (1, 0), (-1, 1), (0, 1), (1, 1)]
 
@@ -55,36 +53,6 @@ def tile_origin(d, b, shift):
     q = b // ntx
     return ((b - q * ntx) * TX + shift * (TX // 2), (q % nty) * TY + shift * (TY // 2),
             (q // nty) * TZ + shift * (TZ // 2))
-
-
-def fpos(x, y, z):
-    assert 0 <= x < TX and 0 <= y < TY and 0 <= z < TZ
-    return ((x >> 3) + 2 * (y >> 3) + 4 * (z >> 2)) * FBOX + ((z & 3) * FBY + (y & 7)) * FBX + (x & 7)
-
-
-def f_box(d, f, x0, y0, z0):
-    """The eight TMA copies: box q = {8, 8, 4, 3} of the right-hand side at the wrapped origin
-    (x0 + 8 (q & 1), y0 + 8 ((q >> 1) & 1), z0 + 4 (q >> 2), 0), landing at q * 768, x fastest."""
-    nx, ny, nz = d
-    nv = nx * ny * nz
-    box = np.full(8 * FBOX, np.nan)
-    for q in range(8):
-        X, Y, Z = wrapm(x0 + FBX * (q & 1), nx), wrapm(y0 + FBY * ((q >> 1) & 1), ny), wrapm(z0 + FBZ * (q >> 2), nz)
-        assert X + FBX <= nx and Y + FBY <= ny and Z + FBZ <= nz, "a box never crosses the periodic boundary"
-        assert (X * 4) % 16 == 0, "TMA: the innermost coordinate times the element size is a multiple of 16 bytes"
-        for c in range(3):
-            for z in range(FBZ):
-                for y in range(FBY):
-                    for x in range(FBX):
-                        box[q * FBOX + ((c * FBZ + z) * FBY + y) * FBX + x] = f[c * nv + gidx(d, X + x, Y + y, Z + z)]
-    # the position function the passes use reads the values of the global array
-    for c in range(3):
-        for z in range(TZ):
-            for y in range(TY):
-                for x in range(TX):
-                    g = gidx(d, wrapm(x0 + x, nx), wrapm(y0 + y, ny), wrapm(z0 + z, nz))
-                    assert box[fpos(x, y, z) + c * FCASE] == f[c * nv + g]
-    return box
 
 
 def plane_coef(K):
@@ -121,35 +89,68 @@ class Smem:
         self.writes, self.reads = {}, {}
 
 
-def emulate_pass(sm, px, py, fsm, fs):
-    """tile_pass<PX, PY>: 128 threads, each a column segment of 4 vertices, 6 planes streamed."""
+class Block:
+    """A thread's register block: 2 x 2 columns from (lx, ly), planes lz0 .. lz0 + 3; value of column
+    c = cx + 2 cy, plane q in v[c][q] (u of the three cases and the conductivity)."""
+
+    def __init__(self, sm, t):
+        self.lx, self.ly, self.lz0 = 2 * (t & 7) + 1, 2 * ((t >> 3) & 7) + 1, 1 + SEG * (t >> 6)
+        assert self.lx + 1 <= TX and self.ly + 1 <= TY and self.lz0 + SEG - 1 <= TZ
+        self.v = [[list(sm.rd(tsite(self.lx + (c & 1), self.ly + (c >> 1), self.lz0 + q), t)) for q in range(SEG)]
+                  for c in range(4)]
+
+
+def tile_rhs(d, f, blk, x0, y0, z0, py):
+    """tile_rhs<PY>: the right-hand side of row py of the block, both columns by one 8-byte load."""
+    nx, ny, nz = d
+    nv = nx * ny * nz
+    X, Y = wrapm(x0 + blk.lx - 1, nx), wrapm(y0 + blk.ly - 1 + py, ny)
+    out = []
+    for q in range(SEG):
+        g = gidx(d, X, Y, wrapm(z0 + blk.lz0 - 1 + q, nz))
+        assert g % 2 == 0 and X + 1 < nx, "an aligned pair inside the row"
+        out.append([(f[c * nv + g], f[c * nv + g + 1]) for c in range(3)])
+    return out
+
+
+def emulate_pass(sm, blocks, rhs, px, py, last, fs):
+    """tile_pass<PX, PY, kLast>: every thread updates column (px, py) of its block, 6 planes streamed."""
     oL, oR = (SHALF - 1, SHALF) if px else (-SHALF, -SHALF + 1)
+    kcol = px + 2 * py
     for t in range(THREADS):
-        i, j, seg = t & 7, (t >> 3) & 7, t >> 6
-        lx, ly, lz0 = 2 * i + 1 + px, 2 * j + 1 + py, 1 + SEG * seg
-        assert 1 <= lx <= TX and 1 <= ly <= TY and 1 <= lz0 and lz0 + SEG - 1 <= TZ
+        own = blocks[t]
+        lx, ly, lz0 = own.lx, own.ly, own.lz0
+        cx0, cy0 = lx + px, ly + py
         # the compile-time neighbour offsets equal the site order's
-        assert tsite(lx - 1, ly, 1) - tsite(lx, ly, 1) == oL and tsite(lx + 1, ly, 1) - tsite(lx, ly, 1) == oR
-        fcol = fpos(lx - 1, ly - 1, lz0 - 1)
+        assert tsite(cx0 - 1, cy0, 1) - tsite(cx0, cy0, 1) == oL and tsite(cx0 + 1, cy0, 1) - tsite(cx0, cy0, 1) == oR
+        col = tsite(cx0, cy0, lz0 - 1)
         Kp, Cp = [0.0] * 4, None
         accA, accB, accC = [0.0] * 3, [0.0] * 3, [0.0] * 3
         dA = dB = 0.0
         for s in range(SEG + 2):
             P = lz0 - 1 + s
-            b = tsite(lx, ly, P)
-            offs = [oL - SROW, -SROW, oR - SROW, oL, oR, oL + SROW, SROW, oR + SROW]
-            for n, (ox, oy) in enumerate(NBR):
-                assert b + offs[n] == tsite(lx + ox, ly + oy, P)
-            nb = [sm.rd(b + o, t) for o in offs]
-            kown = sm.rd(b, t, "w")[3]
+            b = col + s * SPLANE
+            assert b == tsite(cx0, cy0, P)
+            nb = []
+            for ox, oy in NBR:
+                cx, cy = px + ox, py + oy
+                if 1 <= s <= SEG and 0 <= cx <= 1 and 0 <= cy <= 1:
+                    nb.append(own.v[cx + 2 * cy][s - 1])
+                else:
+                    i = b + (oL if ox < 0 else (oR if ox > 0 else 0)) + oy * SROW
+                    assert i == tsite(cx0 + ox, cy0 + oy, P)
+                    nb.append(sm.rd(i, t))
+            kown = 0.0
+            if 1 <= s <= SEG:
+                kown = own.v[kcol][s - 1][3]
+            elif s == 0:
+                kown = sm.rd(b, t, "w")[3]
             K = [nb[0][3], nb[1][3], nb[3][3], kown]
             sK = (K[0] + K[1]) + (K[2] + K[3])
-            C = plane_coef(K)
+            C = plane_coef(K) if s <= SEG else None
             dC = 0.0
             if s < SEG:
-                fv = fcol + s * (FBX * FBY)
-                assert fv == fpos(lx - 1, ly - 1, lz0 - 1 + s)
-                accC = [fsm[fv + c * FCASE] * fs[c] for c in range(3)]
+                accC = [rhs[t][s][c][px] * fs[c] for c in range(3)]
                 for n in range(8):
                     for c in range(3):
                         accC[c] -= C[n] * nb[n][c]
@@ -165,7 +166,9 @@ def emulate_pass(sm, px, py, fsm, fs):
                     for c in range(3):
                         accA[c] -= Cp[n] * nb[n][c]
                 inv = 1.0 / (OP["c0"] * dA)
-                sm.wr(tsite(lx, ly, P - 1), [accA[0] * inv, accA[1] * inv, accA[2] * inv, Kp[3]], t)
+                own.v[kcol][s - 2][:3] = [accA[c] * inv for c in range(3)]
+                if not last:
+                    sm.wr(tsite(cx0, cy0, lz0 + s - 2), own.v[kcol][s - 2], t)
             accA, accB = accB, accC
             accC = [0.0] * 3
             dA, dB = dB, dC
@@ -229,7 +232,6 @@ def emulate_sweep(d, dc, ks, u_in, uc, f, start, shift, reverse, fs=(1.0, 1.0, 1
     assert len(set(pos)) == SX * SY * SZ and pos[-1] < SSITES, "the site order is one-to-one and in bounds"
     for b in range(ntiles):
         x0, y0, z0 = tile_origin(d, b, shift)
-        fsm = f_box(d, f, x0, y0, z0)
         sm = Smem(SSITES)
         c0x, c0y, c0z = x0 // 2 - 1, y0 // 2 - 1, z0 // 2 - 1
         cb = np.zeros((CSITES, 4))
@@ -274,18 +276,26 @@ def emulate_sweep(d, dc, ks, u_in, uc, f, start, shift, reverse, fs=(1.0, 1.0, 1
             sm.wr(i, v, -1)
         assert len(staged) == SX * SY * SZ and set(staged.values()) == {1}, "every site staged once"
         sm.writes, sm.reads = {}, {}
-        for p in ((3, 2, 1, 0) if reverse else (0, 1, 2, 3)):
-            emulate_pass(sm, p & 1, p >> 1, fsm, fs)
-        for w in range(TX * TY * TZ // 4):
-            q, row = w & 3, w >> 2
-            ly, lz = 1 + row % TY, 1 + row // TY
-            g = gidx(d, wrapm(x0 + 4 * q, nx), wrapm(y0 + ly - 1, ny), wrapm(z0 + lz - 1, nz))
-            assert g % 4 == 0
-            for e in range(4):
-                o = sm.v[tsite(1 + 4 * q + e, ly, lz)]
-                written[g + e] += 1
-                for c in range(3):
-                    out[c * nv + g + e] = o[c]
+        blocks = [Block(sm, t) for t in range(THREADS)]
+        sm.writes, sm.reads = {}, {}
+        pa = 1 if reverse else 0
+        pb = 1 - pa
+        rhs = [tile_rhs(d, f, blk, x0, y0, z0, pa) for blk in blocks]
+        emulate_pass(sm, blocks, rhs, pa, pa, False, fs)
+        rhs2 = [tile_rhs(d, f, blk, x0, y0, z0, pb) for blk in blocks]
+        emulate_pass(sm, blocks, rhs, pb, pa, False, fs)
+        emulate_pass(sm, blocks, rhs2, pa, pb, False, fs)
+        emulate_pass(sm, blocks, rhs2, pb, pb, True, fs)
+        for blk in blocks:
+            X = wrapm(x0 + blk.lx - 1, nx)
+            for q in range(SEG):
+                for e in range(2):
+                    g = gidx(d, X, wrapm(y0 + blk.ly - 1 + e, ny), wrapm(z0 + blk.lz0 - 1 + q, nz))
+                    assert g % 2 == 0 and X + 1 < nx
+                    for px in range(2):
+                        written[g + px] += 1
+                        for c in range(3):
+                            out[c * nv + g + px] = blk.v[2 * e + px][q][c]
     assert (written == 1).all()
     return out
 
@@ -298,7 +308,6 @@ def emulate_resid(d, ks, u, f, fs=(1.0, 1.0, 1.0)):
     written = np.zeros(nv, dtype=int)
     for b in range((nx // TX) * (ny // TY) * (nz // TZ)):
         x0, y0, z0 = tile_origin(d, b, 0)
-        fsm = f_box(d, f, x0, y0, z0)
         sm = np.full((SSITES, 4), np.nan)
         for w in range(SY * SZ * (TX // 4)):
             q, row = w & 3, w >> 2
@@ -314,8 +323,9 @@ def emulate_resid(d, ks, u, f, fs=(1.0, 1.0, 1.0)):
             sm[rsite(lx, ly, lz)] = [u[g], u[nv + g], u[2 * nv + g], ks[g]]
         for t in range(RTHREADS):
             lx, ly = 1 + (t & 15), 1 + (t >> 4)
-            col = gidx(d, x0 + lx - 1, y0 + ly - 1, 0)
             pl = nx * ny
+            col = gidx(d, x0 + lx - 1, y0 + ly - 1, z0)
+            fn = [f[c * nv + col] for c in range(3)]  # right-hand side of vertex P + 1
             Kp, Cp = [0.0] * 4, None
             accA, accB, accC = [0.0] * 3, [0.0] * 3, [0.0] * 3
             dA = dB = 0.0
@@ -333,8 +343,10 @@ def emulate_resid(d, ks, u, f, fs=(1.0, 1.0, 1.0)):
                 C = plane_coef(K)
                 dC = 0.0
                 if P + 1 <= TZ:
-                    fv = fpos(lx - 1, ly - 1, P)
-                    accC = [fsm[fv + c * FCASE] * fs[c] for c in range(3)]
+                    accC = [fn[c] * fs[c] for c in range(3)]
+                    if P + 2 <= TZ:
+                        assert col + (P + 1) * pl < nv
+                        fn = [f[c * nv + col + (P + 1) * pl] for c in range(3)]
                     for n in range(8):
                         for c in range(3):
                             accC[c] -= C[n] * nb[n][c]
@@ -351,7 +363,7 @@ def emulate_resid(d, ks, u, f, fs=(1.0, 1.0, 1.0)):
                         for c in range(3):
                             accA[c] -= Cp[n] * nb[n][c]
                     diag = OP["c0"] * dA
-                    g = col + (z0 + P - 2) * pl
+                    g = col + (P - 2) * pl
                     assert 0 <= g < nv
                     written[g] += 1
                     for c in range(3):
@@ -620,6 +632,118 @@ def emulate_csweep(d, dc, st, u_in, uc, f, start, shift, reverse):
     return out
 
 
+# few tiles: k_ctile_sweep_small
+SMALL_THREADS = 3 * CTHREADS
+SMALL_ROW = 20
+SMALL_PLANE, SMALL_CASE = SMALL_ROW * CSY, SMALL_ROW * CSY * CSZ
+SMALL_STENCILS = 8 * 27 * CTHREADS
+
+
+def cspos(lx, ly, lz):
+    assert 0 <= lx < CSX and 0 <= ly < CSY and 0 <= lz < CSZ
+    return lz * SMALL_PLANE + ly * SMALL_ROW + ((CSHALF + (lx >> 1)) if (lx & 1) else (lx >> 1))
+
+
+def small_stencils(d, st, x0, y0, z0, reverse):
+    """The copies of a CTA's stencils, 16 bytes each, and after which copy group each word has landed."""
+    nx, ny, nz = d
+    nv, nsub = nx * ny * nz, nx * ny * nz // 8
+    hx, hy, hz = nx // 2, ny // 2, nz // 2
+    sm = np.full(SMALL_STENCILS, np.nan)
+    group = np.full(SMALL_STENCILS, -1)
+    for warp in range(SMALL_THREADS // 32):
+        for lane in range(32):
+            h, r = lane & 1, lane >> 1
+            X, Y, Z = wrapm(x0 // 2 + 4 * h, hx), wrapm(y0 // 2 + (r & 3), hy), wrapm(z0 // 2 + (r >> 2), hz)
+            src, dst = X + hx * (Y + hy * Z), r * 8 + h * 4
+            assert X + 4 <= hx, "half a row never crosses the periodic boundary"
+            q = warp
+            for p in range(8):
+                c = 7 - p if reverse else p
+                for _ in range(3):
+                    if q < 27 * (p + 1):
+                        o = q - 27 * p
+                        assert 0 <= o < 27
+                        a, g = dst + (c * 27 + o) * CTHREADS, src + o * nv + c * nsub
+                        assert a % 4 == 0 and g % 4 == 0 and 0 <= g and g + 3 < 27 * nv
+                        assert (group[a:a + 4] == -1).all(), "every word copied once"
+                        sm[a:a + 4], group[a:a + 4] = st[g:g + 4], p
+                        q += SMALL_THREADS // 32
+            assert q >= 27 * 8
+    assert (group >= 0).all()
+    return sm, group
+
+
+def emulate_csmall(d, dc, st, u_in, uc, f, start, shift, reverse):
+    """k_ctile_sweep_small<start, reverse> over all coarse tiles of tiling `shift`: a lane per vertex of a
+    colour and load case, stencils in shared memory."""
+    nx, ny, nz = d
+    nv = nx * ny * nz
+    out = np.full(3 * nv, np.nan)
+    written = np.zeros(3 * nv, dtype=int)
+    pos = [cspos(lx, ly, lz) for lz in range(CSZ) for ly in range(CSY) for lx in range(CSX)]
+    assert len(set(pos)) == len(pos) and max(pos) < SMALL_CASE
+    for b in range((nx // CTX) * (ny // CTY) * (nz // CTZ)):
+        x0, y0, z0 = ctile_origin(d, b, shift)
+        st_sm, group = small_stencils(d, st, x0, y0, z0, reverse)
+        c0x, c0y, c0z = x0 // 2 - 1, y0 // 2 - 1, z0 // 2 - 1
+        cb = np.zeros((CCSITES, 4))
+        if start == 2:
+            cnx, cny, cnz = dc
+            nvc = cnx * cny * cnz
+            for q in range(3 * CCSITES):
+                c, s = q // CCSITES, q % CCSITES
+                ax, ay, az = s % CCX, (s // CCX) % CCY, s // (CCX * CCY)
+                cb[s, c] = uc[c * nvc + gidx(dc, wrapm(c0x + ax, cnx), wrapm(c0y + ay, cny), wrapm(c0z + az, cnz))]
+        sites = np.full(3 * SMALL_CASE, np.nan)
+        nsites = CSX * CSY * CSZ
+        for q in range(3 * nsites):
+            c, s = q // nsites, q % nsites
+            lx, ly, lz = s % CSX, (s // CSX) % CSY, s // (CSX * CSY)
+            ux, uy, uz = x0 - 1 + lx, y0 - 1 + ly, z0 - 1 + lz
+            v = u_in[c * nv + gidx(d, wrapm(ux, nx), wrapm(uy, ny), wrapm(uz, nz))] if start >= 1 else 0.0
+            if start == 2:
+                v += cprolong_site(cb, ux, uy, uz, c0x, c0y, c0z)[c]
+            sites[c * SMALL_CASE + cspos(lx, ly, lz)] = v
+        for p in range(8):
+            C = 7 - p if reverse else p
+            cx, cy, cz = C & 1, (C >> 1) & 1, C >> 2
+            oL, oR = (-CSHALF, -CSHALF + 1) if cx == 0 else (CSHALF - 1, CSHALF)
+            reads, writes = [], {}
+            for t in range(SMALL_THREADS):
+                warp, lane = t >> 5, t & 31
+                i, j, k, cs = lane & 7, lane >> 3, warp & 3, warp >> 2
+                X, Y, Z = (wrapm(x0 + 2 * i + cx, nx), wrapm(y0 + 2 * j + cy, ny), wrapm(z0 + 2 * k + cz, nz))
+                sp = C * 27 * CTHREADS + i + 8 * j + 32 * k
+                assert (group[sp:sp + 27 * CTHREADS:CTHREADS] <= p).all(), "the pass waits for its copies"
+                assert all(st_sm[sp + o * CTHREADS] == st[o * nv + cb_index(d, X, Y, Z)] for o in (0, 13, 26))
+                base = cs * SMALL_CASE + cspos(1 + 2 * i + cx, 1 + 2 * j + cy, 1 + 2 * k + cz)
+                acc = f[cs * nv + gidx(d, X, Y, Z)]
+                for o in range(27):
+                    if o == 13:
+                        continue
+                    ox, oy, oz = o % 3 - 1, (o // 3) % 3 - 1, o // 9 - 1
+                    off = (oL if ox < 0 else (oR if ox > 0 else 0)) + oy * SMALL_ROW + oz * SMALL_PLANE
+                    assert base + off == cs * SMALL_CASE + cspos(1 + 2 * i + cx + ox, 1 + 2 * j + cy + oy, 1 + 2 * k + cz + oz)
+                    reads.append(base + off)
+                    acc -= st_sm[sp + o * CTHREADS] * sites[base + off]
+                assert base not in writes
+                writes[base] = acc / st_sm[sp + 13 * CTHREADS]
+            assert not set(reads) & set(writes), "no lane reads what another writes in the pass"
+            for a, v in writes.items():
+                sites[a] = v
+        for t in range(SMALL_THREADS):
+            cs = t // CTHREADS
+            for it in range(CTX * CTY * CTZ // CTHREADS):
+                s = t - cs * CTHREADS + it * CTHREADS
+                lx, ly, lz = 1 + s % CTX, 1 + (s // CTX) % CTY, 1 + s // (CTX * CTY)
+                g = cs * nv + gidx(d, wrapm(x0 + lx - 1, nx), wrapm(y0 + ly - 1, ny), wrapm(z0 + lz - 1, nz))
+                written[g] += 1
+                out[g] = sites[cs * SMALL_CASE + cspos(lx, ly, lz)]
+    assert (written == 1).all()
+    return out
+
+
 def block_gs_stencil(d, st, u0, f, order, shift):
     """Colour Gauss-Seidel with 27-point stencils per 16 x 8 x 8 block of tiling `shift`, halo frozen."""
     nx, ny, nz = d
@@ -682,4 +806,13 @@ def test_coarse_sweep_with_prolongation_reverse_shifted(cfields):
     d, dc, st, f, u_in, uc = cfields
     got = emulate_csweep(d, dc, st, u_in, uc, f, start=2, shift=1, reverse=True)
     ref = block_gs_stencil(d, st, u_in + prolong(d, dc, uc), f, list(range(8))[::-1], 1)
+    assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("start,shift,reverse", [(0, 0, False), (1, 1, False), (2, 1, True), (1, 0, True)])
+def test_small_coarse_sweep(cfields, start, shift, reverse):
+    d, dc, st, f, u_in, uc = cfields
+    got = emulate_csmall(d, dc, st, u_in, uc, f, start, shift, reverse)
+    u0 = [np.zeros_like(f), u_in, u_in + prolong(d, dc, uc)][start]
+    ref = block_gs_stencil(d, st, u0, f, list(range(8))[::-1] if reverse else list(range(8)), shift)
     assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()
