@@ -396,6 +396,7 @@ otm_status Homo::build(const otm_config& c, cudaStream_t ext_stream, cudaMemPool
     OTM_CUDA(cudaMemsetAsync(V.f, 0, bytes, stream));
   }
   OTM_CUDA(cudaMemsetAsync(x, 0, 3 * nv * sizeof(float), stream));
+  x_zero = true;
   if (mixed) {
     OTM_CUDA(cudaMemsetAsync(x64, 0, 3 * nv * sizeof(double), stream));
     OTM_CUDA(cudaMemsetAsync(u16, 0, 3 * nv * 2, stream));
