@@ -86,7 +86,7 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// ---- vector loads and stores of 4 consecutive values in the storage types --------------------
+// ---- vector loads and stores of consecutive values in the storage types --------------------
 __device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
   const float4 q = __ldg(reinterpret_cast<const float4*>(p));
   v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
@@ -103,23 +103,6 @@ __device__ __forceinline__ void ld4(const __half* p, float (&v)[4]) {
   const __half2 b = *reinterpret_cast<const __half2*>(&q.y);
   v[0] = __low2float(a), v[1] = __high2float(a), v[2] = __low2float(b), v[3] = __high2float(b);
 }
-__device__ __forceinline__ void st4(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void st4(__nv_bfloat16* p, const float (&v)[4]) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-  uint2 q;
-  q.x = *reinterpret_cast<const uint32_t*>(&a);
-  q.y = *reinterpret_cast<const uint32_t*>(&b);
-  *reinterpret_cast<uint2*>(p) = q;
-}
-__device__ __forceinline__ void st4(__half* p, const float (&v)[4]) {
-  const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
-  uint2 q;
-  q.x = *reinterpret_cast<const uint32_t*>(&a);
-  q.y = *reinterpret_cast<const uint32_t*>(&b);
-  *reinterpret_cast<uint2*>(p) = q;
-}
 
 // 2 consecutive values (8 bytes in FP32, 4 bytes in 16-bit storage)
 __device__ __forceinline__ void st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
@@ -129,6 +112,7 @@ __device__ __forceinline__ void st2(__nv_bfloat16* p, float a, float b) {
 __device__ __forceinline__ void st2(__half* p, float a, float b) {
   *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
 }
+
 // ---- coefficients ------------------------------------------------------------------------------
 // Coefficients of the 8 neighbour columns of a vertex for one element plane, from the 4
 // conductivities K[b] (b = bx + 2 by: the element whose lower corner is (x - 1 + bx, y - 1 + by)
