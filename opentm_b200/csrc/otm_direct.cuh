@@ -147,7 +147,7 @@ __device__ __forceinline__ void dir_make_panel(const double* rows, int kb, int n
   }
 }
 
-// Bound by the chain of steps (panel copy, update of the next block, 16 pivots, one barrier: about 5 us
+// Bound by the chain of steps (panel copy, update of the next block, 16 pivots, one barrier: about 8 us
 // each), not by its 2 n^3 FP64 operations. update() + solve, in us, against one CTA that eliminated one
 // pivot at a time (matrix in shared memory up to n = 160, else in L2):
 //   n         64    125    216    315    343     729     990

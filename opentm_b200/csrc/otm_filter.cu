@@ -65,15 +65,15 @@ static otm_status make_weights(int type, float radius, ConvWeights* cw) {
 // the chunk (and H planes either side) is staged once in shared memory, with periodic wrap or zeros
 // outside, the next one being fetched into registers meanwhile; a thread reads the (kNY + 2H) x (2H + 1)
 // window around its outputs once per plane and adds every value to the 2H + 1 outputs along z that it
-// is a tap of (rolling accumulators): 9 reads per output at radius 2 with one row, 17.5 at radius 3 with
+// is a tap of (rolling accumulators): 9 reads per output at radius 2 with one row, 10 at radius 3 with
 // four, where a read per tap takes 27 and 93. The weight depends on the squared distance only, and with the
 // loops unrolled its place in the parameter bank is a constant, so a tap is one FMA. The radii in common
 // use (1.5 to 2, 2.5 to 3, 3.5 to 3.6, 3.75 to 4) have their set of taps compiled in; the other radii of a half
 // width H share the taps within H - 1/2, and those from there to H + 1/2 are predicated on the radius. (With a
 // branch per tap, and from half width 5 on with weights looked up by a run-time index and four rows a thread,
 // these radii took up to four times the time of a kernel that reads every tap's value for itself: 128^3,
-// radius 4.4, 5 and 6: 194, 333 and 845 us against 140, 189 and 297; now 92, 127 and 187.) An output's taps are summed in the reference's order (x fastest, z
-// slowest; the adjoint streams z downwards for that).
+// radius 4.4, 5 and 6: 194, 333 and 845 us against 140, 189 and 297; now 92, 127 and 187.) An output's taps
+// are summed in the reference's order (x fastest, z slowest; the adjoint streams z downwards for that).
 //   MODE 0: forward            out = sum w src / sum_valid w
 //   MODE 1: forward + SIMP     also k = (k0 - kmin) out^p + kmin and dk = dk/dout
 //   MODE 2: adjoint            out = sum_off w g(i - off) / ws(i - off)
