@@ -120,27 +120,35 @@ __device__ __forceinline__ void valid_weights(const Radial<H>& rw, int xlo, int 
   float a = 0.f;
 #pragma unroll
   for (int g = 0; g <= H; g++) low[g] = 0.f;
-#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
-  for (int ez = -H; ez <= H; ez++) {
-#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
-    for (int ey = -H; ey <= H; ey++) {
-      if (ey < ylo || ey > yhi || ey * ey + ez * ez >= rw.smax) continue;  // the same for all lanes of a warp
-      float w[2 * H + 1];
-      auto beyond = [&](int ex) { return H <= 4 && ex * ex + ey * ey + ez * ez >= kReach; };  // of every radius
+  auto row = [&](int ez, int ey) {
+    float w[2 * H + 1];
+    auto beyond = [&](int ex) { return H <= 4 && ex * ex + ey * ey + ez * ez >= kReach; };  // of every radius
+#pragma unroll
+    for (int ex = -H; ex <= H; ex++)
+      if (!beyond(ex)) w[ex + H] = ex >= xlo && ex <= xhi ? rw.w[ex * ex + ey * ey + ez * ez] : 0.f;
+    if (H <= 4 || !kLow || g1 >= H)
 #pragma unroll
       for (int ex = -H; ex <= H; ex++)
-        if (!beyond(ex)) w[ex + H] = ex >= xlo && ex <= xhi ? rw.w[ex * ex + ey * ey + ez * ez] : 0.f;
-      if (H <= 4 || !kLow || g1 >= H)
+        if (!beyond(ex)) a += w[ex + H];
+    if (kLow)
 #pragma unroll
-        for (int ex = -H; ex <= H; ex++)
-          if (!beyond(ex)) a += w[ex + H];
-      if (kLow)
+      for (int g = 0; g < H; g++)
+        if (ez >= -g && (H <= 4 || (g >= g0 && g < g1)))
 #pragma unroll
-        for (int g = 0; g < H; g++)
-          if (ez >= -g && (H <= 4 || (g >= g0 && g < g1)))
+          for (int ex = -H; ex <= H; ex++)
+            if (!beyond(ex)) low[g] += w[ex + H];
+  };
+#pragma unroll(H <= 4 ? 2 * H + 1 : 1)
+  for (int ez = -H; ez <= H; ez++) {
+    if (H <= 4) {
 #pragma unroll
-            for (int ex = -H; ex <= H; ex++)
-              if (!beyond(ex)) low[g] += w[ex + H];
+      for (int ey = -H; ey <= H; ey++)
+        if (ey >= ylo && ey <= yhi && ey * ey + ez * ez < rw.smax) row(ez, ey);  // the same for all lanes of a warp
+    } else {
+      int ry = H;  // rows of the plane within the filter's reach
+      while (ry >= 0 && ry * ry + ez * ez >= rw.smax) ry--;
+#pragma unroll 4
+      for (int ey = max(ylo, -ry); ey <= min(yhi, ry); ey++) row(ez, ey);
     }
 #pragma unroll
     for (int m = 0; m <= H; m++)
